@@ -58,6 +58,7 @@ GPU_SOURCES = [
     "gpuforce/pgf_kernels_fp64.cu",
     "gpuforce/pgf_kernels_mixed.cu",
     "gpuforce/pgf_kernels_ws.cu",
+    "gpuforce/pgf_kernels_far.cu",
     "gpuforce/pgf_noalloc.cu",
     "gpuforce/pgf_hostdirect.cu",
     "gpuforce/pgf_kernels_gradient.cu",
@@ -70,6 +71,7 @@ GPU_FILE_FLAGS = {
 }
 GPU_HEADERS = [
     "gpuforce/pgf_internal.cuh",
+    "gpuforce/pgf_localexp.cuh",
 ]
 
 

@@ -33,7 +33,7 @@ using namespace pgf;
 constexpr int kMaxTags = 16;
 constexpr int kMaxChunks = 8;                       // pipeline stages of a large dispatch
 constexpr int64_t kChunkIdEntries = 12 << 20;       // about 48 MB of id lists per stage
-constexpr int kScratchInts = 8 + 2 * kMaxChunks;
+constexpr int kScratchInts = 8 + kLaunchCounters * kMaxChunks;
 constexpr int kHdErrWords = 4;  // HdWalkArgs::err
 static_assert(PGF_NUM_KERNEL_VARIANTS == 1 + kNumWsVariants, "variant 0 plus the warp-specialised variants");
 constexpr int64_t kMaxRows = 0x7fffffff;
@@ -113,6 +113,8 @@ struct TagState {
     std::vector<int64_t> epi_disp;
     DevBuf<EpiDev> epi;
     DevBuf<int32_t> id_epj, id_spj, order;
+    DevBuf<int32_t> id_spj_near;  // far-field pass: Params::id_spj_near, spj_near
+    DevBuf<SpjNear> spj_near;
     DevBuf<WalkDesc> walks;
     DevBuf<Accp> accp;
     DevBuf<int32_t> nnb;
@@ -121,7 +123,7 @@ struct TagState {
     HostBuf<WalkDesc> h_walks;
     HostBuf<Accp> h_accp;
     HostBuf<int32_t> h_nnb;
-    HostBuf<int32_t> h_flags;  // queue head, n_retest, err, re-tested records
+    HostBuf<int32_t> h_flags;  // -, -, err, re-tested records
     DevBuf<CoRec> epi_co;      // fused changeover mode
     HostBuf<CoRec> h_epi_co;
     DevBuf<double> pot_soft;
@@ -203,8 +205,8 @@ struct State {
     int64_t n_epj_tot = 0, n_spj_tot = 0;
     bool j_sent = false;
     // scratch
-    // [0] queue head, [1] n_retest (single launch), [2] err, [3] re-tested
-    // records, [8 + 2s], [9 + 2s]: queue head and n_retest of pipeline stage s
+    // [2] err, [3] re-tested records, [4..6] launch counters of a single
+    // launch, [8 + 3s ..] those of pipeline stage s
     DevBuf<int32_t> scratch;
     DevBuf<Retest> retest;
     int retest_cap = 0;
@@ -622,24 +624,32 @@ void bind_scratch(Params& p, int stage = -1, int n_stages = 1) {
     p.err = g.scratch.d + 2;
     p.retest_total = g.scratch.d + 3;
     if (stage < 0) {
-        p.queue_head = g.scratch.d;
-        p.n_retest = g.scratch.d + 1;
+        bind_counters(p, g.scratch.d + 4);
         p.retest = g.retest.d;
         p.retest_cap = g.retest_cap;
     } else {
         const int cap = g.retest_cap / n_stages;
-        p.queue_head = g.scratch.d + 8 + 2 * stage;
-        p.n_retest = g.scratch.d + 9 + 2 * stage;
+        bind_counters(p, g.scratch.d + 8 + kLaunchCounters * stage);
         p.retest = g.retest.d + (size_t)stage * cap;
         p.retest_cap = cap;
     }
+}
+
+// Whether the far-field pass runs before the tag's pair kernel: the warp-
+// specialised and gradient kernels read its lists.
+bool runs_far(const TagState& t) {
+    if (t.mode == PGF_MODE_NEIGHBOR_SEARCH) return false;
+    if (t.mode == PGF_MODE_GRADIENT || t.mode == PGF_MODE_FORCE_CHANGEOVER) return true;
+    return t.precision == PGF_PRECISION_MIXED && t.variant != 0;
 }
 
 // Main kernel of the tag's precision and variant on stream s, bracketed by two
 // events, then the FP64 neighbour re-test.
 int launch_kernels(const TagState& t, const Params& p, cudaStream_t s, cudaEvent_t ev_start, cudaEvent_t ev_end) {
     PGF_CUDA(cudaEventRecord(ev_start, s));
-    cudaError_t e;
+    cudaError_t e = reset_counters(p, s);
+    if (e == cudaSuccess && runs_far(t)) e = launch_far(p, s, g.num_sms);
+    if (e != cudaSuccess) return fail(PGF_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
     if (t.mode == PGF_MODE_GRADIENT) {
         e = launch_gradient(p, s, g.num_sms);
         if (e == cudaSuccess) e = cudaEventRecord(ev_end, s);
@@ -654,7 +664,6 @@ int launch_kernels(const TagState& t, const Params& p, cudaStream_t s, cudaEvent
     } else if (t.precision == PGF_PRECISION_FP64) {
         e = launch_fp64(p, s, g.num_sms);
         if (e == cudaSuccess) e = cudaEventRecord(ev_end, s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(p.n_retest, 0, sizeof(int32_t), s);
     } else {
         e = t.variant == 0 ? launch_mixed(p, s, g.num_sms) : launch_ws(p, s, g.num_sms, t.variant - 1, &g.tmaps);
         if (e == cudaSuccess) e = cudaEventRecord(ev_end, s);
@@ -786,7 +795,9 @@ bool pack_walk(TagState& t, int k, int w, const Slot3& o, const void* const* epi
         d.hx = d.hy = d.hz = d.rs_max = 0.f;
     }
     d.part = 0;
-    d.pad[0] = d.pad[1] = d.pad[2] = 0.f;
+    d.n_parts = 1;
+    d.root = k;
+    d.n_spj_all = n_spj[w];
     d.rcut2 = g.walk_rcut2.empty() ? g.rcut2 : g.walk_rcut2[w];
     t.h_walks.h[k] = d;
     t.h_order.h[k] = k;
@@ -1065,6 +1076,11 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
     PGF_CUDA(t.epi.ensure(ni_all));
     PGF_CUDA(t.id_epj.ensure(ne));
     PGF_CUDA(t.id_spj.ensure(ns));
+    const bool far = far_applies(g.eps2, ni) && ns > 0 && t.mode != PGF_MODE_NEIGHBOR_SEARCH;
+    if (far) {
+        PGF_CUDA(t.id_spj_near.ensure(ns));
+        PGF_CUDA(t.spj_near.ensure(n_walk));
+    }
     PGF_CUDA(t.walks.ensure(n_desc));
     PGF_CUDA(t.order.ensure(n_desc));
     PGF_CUDA(t.accp.ensure(ni_all));
@@ -1104,9 +1120,14 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
     }
     p.id_epj = t.id_epj.d;
     p.id_spj = t.id_spj.d;
+    if (far) {
+        p.id_spj_near = t.id_spj_near.d;
+        p.spj_near = t.spj_near.d;
+    }
     p.walks = t.walks.d;
     p.order = t.order.d;
     p.n_walk = n_desc;
+    p.n_root = n_walk;
     p.gr_compensated = g.gr_compensated;
     // The neighbour search tests r^2 < max(rs_i, rs_j)^2 without softening
     // (src/soft_force.hpp:11-34); the force kernels include eps^2.
@@ -1186,6 +1207,7 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
                     d.n_epj = e1 - e0;
                     d.spj_begin = d0.spj_begin + s0;
                     d.n_spj = s1 - s0;
+                    d.n_parts = sp.parts;
                     if (j == 0) {
                         t.h_walks.h[sp.k] = d;
                         continue;
@@ -1256,7 +1278,7 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
         }
         Params pc = p;
         pc.order = t.order.d + k0;
-        pc.n_walk = k1 - k0;
+        pc.n_walk = pc.n_root = k1 - k0;
         bind_scratch(pc, c, n_chunks);
         if ((r = launch_kernels(t, pc, sc, t.evc[c][2], t.evc[c][3])) != PGF_OK) {
             drain();
@@ -1789,6 +1811,8 @@ int pgf_finalize(void) {
         t.epi.release();
         t.id_epj.release();
         t.id_spj.release();
+        t.id_spj_near.release();
+        t.spj_near.release();
         t.order.release();
         t.walks.release();
         t.accp.release();

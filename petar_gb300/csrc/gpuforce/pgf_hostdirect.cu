@@ -310,7 +310,9 @@ __global__ __launch_bounds__(kGatherThreads) void gather_walks_kernel(HdWalkArgs
                 d.hx = d.hy = d.hz = d.rs_max = 0.f;
             }
             d.part = 0;
-            d.pad[0] = d.pad[1] = d.pad[2] = 0.f;
+            d.n_parts = w.parts;
+            d.root = k;
+            d.n_spj_all = w.n_spj;
             d.rcut2 = w.rcut2;
             // A split walk: part j takes a slice of both lists; parts >= 1
             // read the copy of the walk's rows at rows1 + (j - 1) n_i.

@@ -109,7 +109,9 @@ struct __align__(32) WalkDesc {
     float hx, hy, hz;   // EPI box half-extents, rounded up
     float rs_max;       // largest r_search of the walk's EPI, rounded up
     int32_t part;       // 0, or k >= 1 for part k of a split walk (adds no per-i terms)
-    float pad[3];
+    int32_t n_parts;    // 1, or the parts of a split walk
+    int32_t root;       // descriptor of part 0 (this one when not split)
+    int32_t n_spj_all;  // SPJ of the whole walk
 };
 static_assert(sizeof(WalkDesc) == 96, "WalkDesc layout");
 
@@ -127,6 +129,17 @@ struct Retest {
     int32_t n;        // number of list entries
     int32_t walk;     // walk (descriptor index) of the i-particle
     int32_t pad;
+};
+
+// Superparticles of one walk left to the pair kernels by the far-field pass:
+// the entries in each quarter of the walk's list (n[0] < 0: the list as it
+// is), and whether out_accp of the walk's rows holds the sums of the others
+// (without G, each as an FP32 (hi, lo) pair: far_sum) for the pair kernels to
+// add.
+struct __align__(32) SpjNear {
+    int32_t n[4];
+    int32_t add_far;
+    int32_t pad[3];
 };
 
 struct Params {
@@ -155,11 +168,16 @@ struct Params {
     Accp* out_accp;
     int32_t* out_nnb;
     // scratch
-    int32_t* queue_head;   // work-queue cursor, zeroed before each launch
+    // Launch counters, kLaunchCounters ints that lie together and are zeroed
+    // before each launch (reset_counters): the work-queue cursor, the number
+    // of re-test records pushed (n_retest, may exceed the capacity) and the
+    // far-field pass's cursor.
+    int32_t* queue_head;
+    int32_t* n_retest;     // queue_head + 1
+    int32_t* far_queue;    // queue_head + 2
     Retest* retest;        // FP64 re-test records
-    int32_t* n_retest;     // number of records pushed (may exceed capacity)
     int32_t retest_cap;
-    int32_t pad1;
+    int32_t pad2;
     int32_t* err;          // device error word (0 = ok)
     int32_t* retest_total; // records re-tested since the host last read it (optional)
     // Walk count written by an earlier kernel on the same stream (the device
@@ -171,6 +189,15 @@ struct Params {
     // Test hook: > 0 makes their producer stop after that many ring items.
     int32_t stall_after_items;
     int32_t gr_compensated;  // gradient pass: r^2 and 1/r of far pairs to about 2^-40 (pgf_set_gradient_accuracy)
+    // Far-field pass (pgf_kernels_far.cu), or null: the ids of the
+    // superparticles left to the pair kernels (same offsets as id_spj), and
+    // per walk (by root descriptor) what they hold.
+    int32_t* id_spj_near;
+    SpjNear* spj_near;
+    // Walks without their further parts: when some are split (n_root <
+    // n_walk) the roots are descriptors 0 .. n_root - 1 by descending cost.
+    int32_t n_root;
+    int32_t pad1;
     // Result of the device-side check of a host-direct dispatch's ids, or
     // null: when it is non-zero the force kernels run nothing.
     const int32_t* input_err;
@@ -331,7 +358,82 @@ cudaError_t launch_gather_j(const HdSendArgs& a, int num_sms, cudaStream_t s);
 cudaError_t launch_gather_walks(const HdWalkArgs& a, int num_sms, cudaStream_t s);
 cudaError_t launch_scatter_results(const HdScatterArgs& a, int num_sms, cudaStream_t s);
 
+constexpr int kLaunchCounters = 3;
+inline void bind_counters(Params& p, int32_t* c) {
+    p.queue_head = c;
+    p.n_retest = c + 1;
+    p.far_queue = c + 2;
+}
+inline cudaError_t reset_counters(const Params& p, cudaStream_t s) {
+    return cudaMemsetAsync(p.queue_head, 0, kLaunchCounters * sizeof(int32_t), s);
+}
+
+// The far-field pass pays from some thousand i-particles per launch: below,
+// its launch costs more than the pairs it saves.  It expands unsoftened
+// gravity only.
+constexpr int64_t kFarMinRows = 8192;
+inline bool far_applies(double eps2, int64_t n_i) { return eps2 == 0.0 && n_i >= kFarMinRows; }
+
+// The far-field sums in row gi: acceleration x, y, z and potential.
+__device__ __forceinline__ void far_sum(const Params& p, int gi, double f[4]) {
+    const float4* r = reinterpret_cast<const float4*>(p.out_accp + gi);
+    const float4 a = r[0], b = r[1];
+    f[0] = (double)a.x + (double)a.y;
+    f[1] = (double)a.z + (double)a.w;
+    f[2] = (double)b.x + (double)b.y;
+    f[3] = (double)b.z + (double)b.w;
+}
+
+// The superparticle list the pair kernels run for one descriptor: entries
+// [begin, begin + n) of the walk's own list, or of its compacted one, whose
+// quarter q starts where quarter q of the walk's list does and follows the
+// others in the numbering.  A part of a split walk takes its share of the
+// compacted list.  Part 0 adds the far-field sums.
+struct SpjList {
+    const int32_t* ids;
+    int n;
+    int begin;
+    int after1, after2, after3;  // entries before quarters 1, 2, 3
+    int gap1, gap2, gap3;        // id offset minus entry number in those quarters
+    bool add_far;
+    __device__ __forceinline__ const int32_t* at(int k) const {
+        const int e = begin + k;
+        return ids + e + (e < after2 ? (e < after1 ? 0 : gap1) : (e < after3 ? gap2 : gap3));
+    }
+};
+__device__ __forceinline__ SpjList spj_list(const Params& p, const WalkDesc& wd) {
+    SpjList l;
+    if (p.spj_near) {
+        const SpjNear c = p.spj_near[wd.root];
+        if (c.n[0] >= 0) {
+            const int64_t all = wd.n_spj_all;
+            l.ids = p.id_spj_near + (wd.spj_begin - (int)(all * wd.part / wd.n_parts));
+            l.after1 = c.n[0];
+            l.after2 = l.after1 + c.n[1];
+            l.after3 = l.after2 + c.n[2];
+            l.gap1 = (int)(all / 4) - l.after1;
+            l.gap2 = (int)(all * 2 / 4) - l.after2;
+            l.gap3 = (int)(all * 3 / 4) - l.after3;
+            const int64_t total = l.after3 + c.n[3];
+            l.begin = (int)(total * wd.part / wd.n_parts);
+            l.n = (int)(total * (wd.part + 1) / wd.n_parts) - l.begin;
+            l.add_far = c.add_far != 0 && wd.part == 0;
+            return l;
+        }
+    }
+    l.ids = p.id_spj + wd.spj_begin;
+    l.n = wd.n_spj;
+    l.begin = 0;
+    l.after1 = l.after2 = l.after3 = 0x7fffffff;
+    l.gap1 = l.gap2 = l.gap3 = 0;
+    l.add_far = false;
+    return l;
+}
+
 // Launchers (stream-ordered, asynchronous).
+// Far-field pass of a launch; nothing when p.spj_near is null.  Runs after
+// reset_counters, before the pair kernel.
+cudaError_t launch_far(const Params& p, cudaStream_t s, int num_sms);
 cudaError_t launch_fp64(const Params& p, cudaStream_t s, int num_sms);
 cudaError_t launch_mixed(const Params& p, cudaStream_t s, int num_sms);
 cudaError_t launch_retest(const Params& p, cudaStream_t s, int num_sms);

@@ -1,0 +1,368 @@
+// Far-field pass: the force of distant superparticles on a walk's i-particles
+// through a local expansion about the walk centre (pgf_localexp.cuh), run
+// before the interaction kernel of the same launch.
+//
+// An EP-SP pair costs the interaction kernel 33 FP32 operations, and that
+// kernel is FP32-pipe bound.  A superparticle at distance D from a walk of
+// radius R (the farthest i from the walk centre) with R / D small acts on
+// all n_i particles through the same few derivatives of its field: expanding
+// it costs about 700 operations once, however many i there are.  On the 1M
+// binary Plummer workload 64% of the EP-SP pairs pass the test below (35% at
+// 65k stars, 45% in a King 1M model with theta = 0.4).
+//
+// Test.  A source is expanded when the first dropped terms, bounded for an i
+// at distance R straight towards it, stay below 2e-6 of the source's own
+// force: (P + 1) rho^P for the monopole (P = 8: rho = R / D <= 0.14) and
+// 84 rho^6 |Q| / (m D^2) for the quadrupole, whose terms end two orders
+// earlier.  Summed over a walk's sources, and away from that one direction,
+// the truncation is far below the FP32 rounding of the pair sums (1e-9 rms
+// of the force on Plummer and King models, against 7e-8).  The leading terms
+// (potential and uniform force) are summed as (hi, lo) FP32 pairs.
+//
+// One CTA of four warps per walk, from the same queue order as the
+// interaction kernel (a split walk is handled whole; its parts share the
+// compacted list).  Each warp takes a quarter of the list by itself: the near
+// ids are appended to the compacted list that the interaction kernel reads
+// instead, the far sources go to a ring in shared memory, and whenever 32 are
+// there every lane expands one into 81 coefficients in its registers.  The
+// lanes' coefficients are summed by a shuffle reduce-scatter, and each i
+// evaluates the polynomial; the sums go to the i's result row, to which the
+// interaction kernel adds its pairs.  The order of every sum is fixed by the
+// list, so results do not depend on the grid.
+//
+// Measured on GB300 at the 1M binary workload (all walks in one launch): the
+// pair kernel alone 22.9 ms; this pass 2.7 ms and the pair kernel 12.0 ms
+// after it, with the force error against FP64 at median 5.2e-8 / p99.9
+// 5.9e-7 from 7.0e-8 / 6.5e-7.  FP64 instructions are what costs here (the
+// FP64 pipe issues one per warp in 64 cycles): with the leading sums and the
+// results in FP64 the pass took 3.7 ms.
+#include "pgf_internal.cuh"
+#include "pgf_localexp.cuh"
+
+namespace pgf {
+namespace {
+
+constexpr int kWarps = 4;      // quarters of a list (SpjNear)
+constexpr int kT = kWarps * 32;
+constexpr int kRing = 64;      // per warp: 32 sources arrive while fewer than 32 wait
+constexpr int kMinI = 32;      // fewer i: direct pairs (33 n_i operations) cost about as much
+constexpr float kRhoMax = 0.14f;
+constexpr float kQuadTol = 2e-6f / 84.f;
+constexpr int kKeptI = 512;  // i whose coordinates stay in shared memory
+constexpr int kPad = 96;  // coefficients padded to 3 per lane
+
+struct FarSmem {
+    float src[kWarps][9][kRing];  // x, y, z, m, and the five quadrupole moments (QuadOp), scaled
+    float red[kWarps][kPad];
+    float2 lead[kWarps][4];  // rows 0 and 1 as (hi, lo)
+    float xi[3][kKeptI];      // the first i's coordinates, scaled
+    float c[2][3];            // walk centre (hi, lo)
+    float L[kFarCoefs + 3];
+    float4 ev[kFarCoefs + 3];  // phi and gradient coefficients
+    float rmax[kWarps];
+    int n_near[kWarps], n_far[kWarps];
+    int w;
+};
+
+__device__ __forceinline__ float rsqrt_approx_f(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+struct SpjRec {
+    float4 a, b, c;
+    float2 d;
+};
+__device__ __forceinline__ SpjRec load_spj(const SpjF32* __restrict__ spj, int id) {
+    SpjRec r{};
+    if (id >= 0) {
+        const float4* src = reinterpret_cast<const float4*>(spj + id);
+        r.a = __ldg(src);
+        r.b = __ldg(src + 1);
+        r.c = __ldg(src + 2);
+        r.d = __ldg(reinterpret_cast<const float2*>(src + 3));
+    }
+    return r;
+}
+
+// Sum of two (hi, lo) pairs.
+__device__ __forceinline__ float2 add_pair(float2 a, float2 b) {
+    float s, e;
+    two_sum_le(a.x, b.x, s, e);
+    return make_float2(s, e + (a.y + b.y));
+}
+
+// A shared-memory load that keeps its place: hoisted to the front, the 80
+// coefficients of the evaluation spill.
+__device__ __forceinline__ float4 ld_in_order(const float4* a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(static_cast<unsigned>(__cvta_generic_to_shared(a))));
+    return v;
+}
+
+// Rows N .. kFarOrder of the expansion at one i: adds phi and its gradient.
+template <int N>
+__device__ __forceinline__ void eval_rows(const float (&p1)[2 * kFarOrder + 1], const float (&p2)[2 * kFarOrder + 1],
+                                          float x, float y, float z, float r2, const float4* __restrict__ ev,
+                                          float4& o) {
+    if constexpr (N <= kFarOrder) {
+        float r[2 * kFarOrder + 1];
+        regular_row<N>(p1, p2, x, y, z, r2, r);
+#pragma unroll
+        for (int k = 0; k < 2 * N + 1; ++k) {
+            const float4 e = ld_in_order(ev + N * N + k);
+            o.w = fmaf(e.x, r[k], o.w);
+            if (N < kFarOrder) {
+                o.x = fmaf(e.y, r[k], o.x);
+                o.y = fmaf(e.z, r[k], o.y);
+                o.z = fmaf(e.w, r[k], o.z);
+            }
+        }
+        eval_rows<N + 1>(r, p1, x, y, z, r2, ev, o);
+    }
+}
+
+// One step of the reduce-scatter over lanes: the first H values of v become
+// this lane's half of the 2H summed with its partner's.
+template <int H>
+__device__ __forceinline__ void halve(float (&v)[kPad], int lane, int bit) {
+    const bool up = lane & bit;
+#pragma unroll
+    for (int k = 0; k < H; ++k) {
+        const float send = up ? v[k] : v[k + H];
+        const float keep = up ? v[k + H] : v[k];
+        v[k] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+    }
+}
+
+__global__ __launch_bounds__(kT, 3) void far_kernel(Params p) {
+    if (p.input_err && *p.input_err) return;  // the inputs failed their check: run nothing
+    __shared__ FarSmem s;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const unsigned lane_lt = (1u << lane) - 1u;
+    const int n_walk = p.n_root < p.n_walk ? p.n_root : walk_count(p);
+    for (;;) {
+        __syncthreads();
+        if (t == 0) s.w = atomicAdd(p.far_queue, 1);
+        __syncthreads();
+        if (s.w >= n_walk) break;
+        const int w = p.n_root < p.n_walk ? s.w : p.order[s.w];
+        const WalkDesc wd = p.walks[w];
+        const int n_spj = wd.n_spj_all;
+        if (wd.n_i < kMinI || n_spj == 0) {
+            if (t == 0) p.spj_near[w] = SpjNear{{-1, 0, 0, 0}, 0, {0, 0, 0}};
+            continue;
+        }
+        // Radius of the walk's particles.
+        float r2m = 0.f;
+        for (int i = t; i < wd.n_i; i += kT) {
+            const EpiDev e = p.epi[wd.i_begin + i];
+            const float x = (float)(e.x - wd.cx), y = (float)(e.y - wd.cy), z = (float)(e.z - wd.cz);
+            if (i < kKeptI) {
+                s.xi[0][i] = x;
+                s.xi[1][i] = y;
+                s.xi[2][i] = z;
+            }
+            r2m = fmaxf(r2m, fmaf(x, x, fmaf(y, y, z * z)));
+        }
+        if (t < 3) {
+            const double c = t == 0 ? wd.cx : (t == 1 ? wd.cy : wd.cz);
+            const float h = (float)c;
+            s.c[0][t] = h;
+            s.c[1][t] = (float)(c - (double)h);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) r2m = fmaxf(r2m, __shfl_xor_sync(0xffffffffu, r2m, o));
+        if (lane == 0) s.rmax[warp] = r2m;
+        __syncthreads();
+        r2m = fmaxf(fmaxf(s.rmax[0], s.rmax[1]), fmaxf(s.rmax[2], s.rmax[3]));
+        const float R = sqrtf(r2m) * 1.00001f;
+        if (!(R > 1e-18f && R < 1e18f)) {
+            if (t == 0) p.spj_near[w] = SpjNear{{-1, 0, 0, 0}, 0, {0, 0, 0}};
+            continue;
+        }
+        // Lengths in units of a power of two at the nearest distance expanded,
+        // so that the powers of D and x stay in FP32's range.
+        int ex;
+        (void)frexpf(R / kRhoMax, &ex);
+        const float inv = ldexpf(1.f, -ex);
+        const float Rs = R * inv;  // in (0.07, 0.14]
+        const float lim2 = (Rs / kRhoMax) * (Rs / kRhoMax);
+        const float kq = (Rs * Rs * Rs) * (Rs * Rs * Rs) / kQuadTol;
+        const float chx = s.c[0][0], chy = s.c[0][1], chz = s.c[0][2];
+        const float clx = s.c[1][0], cly = s.c[1][1], clz = s.c[1][2];
+
+        float L[kFarCoefs], lo[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int k = 0; k < kFarCoefs; ++k) L[k] = 0.f;
+        // Each warp takes a quarter of the list by itself: 32 entries at a
+        // time, with the records loaded one chunk ahead and the ids two.
+        const int b0 = (int)((int64_t)n_spj * warp / kWarps), n_w = (int)((int64_t)n_spj * (warp + 1) / kWarps) - b0;
+        const int32_t* __restrict__ ids = p.id_spj + wd.spj_begin + b0;
+        int32_t* __restrict__ near_out = p.id_spj_near + wd.spj_begin + b0;
+        float (*const src)[kRing] = s.src[warp];
+        int head = 0, waiting = 0, n_near = 0, n_far = 0;
+        int id = lane < n_w ? __ldg(ids + lane) : -1;
+        int id_next = 32 + lane < n_w ? __ldg(ids + 32 + lane) : -1;
+        SpjRec rec = load_spj(p.spj32, id);
+        for (int base = 0; base < n_w || waiting > 0; base += 32) {
+            if (base < n_w) {
+                const float hx = ((rec.a.x - chx) + (rec.b.x - clx)) * inv;
+                const float hy = ((rec.a.y - chy) + (rec.b.y - cly)) * inv;
+                const float hz = ((rec.a.z - chz) + (rec.b.z - clz)) * inv;
+                const float m = rec.a.w;
+                const float i2 = inv * inv;
+                const QuadOp q = quad_op(rec.c.x * i2, rec.c.y * i2, rec.c.z * i2, rec.c.w * i2, rec.d.x * i2, rec.d.y * i2);
+                const float qn = sqrtf(fmaf(rec.c.x, rec.c.x, fmaf(rec.c.y, rec.c.y, rec.c.z * rec.c.z)) +
+                                       2.f * fmaf(rec.c.w, rec.c.w, fmaf(rec.d.x, rec.d.x, rec.d.y * rec.d.y))) * i2;
+                const float d2 = fmaf(hx, hx, fmaf(hy, hy, hz * hz));
+                const float d4 = d2 * d2;
+                const bool valid = id >= 0;
+                const bool far = valid && d2 >= lim2 && d2 < 1e16f && fabsf(m) < 1e30f && qn * kq <= fabsf(m) * (d4 * d4);
+                const int id_cur = id;
+                id = id_next;
+                id_next = base + 64 + lane < n_w ? __ldg(ids + base + 64 + lane) : -1;
+                rec = load_spj(p.spj32, id);
+                const unsigned bf = __ballot_sync(0xffffffffu, far);
+                const unsigned bn = __ballot_sync(0xffffffffu, valid && !far);
+                if (far) {
+                    const int e = (head + waiting + __popc(bf & lane_lt)) & (kRing - 1);
+                    src[0][e] = hx;
+                    src[1][e] = hy;
+                    src[2][e] = hz;
+                    src[3][e] = m;
+                    src[4][e] = q.ppr;
+                    src[5][e] = q.ppi;
+                    src[6][e] = q.pzr;
+                    src[7][e] = q.pzi;
+                    src[8][e] = q.zz;
+                } else if (valid) {
+                    near_out[n_near + __popc(bn & lane_lt)] = id_cur;
+                }
+                const int nf = __popc(bf);
+                waiting += nf;
+                n_far += nf;
+                n_near += __popc(bn);
+                __syncwarp();
+                if (waiting < 32 && base + 32 < n_w) continue;
+            }
+            if (waiting == 0) break;
+            // One source per lane (fewer in the last batch).
+            float hx = 1.f, hy = 0.f, hz = 0.f, m = 0.f;
+            QuadOp q{};
+            if (lane < waiting) {
+                const int e = (head + lane) & (kRing - 1);
+                hx = src[0][e];
+                hy = src[1][e];
+                hz = src[2][e];
+                m = src[3][e];
+                q.ppr = src[4][e];
+                q.ppi = src[5][e];
+                q.pzr = src[6][e];
+                q.pzi = src[7][e];
+                q.zz = src[8][e];
+            }
+            __syncwarp();  // the ring's slots may be written again
+            const int take = min(32, waiting);
+            head = (head + take) & (kRing - 1);
+            waiting -= take;
+            const float ri = rsqrt_approx_f(fmaf(hx, hx, fmaf(hy, hy, hz * hz)));
+            add_source(hx, hy, hz, ri, m, q, L, lo);
+        }
+        if (lane == 0) {
+            s.n_near[warp] = n_near;
+            s.n_far[warp] = n_far;
+        }
+        __syncthreads();
+        n_far = (s.n_far[0] + s.n_far[1]) + (s.n_far[2] + s.n_far[3]);
+        if (t == 0)
+            p.spj_near[w] = SpjNear{{s.n_near[0], s.n_near[1], s.n_near[2], s.n_near[3]}, n_far > 0 ? 1 : 0, {0, 0, 0}};
+        if (n_far == 0) continue;
+
+        // Sum over the threads: rows 0 and 1 in FP64, the others by a
+        // reduce-scatter (lane l ends with three coefficients).
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            float2 v = make_float2(L[k], lo[k]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                v = add_pair(v, make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o)));
+            if (lane == 0) s.lead[warp][k] = v;
+        }
+        {
+            float v[kPad];
+#pragma unroll
+            for (int k = 0; k < kPad; ++k) v[k] = k < kFarCoefs ? L[k] : 0.f;
+            halve<48>(v, lane, 16);
+            halve<24>(v, lane, 8);
+            halve<12>(v, lane, 4);
+            halve<6>(v, lane, 2);
+            halve<3>(v, lane, 1);
+            const int b = (lane & 16 ? 48 : 0) + (lane & 8 ? 24 : 0) + (lane & 4 ? 12 : 0) + (lane & 2 ? 6 : 0) +
+                          (lane & 1 ? 3 : 0);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) s.red[warp][b + k] = v[k];
+        }
+        __syncthreads();
+        if (t < kFarCoefs) s.L[t] = (s.red[0][t] + s.red[1][t]) + (s.red[2][t] + s.red[3][t]);
+        __syncthreads();
+        if (t < kFarCoefs) {
+            int n = 0;
+            while ((n + 1) * (n + 1) <= t) ++n;
+            float4 e;
+            eval_coef(n, t - n * n, [&](int i) { return s.L[i]; }, e.x, e.y, e.z, e.w);
+            s.ev[t] = e;
+        }
+        float2 lead[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            lead[k] = add_pair(add_pair(s.lead[0][k], s.lead[1][k]), add_pair(s.lead[2][k], s.lead[3][k]));
+        __syncthreads();
+        const float inv2 = inv * inv;  // powers of two: scaling the results is exact
+#pragma unroll 1
+        for (int i = t; i < wd.n_i; i += kT) {
+            const int gi = wd.i_begin + i;
+            float x, y, z;
+            if (i < kKeptI) {
+                x = s.xi[0][i] * inv;
+                y = s.xi[1][i] * inv;
+                z = s.xi[2][i] * inv;
+            } else {
+                const EpiDev e = p.epi[gi];
+                x = (float)(e.x - wd.cx) * inv;
+                y = (float)(e.y - wd.cy) * inv;
+                z = (float)(e.z - wd.cz) * inv;
+            }
+            float r0[2 * kFarOrder + 1] = {1.f}, rz[2 * kFarOrder + 1] = {};
+            float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+            eval_rows<1>(r0, rz, x, y, z, fmaf(x, x, fmaf(y, y, z * z)), s.ev, o);
+            // rows 0: phi = L_00, gradient (Re L_11, Im L_11, L_10)
+            const float2 ax = add_pair(lead[2], make_float2(o.x, 0.f)), ay = add_pair(lead[3], make_float2(o.y, 0.f));
+            const float2 az = add_pair(lead[1], make_float2(o.z, 0.f)), ph = add_pair(lead[0], make_float2(o.w, 0.f));
+            float4* out = reinterpret_cast<float4*>(p.out_accp + gi);
+            out[0] = make_float4(ax.x * inv2, ax.y * inv2, ay.x * inv2, ay.y * inv2);
+            out[1] = make_float4(az.x * inv2, az.y * inv2, -ph.x * inv, -ph.y * inv);
+        }
+    }
+}
+
+}  // namespace
+
+cudaError_t launch_far(const Params& p, cudaStream_t s, int num_sms) {
+    if (!p.spj_near || p.n_walk <= 0) return cudaSuccess;
+    static int per_sm = 0;
+    if (per_sm == 0) {
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, far_kernel, kT, 0);
+        if (e != cudaSuccess) return e;
+        if (per_sm < 1) per_sm = 1;
+    }
+    int grid = num_sms * per_sm;
+    if (grid > p.n_walk) grid = p.n_walk;
+    far_kernel<<<grid, kT, 0, s>>>(p);
+    return cudaGetLastError();
+}
+
+}  // namespace pgf

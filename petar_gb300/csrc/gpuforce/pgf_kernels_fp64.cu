@@ -133,11 +133,9 @@ __global__ __launch_bounds__(kT) void fp64_kernel(Params p) {
 }  // namespace
 
 cudaError_t launch_fp64(const Params& p, cudaStream_t s, int num_sms) {
-    cudaError_t e = cudaMemsetAsync(p.queue_head, 0, sizeof(int32_t), s);
-    if (e != cudaSuccess) return e;
     if (p.n_walk <= 0) return cudaSuccess;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fp64_kernel, kT, 0);
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fp64_kernel, kT, 0);
     if (e != cudaSuccess) return e;
     int grid = num_sms * (per_sm > 0 ? per_sm : 1);
     if (grid > p.n_walk) grid = p.n_walk;

@@ -140,6 +140,7 @@ __global__ __launch_bounds__(kThreadsG, 2) void gradient_kernel_pk(Params p) {
         const int wq = s.w;
         if (wq >= n_walk) break;
         const WalkDesc wd = p.walks[p.order[wq]];
+        const SpjList spj = spj_list(p, wd);
         const float chx = (float)wd.cx, chy = (float)wd.cy, chz = (float)wd.cz;
         const float clx = (float)(wd.cx - (double)chx), cly = (float)(wd.cy - (double)chy),
                     clz = (float)(wd.cz - (double)chz);
@@ -416,11 +417,11 @@ __global__ __launch_bounds__(kThreadsG, 2) void gradient_kernel_pk(Params p) {
                 }
             }
             // SPJ tiles: the quadrupole force.
-            for (int t = 0; t < wd.n_spj; t += kTileSPG) {
-                const int nt = min(kTileSPG, wd.n_spj - t);
+            for (int t = 0; t < spj.n; t += kTileSPG) {
+                const int nt = min(kTileSPG, spj.n - t);
                 __syncthreads();
                 if (tid < nt) {
-                    const int id = p.id_spj[wd.spj_begin + t + tid];
+                    const int id = *spj.at(t + tid);
                     const SpjF32 r = p.spj32[id];
                     float* f = reinterpret_cast<float*>(&s.S[tid >> 1][0]) + (tid & 1);
                     f[0] = (r.xh - chx) + (r.xl - clx);
@@ -499,6 +500,11 @@ __global__ __launch_bounds__(kThreadsG, 2) void gradient_kernel_pk(Params p) {
 #pragma unroll
                         for (int c = 0; c < 7; ++c) r[c] += (double)s.acc[k][c][src].x + (double)s.acc[k][c][src].y;
                     }
+                    if (spj.add_far) {  // the far-field pass's sums
+                        double f[4];
+                        far_sum(p, gi, f);
+                        for (int c = 0; c < 4; ++c) r[3 + c] += f[c];
+                    }
                     // a_i once: parts of a split walk add their pairs only
                     const Accp a = wd.part == 0 ? p.epi_acc64[gi] : Accp{0.0, 0.0, 0.0, 0.0};
                     const double G = p.G;
@@ -535,9 +541,7 @@ cudaError_t launch_gradient_t(const Params& p, cudaStream_t s, int num_sms) {
 }  // namespace
 
 cudaError_t launch_gradient(const Params& p, cudaStream_t s, int num_sms) {
-    cudaError_t e = cudaMemsetAsync(p.queue_head, 0, sizeof(int32_t), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(p.n_retest, 0, sizeof(int32_t), s);
-    if (e != cudaSuccess || p.n_walk <= 0) return e;
+    if (p.n_walk <= 0) return cudaSuccess;
     return p.gr_compensated ? launch_gradient_t<true>(p, s, num_sms) : launch_gradient_t<false>(p, s, num_sms);
 }
 

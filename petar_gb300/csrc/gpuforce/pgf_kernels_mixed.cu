@@ -561,10 +561,8 @@ __global__ __launch_bounds__(256) void retest_kernel(Params p) {
 }  // namespace
 
 cudaError_t launch_mixed(const Params& p, cudaStream_t s, int num_sms) {
-    cudaError_t e = cudaMemsetAsync(p.queue_head, 0, sizeof(int32_t), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(p.n_retest, 0, sizeof(int32_t), s);
-    if (e != cudaSuccess) return e;
     if (p.n_walk <= 0) return cudaSuccess;
+    cudaError_t e;
     static int per_sm = 0;
     if (per_sm == 0) {
         e = cudaFuncSetAttribute(mixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));

@@ -383,7 +383,9 @@ __device__ void producer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
         const float rsmax2 = wd.rs_max * wd.rs_max;
         const float hmax = fmaxf(wd.hx, fmaxf(wd.hy, wd.hz));
         const int n_ept = (wd.n_epj + kTileEP - 1) / kTileEP;
-        const int n_spt = SR ? 0 : (wd.n_spj + kTileSP - 1) / kTileSP;
+        const SpjList spj = SR ? SpjList{} : spj_list(p, wd);
+        const int n_spj = spj.n;
+        const int n_spt = (n_spj + kTileSP - 1) / kTileSP;
         const int n_tiles = n_ept + n_spt;
         // TMA staging: tile u (EP tiles, then SP tiles) is gathered into
         // stage[u & 1] while tile u - 1 is converted.  Lane l gathers entries
@@ -396,16 +398,15 @@ __device__ void producer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
                 // the buffer's previous contents were read through the generic proxy
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 const int t = ep ? u : u - n_ept;
-                const int64_t base = ep ? wd.epj_begin + (int64_t)t * kTileEP : wd.spj_begin + (int64_t)t * kTileSP;
-                const int nt = ep ? min(kTileEP, wd.n_epj - t * kTileEP) : min(kTileSP, wd.n_spj - t * kTileSP);
-                const int32_t* ids = ep ? p.id_epj : p.id_spj;
+                const int64_t base = ep ? wd.epj_begin + (int64_t)t * kTileEP : (int64_t)t * kTileSP;
+                const int nt = ep ? min(kTileEP, wd.n_epj - t * kTileEP) : min(kTileSP, n_spj - t * kTileSP);
                 const int n_lanes = ep ? kTileEP / 4 : kTileSP / 4;
                 int r[4] = {0, 0, 0, 0};
                 if (lane < n_lanes) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const int e = 4 * lane + j;
-                        r[j] = e < nt ? ld_streamed(ids + base + e, stream_pol) : 0;
+                        r[j] = e < nt ? ld_streamed(ep ? p.id_epj + base + e : spj.at((int)base + e), stream_pol) : 0;
                     }
                 }
                 if (lane == 0) mbar_arrive_expect_tx(&s.tm.bar[b], 4096u);
@@ -562,8 +563,8 @@ __device__ void producer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
             }
             // SPJ tiles: 64-byte records, QSB entries per lane at a time.
             for (int t = 0; t < n_spt; ++t) {
-                const int64_t base = wd.spj_begin + (int64_t)t * kTileSP;
-                const int nt = min(kTileSP, wd.n_spj - t * kTileSP);
+                const int64_t base = (int64_t)t * kTileSP;
+                const int nt = min(kTileSP, n_spj - t * kTileSP);
                 if constexpr (TM) {
                     const int u = n_ept + t;
                     if (u + 1 < n_tiles) tm_issue(u + 1);
@@ -585,7 +586,7 @@ __device__ void producer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
 #pragma unroll
                     for (int qq = 0; qq < QSB; ++qq) {
                         const int e = (qb + qq) * 32 + lane;
-                        id[qq] = e < nt ? ld_streamed(p.id_spj + base + e, stream_pol) : -1;
+                        id[qq] = e < nt ? ld_streamed(spj.at((int)base + e), stream_pol) : -1;
                     }
 #pragma unroll
                     for (int qq = 0; qq < QSB; ++qq) {
@@ -690,7 +691,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
     // leaves fewer lanes idle; the tile bodies are instantiated for both.
     float rcut2 = 0.f;
     int nip = 0, S = 1, n_js = 1, js = 0, slot = 0, ku = KI, gbase = 0;
-    bool active = false;
+    bool active = false, add_far = false;
     // Scalar path: i coordinates and accumulators a[0..2] acceleration, a[3]
     // potential.  Packed path: (-x_i, -x_i) operands and pair accumulators
     // b[0..2] acceleration, b[3] minus the potential.
@@ -897,6 +898,9 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
             }
 #pragma unroll
             for (int k = 0; k < KU; ++k) s.cnt[k][ct] += c[k];
+            // A close neighbour's term can exceed the whole rest of the sum:
+            // what follows must not be rounded against it.
+            if constexpr (!SR) flush();
         }
         int nfar = 0;
         if constexpr (SR) {
@@ -958,7 +962,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
             }
             nfar = f1 - f0;
         }
-        since += (j1 - j0) + nfar;
+        since += nfar;
     };
 
     // One SPJ tile with KU i-particles per thread.
@@ -1067,6 +1071,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
             slot = ct - js * S;
             active = js < n_js;
             gbase = wd.i_begin + h.ipass + slot;
+            if constexpr (!SR) add_far = spj_list(p, wd).add_far;
             if constexpr (CO) {
                 r_out_walk = sqrt(wd.rcut2);
                 rcut2d = wd.rcut2;
@@ -1155,6 +1160,11 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
                         n += s.cnt[k][src];
                     }
                     const int gi = gbase + k * S;
+                    if (!SR && add_far) {  // the far-field pass's sums
+                        double f[4];
+                        far_sum(p, gi, f);
+                        for (int c = 0; c < 4; ++c) r[c] += f[c];
+                    }
                     if constexpr (CO) {
                         // self-potential G m / r_out removed (src/hard.hpp:1663-1674)
                         const double self = self_scale * (double)s.co.coi[k][slot].mass / r_out_walk;
@@ -1201,10 +1211,8 @@ __global__ __launch_bounds__((CW + 1) * 32, MINB) void ws_kernel(Params p, const
 
 template <int CW, int KI, int MINB, bool PK, int MD = kModeForce, int TE = 128, int NS = 4, bool TM = false>
 cudaError_t launch_ws_t(const Params& p, cudaStream_t st, int num_sms, const TensorMaps* tm = nullptr) {
-    cudaError_t e = cudaMemsetAsync(p.queue_head, 0, sizeof(int32_t), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(p.n_retest, 0, sizeof(int32_t), st);
-    if (e != cudaSuccess) return e;
     if (p.n_walk <= 0) return cudaSuccess;
+    cudaError_t e;
     static int per_sm = 0;
     const size_t smem = sizeof(Smem<CW, KI, PK, TE, NS, MD, TM>);
     static const CUtensorMap none{};

@@ -1080,7 +1080,9 @@ __global__ __launch_bounds__(128) void group_reduce_kernel(TreeHdr* h, const TCe
         d.rs_max = gc.rs_max;
         d.rcut2 = rcut2;
         d.part = 0;
-        d.pad[0] = d.pad[1] = d.pad[2] = 0.f;
+        d.n_parts = 1;
+        d.root = (int32_t)g;
+        d.n_spj_all = ns;
         walks[g] = d;
         cnt_e[g] = ne;
         cnt_s[g] = ns;
@@ -1461,10 +1463,12 @@ struct pgf_nbody {
     DArr<WalkDesc> walks;
     int64_t cap_e = 0, cap_s = 0;
     DArr<int32_t> id_epj, id_spj;
+    DArr<int32_t> id_spj_near;  // far-field pass (far_applies): the compacted lists and their lengths
+    DArr<SpjNear> spj_near;
     // force scratch and results
     DArr<Accp> out_accp;
     DArr<int32_t> out_nnb;
-    DArr<int32_t> flags;  // [0] queue head, [1] n_retest, [2] kernel error word
+    DArr<int32_t> flags;  // [2] kernel error word, [4..6] launch counters
     DArr<Retest> retest;
     int retest_cap = 1 << 20;
     DArr<TreeHdr> hdr;
@@ -1565,13 +1569,15 @@ cudaError_t enqueue_build(pgf_nbody* h) {
 }
 
 cudaError_t enqueue_force(pgf_nbody* h) {
-    if (h->cfg.precision == PGF_PRECISION_FP64) {
-        cudaError_t e = launch_fp64(h->p, h->stream, h->num_sms);
-        if (e == cudaSuccess) e = cudaMemsetAsync(h->p.n_retest, 0, sizeof(int32_t), h->stream);
-        return e;
+    cudaError_t e = reset_counters(h->p, h->stream);
+    if (e != cudaSuccess) return e;
+    if (h->cfg.precision == PGF_PRECISION_FP64) return launch_fp64(h->p, h->stream, h->num_sms);
+    if (h->variant == 0) {
+        e = launch_mixed(h->p, h->stream, h->num_sms);
+    } else {
+        e = launch_far(h->p, h->stream, h->num_sms);
+        if (e == cudaSuccess) e = launch_ws(h->p, h->stream, h->num_sms, h->variant - 1, nullptr);
     }
-    cudaError_t e = h->variant == 0 ? launch_mixed(h->p, h->stream, h->num_sms)
-                                    : launch_ws(h->p, h->stream, h->num_sms, h->variant - 1, nullptr);
     if (e == cudaSuccess) e = launch_retest(h->p, h->stream, h->num_sms);
     return e;
 }
@@ -1633,13 +1639,17 @@ void bind_params(pgf_nbody* h) {
     p.walks = h->walks.d;
     p.order = h->queue.d;
     p.n_walk = (int32_t)h->n;  // capacity; the build writes the count
+    p.n_root = p.n_walk;
     p.n_walk_dev = &h->hdr.d->n_walk;
     p.eps2 = h->cfg.eps2;
     p.G = h->cfg.G;
     p.out_accp = h->out_accp.d;
     p.out_nnb = h->out_nnb.d;
-    p.queue_head = h->flags.d;
-    p.n_retest = h->flags.d + 1;
+    bind_counters(p, h->flags.d + 4);
+    if (far_applies(h->cfg.eps2, h->n)) {
+        p.id_spj_near = h->id_spj_near.d;
+        p.spj_near = h->spj_near.d;
+    }
     p.err = h->flags.d + 2;
     p.retest = h->retest.d;
     p.retest_cap = h->retest_cap;
@@ -1663,6 +1673,12 @@ cudaError_t alloc_tasks(pgf_nbody* h, int64_t cap) {
     h->cap_tasks = cap;
     cudaError_t e = h->task_e.alloc(cap);
     if (e == cudaSuccess) e = h->task_s.alloc(cap);
+    return e;
+}
+
+cudaError_t alloc_spj(pgf_nbody* h) {
+    cudaError_t e = h->id_spj.alloc(h->cap_s);
+    if (e == cudaSuccess && far_applies(h->cfg.eps2, h->n)) e = h->id_spj_near.alloc(h->cap_s);
     return e;
 }
 
@@ -1702,7 +1718,7 @@ int build_fit(pgf_nbody* h) {
             const double ts = f * (double)t.n_spj_entries + 1024;
             if (off((double)h->cap_s, ts)) {
                 h->cap_s = (int64_t)std::ceil(ts);
-                NB_CUDA(h->id_spj.alloc(h->cap_s));
+                NB_CUDA(alloc_spj(h));
                 resized = true;
             }
             const double tt = f * (double)t.n_groups * (double)((t.n_fronts + kChunk - 1) / kChunk) + 1024;
@@ -1728,7 +1744,7 @@ int build_fit(pgf_nbody* h) {
         }
         if (t.err & kErrSpj) {
             h->cap_s = (int64_t)(f * (double)t.n_spj_entries) + 1024;
-            NB_CUDA(h->id_spj.alloc(h->cap_s));
+            NB_CUDA(alloc_spj(h));
         }
         if (t.err & kErrTasks)
             NB_CUDA(alloc_tasks(h, (int64_t)(f * (double)t.n_groups * (double)((t.n_fronts + kChunk - 1) / kChunk)) + 1024));
@@ -1811,7 +1827,8 @@ int pgf_nbody_create(const pgf_nbody_config* cfg, int64_t n, const double* pos, 
     h->cap_e = 8 * n + 1024;  // first guesses; the first build sizes them
     h->cap_s = 8 * n + 1024;
     NB_TRY(h->id_epj.alloc(h->cap_e));
-    NB_TRY(h->id_spj.alloc(h->cap_s));
+    NB_TRY(alloc_spj(h));
+    if (far_applies(cfg->eps2, n)) NB_TRY(h->spj_near.alloc(n));
     NB_TRY(h->blocksum.alloc(kLevelBlocks));
     NB_TRY(h->out_accp.alloc(n));
     NB_TRY(h->out_nnb.alloc(n));

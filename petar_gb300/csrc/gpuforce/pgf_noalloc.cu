@@ -30,7 +30,7 @@ constexpr int kMaxWalks = PGF_NOALLOC_MAX_WALKS;
 constexpr int kRetestCap = 1 << 16;
 constexpr int kMaxDevices = 64;
 constexpr size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
-constexpr size_t kFlagsOff = 0;  // [0] queue cursor, [1] re-test count, [2] error bits
+constexpr size_t kFlagsOff = 0;  // [2] error bits, [4..6] launch counters
 constexpr size_t kDescOff = 256;
 constexpr size_t kOrderOff = align256(kDescOff + sizeof(WalkDesc) * kMaxWalks);
 constexpr size_t kRetestOff = align256(kOrderOff + sizeof(int32_t) * kMaxWalks);
@@ -137,7 +137,9 @@ __global__ __launch_bounds__(128) void walk_prep_kernel(int n_walk, const int64_
             d.hx = d.hy = d.hz = d.rs_max = 0.f;
         }
         d.part = 0;
-        d.pad[0] = d.pad[1] = d.pad[2] = 0.f;
+        d.n_parts = 1;
+        d.root = w;
+        d.n_spj_all = d.n_spj;
         d.rcut2 = rcut2;
         desc[w] = d;
         order[w] = w;
@@ -236,12 +238,12 @@ extern "C" int pgf_force_device_noalloc(int n_walk, const int64_t* walk_table, c
     p.G = G;
     p.out_accp = reinterpret_cast<Accp*>(accp);
     p.out_nnb = n_ngb;
-    p.queue_head = flags;
-    p.n_retest = flags + 1;
+    bind_counters(p, flags + 4);
     p.retest = retest;
     p.retest_cap = kRetestCap;
     p.err = flags + 2;
-    e = launch_mixed(p, s, g_num_sms[dev]);
+    e = reset_counters(p, s);
+    if (e == cudaSuccess) e = launch_mixed(p, s, g_num_sms[dev]);
     if (e == cudaSuccess) e = launch_retest(p, s, g_num_sms[dev]);
     if (e != cudaSuccess) return fail(errbuf, errbuf_len, PGF_ERR_CUDA, "pgf_force_device_noalloc: launch: %s", cudaGetErrorString(e));
     return PGF_OK;
