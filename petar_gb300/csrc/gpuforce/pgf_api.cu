@@ -112,6 +112,7 @@ struct TagState {
     std::vector<int> n_epi;
     std::vector<int64_t> epi_disp;
     DevBuf<EpiDev> epi;
+    DevBuf<EpiRel> epi_rel;
     DevBuf<int32_t> id_epj, id_spj, order;
     DevBuf<int32_t> id_spj_near;  // far-field pass: Params::id_spj_near, spj_near
     DevBuf<SpjNear> spj_near;
@@ -644,7 +645,7 @@ bool runs_far(const TagState& t) {
 }
 
 // Main kernel of the tag's precision and variant on stream s, bracketed by two
-// events, then the FP64 neighbour re-test.
+// events, then the FP64 neighbour re-test of the CTA-synchronous kernel.
 int launch_kernels(const TagState& t, const Params& p, cudaStream_t s, cudaEvent_t ev_start, cudaEvent_t ev_end) {
     PGF_CUDA(cudaEventRecord(ev_start, s));
     cudaError_t e = reset_counters(p, s);
@@ -656,18 +657,16 @@ int launch_kernels(const TagState& t, const Params& p, cudaStream_t s, cudaEvent
     } else if (t.mode == PGF_MODE_FORCE_CHANGEOVER) {
         e = launch_ws_changeover(p, s, g.num_sms);
         if (e == cudaSuccess) e = cudaEventRecord(ev_end, s);
-        if (e == cudaSuccess && p.n_walk > 0) e = launch_retest(p, s, g.num_sms);
     } else if (t.mode == PGF_MODE_NEIGHBOR_SEARCH) {
         e = launch_ws_search(p, s, g.num_sms);
         if (e == cudaSuccess) e = cudaEventRecord(ev_end, s);
-        if (e == cudaSuccess && p.n_walk > 0) e = launch_retest(p, s, g.num_sms);
     } else if (t.precision == PGF_PRECISION_FP64) {
         e = launch_fp64(p, s, g.num_sms);
         if (e == cudaSuccess) e = cudaEventRecord(ev_end, s);
     } else {
         e = t.variant == 0 ? launch_mixed(p, s, g.num_sms) : launch_ws(p, s, g.num_sms, t.variant - 1, &g.tmaps);
         if (e == cudaSuccess) e = cudaEventRecord(ev_end, s);
-        if (e == cudaSuccess && p.n_walk > 0) e = launch_retest(p, s, g.num_sms);
+        if (e == cudaSuccess && t.variant == 0 && p.n_walk > 0) e = launch_retest(p, s, g.num_sms);
     }
     if (e != cudaSuccess) return fail(PGF_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
     return PGF_OK;
@@ -678,8 +677,10 @@ int launch_tag(TagState& t) {
     bind_scratch(t.params);
     if (int r = launch_kernels(t, t.params, g.stream, t.ev[1], t.ev[2])) return r;
     if (t.n_split > 0) {
+        const bool pairs = t.mode == PGF_MODE_FORCE_CHANGEOVER || t.mode == PGF_MODE_NEIGHBOR_SEARCH ||
+                           (t.mode == PGF_MODE_FORCE && t.precision == PGF_PRECISION_MIXED && t.variant != 0);
         const cudaError_t e = launch_combine_parts(t.splits.d, t.n_split, t.params.out_accp, t.params.out_nnb,
-                                                   t.params.out_pot_soft, t.params.out_acorr, g.stream);
+                                                   t.params.out_pot_soft, t.params.out_acorr, pairs, t.params.G, g.stream);
         if (e != cudaSuccess) return fail(PGF_ERR_CUDA, "combine kernel failed: %s", cudaGetErrorString(e));
     }
     PGF_CUDA(cudaEventRecord(t.ev[3], g.stream));
@@ -796,6 +797,7 @@ bool pack_walk(TagState& t, int k, int w, const Slot3& o, const void* const* epi
     }
     d.part = 0;
     d.n_parts = 1;
+    d.i_root = d.i_begin;
     d.root = k;
     d.n_spj_all = n_spj[w];
     d.rcut2 = g.walk_rcut2.empty() ? g.rcut2 : g.walk_rcut2[w];
@@ -807,7 +809,7 @@ bool pack_walk(TagState& t, int k, int w, const Slot3& o, const void* const* epi
 // A walk of a single-launch dispatch that runs as several parts.
 struct SplitPlan {
     int k, parts;
-    int64_t rows1;  // first EPI row of part 1
+    int64_t rows1;  // first result row of part 1
     int desc1;      // layout position of part 1's descriptor
 };
 
@@ -925,6 +927,8 @@ int dispatch_host_direct(TagState& t, int n_walk, const std::vector<int32_t>& or
     a.n_epj_tot = g.n_epj_tot;
     a.n_spj_tot = g.n_spj_tot;
     a.out_epi = t.epi.d;
+    a.out_epi_rel = t.epi_rel.d;
+    a.eps2 = (float)t.params.eps2;
     a.out_id_epj = t.id_epj.d;
     a.out_id_spj = t.id_spj.d;
     a.out_walks = t.walks.d;
@@ -1024,8 +1028,7 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
     // of one SM's even share of the dispatch's cost; each walk that costs
     // more than a unit runs as parts of at most a unit (at most 16 parts, at
     // least 256 list entries each), each with a slice of its EPJ and SPJ
-    // lists and its own copy of the walk's EPI rows (made on the device), and
-    // a combine kernel adds the parts up.  The kernels add per-i terms
+    // lists and result rows of its own, and a combine kernel adds the parts up.  The kernels add per-i terms
     // (changeover self-potential, the gradient pass's a_i) in part 0 only.
     // On 200-walk batches of the 1M binary Plummer workload an eighth ran
     // the kernels 24% faster than parts of a quarter share split only above
@@ -1057,12 +1060,12 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
     t.n_split = 0;
     if (gr_mode) {
         if (!hd_single) PGF_CUDA(t.h_epi_acc.ensure(ni));
-        PGF_CUDA(t.epi_acc.ensure(ni_all));
+        PGF_CUDA(t.epi_acc.ensure(ni));
         PGF_CUDA(t.acorr.ensure(ni_all));
     }
     if (co_mode) {
         if (!hd_single) PGF_CUDA(t.h_epi_co.ensure(ni));
-        PGF_CUDA(t.epi_co.ensure(ni_all));
+        PGF_CUDA(t.epi_co.ensure(ni));
         PGF_CUDA(t.pot_soft.ensure(ni_all));
     }
 
@@ -1073,7 +1076,8 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
         PGF_CUDA(t.h_walks.ensure(n_desc));
     }
     PGF_CUDA(t.h_order.ensure(n_desc));
-    PGF_CUDA(t.epi.ensure(ni_all));
+    PGF_CUDA(t.epi.ensure(ni));
+    PGF_CUDA(t.epi_rel.ensure(ni));
     PGF_CUDA(t.id_epj.ensure(ne));
     PGF_CUDA(t.id_spj.ensure(ns));
     const bool far = far_applies(g.eps2, ni) && ns > 0 && t.mode != PGF_MODE_NEIGHBOR_SEARCH;
@@ -1101,6 +1105,7 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
     Params& p = t.params;
     p = Params{};
     p.epi = t.epi.d;
+    p.epi_rel = t.epi_rel.d;
     p.epj = g.epj.d;
     p.epj_m64 = g.epj_m64.d;
     p.epj_rs64 = g.epj_rs64.d;
@@ -1207,15 +1212,14 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
                     d.n_epj = e1 - e0;
                     d.spj_begin = d0.spj_begin + s0;
                     d.n_spj = s1 - s0;
-                    d.n_parts = sp.parts;
+                    d.n_parts = (uint16_t)sp.parts;
                     if (j == 0) {
                         t.h_walks.h[sp.k] = d;
                         continue;
                     }
-                    // Part j reads a copy of the walk's rows, made on the
-                    // device after the copies (launch_split_rows).
+                    // Part j writes result rows of its own.
                     d.i_begin = (int32_t)(sp.rows1 + (int64_t)(j - 1) * d0.n_i);
-                    d.part = j;
+                    d.part = (uint16_t)j;
                     t.h_walks.h[sp.desc1 + j - 1] = d;
                 }
                 t.h_splits.h[q] = SplitRec{d0.i_begin, (int32_t)sp.rows1, d0.n_i, sp.parts};
@@ -1238,10 +1242,11 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
                                      g.stream));
             PGF_CUDA(cudaMemcpyAsync(t.splits.d, t.h_splits.h, plan.size() * sizeof(SplitRec),
                                      cudaMemcpyHostToDevice, g.stream));
-            const cudaError_t e = launch_split_rows(t.splits.d, (int)plan.size(), t.epi.d, co_mode ? t.epi_co.d : nullptr,
-                                                    gr_mode ? t.epi_acc.d : nullptr, g.stream);
-            if (e != cudaSuccess) return fail(PGF_ERR_CUDA, "split rows kernel failed: %s", cudaGetErrorString(e));
             t.n_split = (int)plan.size();
+        }
+        {
+            const cudaError_t e = launch_epi_rel(t.params, t.epi_rel.d, g.stream, g.num_sms);
+            if (e != cudaSuccess) return fail(PGF_ERR_CUDA, "EPI row kernel failed: %s", cudaGetErrorString(e));
         }
         return launch_tag(t);
     }
@@ -1280,6 +1285,10 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
         pc.order = t.order.d + k0;
         pc.n_walk = pc.n_root = k1 - k0;
         bind_scratch(pc, c, n_chunks);
+        if (launch_epi_rel(pc, t.epi_rel.d, sc, g.num_sms) != cudaSuccess) {
+            drain();
+            return fail(PGF_ERR_CUDA, "EPI row kernel of stage %d failed", c);
+        }
         if ((r = launch_kernels(t, pc, sc, t.evc[c][2], t.evc[c][3])) != PGF_OK) {
             drain();
             return r;
@@ -1809,6 +1818,7 @@ int pgf_finalize(void) {
     if (g.d2h_stream) cudaStreamSynchronize(g.d2h_stream);
     for (auto& t : g.tags) {
         t.epi.release();
+        t.epi_rel.release();
         t.id_epj.release();
         t.id_spj.release();
         t.id_spj_near.release();

@@ -138,8 +138,8 @@ __global__ __launch_bounds__(256) void gather_j_kernel(HdSendArgs a) {
 
 // kIdParts CTAs per walk (grid-stride over the units): each copies a slice
 // of the walk's id lists and checks it against the sent arrays; the first
-// also writes the walk's EPI rows (with the copies that the parts of a split
-// walk read), its box and descriptor(s) and its split record.  Host memory
+// also writes the walk's EPI rows, its box and descriptor(s), its split record
+// and the rows about the walk's centre.  Host memory
 // answers in
 // microseconds and serves whole lines best, so a CTA reads a walk's EPI
 // records as contiguous 8-byte words into shared memory (up to kEpiWords per
@@ -154,14 +154,12 @@ constexpr int kIdParts = 4;  // CTAs per walk for the id lists
 constexpr int kEpiWords = 3072;
 constexpr int kEpiPerThread = kEpiWords / kGatherThreads;
 
-__device__ __forceinline__ void write_rows(const HdWalkArgs& a, const WalkSrc& w, int i, const EpiDev& e,
-                                           const Accp& ac, const CoRec& co) {
-    for (int j = 0; j < w.parts; ++j) {
-        const int64_t row = j == 0 ? w.i_off + i : w.rows1 + (int64_t)(j - 1) * w.n_i + i;
-        a.out_epi[row] = e;
-        if (a.out_epi_acc) a.out_epi_acc[row] = ac;
-        if (a.out_epi_co) a.out_epi_co[row] = co;
-    }
+__device__ __forceinline__ void write_row(const HdWalkArgs& a, const WalkSrc& w, int i, const EpiDev& e,
+                                          const Accp& ac, const CoRec& co) {
+    const int64_t row = w.i_off + i;
+    a.out_epi[row] = e;
+    if (a.out_epi_acc) a.out_epi_acc[row] = ac;
+    if (a.out_epi_co) a.out_epi_co[row] = co;
 }
 
 // Loads the 8-byte words [0, n) of src, kEpiPerThread per thread.
@@ -261,7 +259,7 @@ __global__ __launch_bounds__(kGatherThreads) void gather_walks_kernel(HdWalkArgs
                     co = make_co_dev(*dptr(r, a.co_epi_off_r_in), *dptr(r, a.co_epi_off_r_out),
                                      *dptr(r, a.co_epi_off_self_mass), id);
                 }
-                write_rows(a, w, i0 + i, e, ac, co);
+                write_row(a, w, i0 + i, e, ac, co);
                 rs_max = fmax(rs_max, e.rs);
                 lo[0] = fmin(lo[0], e.x);
                 lo[1] = fmin(lo[1], e.y);
@@ -310,12 +308,13 @@ __global__ __launch_bounds__(kGatherThreads) void gather_walks_kernel(HdWalkArgs
                 d.hx = d.hy = d.hz = d.rs_max = 0.f;
             }
             d.part = 0;
-            d.n_parts = w.parts;
+            d.n_parts = (uint16_t)w.parts;
+            d.i_root = d.i_begin;
             d.root = k;
             d.n_spj_all = w.n_spj;
             d.rcut2 = w.rcut2;
             // A split walk: part j takes a slice of both lists; parts >= 1
-            // read the copy of the walk's rows at rows1 + (j - 1) n_i.
+            // write result rows of their own at rows1 + (j - 1) n_i.
             for (int j = 0; j < w.parts; ++j) {
                 WalkDesc q = d;
                 if (w.parts > 1) {
@@ -330,11 +329,18 @@ __global__ __launch_bounds__(kGatherThreads) void gather_walks_kernel(HdWalkArgs
                     a.out_walks[k] = q;
                 } else {
                     q.i_begin = (int32_t)(w.rows1 + (int64_t)(j - 1) * w.n_i);
-                    q.part = j;
+                    q.part = (uint16_t)j;
                     a.out_walks[w.desc1 + j - 1] = q;
                 }
             }
             if (w.parts > 1) a.out_splits[w.split] = SplitRec{(int32_t)w.i_off, (int32_t)w.rows1, w.n_i, w.parts};
+        }
+        // The rows about the centre (this CTA's own writes, read back).
+        for (int i = t; i < w.n_i; i += kGatherThreads) {
+            const double cx = __dmul_rn(0.5, __dadd_rn(red[0][0], red[3][0]));
+            const double cy = __dmul_rn(0.5, __dadd_rn(red[1][0], red[4][0]));
+            const double cz = __dmul_rn(0.5, __dadd_rn(red[2][0], red[5][0]));
+            a.out_epi_rel[w.i_off + i] = make_epi_rel(a.out_epi[w.i_off + i], cx, cy, cz, a.eps2);
         }
         __syncthreads();
     }

@@ -16,6 +16,8 @@
 //   WalkDesc[n_walk]     96 B: list offsets, walk centre (FP64), box
 //                              half-extents, largest i r_search, r_out^2
 //   order[n_walk]        walks sorted by descending work (the work queue)
+//   EpiRel[ni_tot]       32 B: FP32 (hi, lo) position about the walk centre,
+//                              r_search^2, guard band (warp-specialised kernels)
 //   out_accp[ni_tot]     Accp (32 B): acc.xyz, pot (G applied)
 //   out_nnb[ni_tot]      int32 neighbour count
 // The j arrays of a 1.5M-particle problem (about 50 MB EPJ + 18 MB SPJ for the
@@ -97,6 +99,67 @@ struct __align__(32) EpiDev {
 };
 static_assert(sizeof(EpiDev) == 32, "EpiDev layout");
 
+// An i-particle as the warp-specialised kernels read it: x - c of its walk as
+// an FP32 (hi, lo) pair, r_search^2 and the guard band of its neighbour test
+// in ulps.  Formed in FP64 once per dispatch (a split walk's parts and every
+// pass share it): GB300's FP64 pipe holds a warp instruction for 64 cycles.
+struct __align__(32) EpiRel {
+    float hx, hy, hz, rs2;
+    float lx, ly, lz;
+    int32_t kb;
+};
+static_assert(sizeof(EpiRel) == 32, "EpiRel layout");
+
+constexpr int kKMax = 1 << 22;
+
+__device__ __forceinline__ float rsqrt_approx(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// Guard band in ulps of rs2 for the near-pair neighbour test of one i at
+// distance D (max norm) from the walk centre; see kband_near64 in
+// pgf_kernels_mixed.cu for the derivation: the FP32 test is off by less than
+// 8 + 1.3e-6 D / r_ref ulps, r_ref = sqrt(rs^2 - eps2), and the band is
+// 48 + 1e-5 D / r_ref.  Evaluated here in FP32; the few ulps of rounding of
+// the FP32 form are far inside the factor of six between the band and the
+// bound, and a larger band only adds exact re-tests.
+__device__ __forceinline__ int kband_near(float D, float rs2, float eps2) {
+    const float r2ref = rs2 - eps2;
+    if (!(r2ref > 0.f)) return kKMax;
+    const float k = 48.f + 1e-5f * D * rsqrt_approx(r2ref) * 1.001f;
+    return k >= float(kKMax) ? kKMax : int(k) + 1;
+}
+
+__device__ __forceinline__ EpiRel make_epi_rel(const EpiDev& e, double cx, double cy, double cz, float eps2) {
+    const double dx = __dsub_rn(e.x, cx), dy = __dsub_rn(e.y, cy), dz = __dsub_rn(e.z, cz);
+    EpiRel r;
+    r.hx = __double2float_rn(dx);
+    r.hy = __double2float_rn(dy);
+    r.hz = __double2float_rn(dz);
+    r.rs2 = __double2float_rn(__dmul_rn(e.rs, e.rs));
+    r.lx = __double2float_rn(__dsub_rn(dx, (double)r.hx));
+    r.ly = __double2float_rn(__dsub_rn(dy, (double)r.hy));
+    r.lz = __double2float_rn(__dsub_rn(dz, (double)r.hz));
+    r.kb = kband_near(fmaxf(fabsf(r.hx), fmaxf(fabsf(r.hy), fabsf(r.hz))), r.rs2, eps2);
+    return r;
+}
+
+// Error-free sum: s + e == a + b exactly (round-to-nearest, no reassociation).
+__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
+    s = a + b;
+    const float bb = s - a;
+    e = (a - (s - bb)) + (b - bb);
+}
+
+// Sum of two (hi, lo) pairs.
+__device__ __forceinline__ float2 add_pair(float2 a, float2 b) {
+    float s, e;
+    two_sum(a.x, b.x, s, e);
+    return make_float2(s, e + (a.y + b.y));
+}
+
 struct __align__(32) WalkDesc {
     int64_t epj_begin;  // offset of the walk's EPJ ids in id_epj
     int64_t spj_begin;  // offset of the walk's SPJ ids in id_spj
@@ -108,10 +171,11 @@ struct __align__(32) WalkDesc {
     double rcut2;       // r_out^2 of the walk
     float hx, hy, hz;   // EPI box half-extents, rounded up
     float rs_max;       // largest r_search of the walk's EPI, rounded up
-    int32_t part;       // 0, or k >= 1 for part k of a split walk (adds no per-i terms)
-    int32_t n_parts;    // 1, or the parts of a split walk
+    uint16_t part;      // 0, or k >= 1 for part k of a split walk (adds no per-i terms)
+    uint16_t n_parts;   // 1, or the parts of a split walk
     int32_t root;       // descriptor of part 0 (this one when not split)
     int32_t n_spj_all;  // SPJ of the whole walk
+    int32_t i_root;     // first EPI row of the walk; i_begin is the first result row
 };
 static_assert(sizeof(WalkDesc) == 96, "WalkDesc layout");
 
@@ -128,13 +192,13 @@ struct Retest {
     int32_t i;        // EPI row
     int32_t n;        // number of list entries
     int32_t walk;     // walk (descriptor index) of the i-particle
-    int32_t pad;
+    int32_t row;      // result row
 };
 
 // Superparticles of one walk left to the pair kernels by the far-field pass:
 // the entries in each quarter of the walk's list (n[0] < 0: the list as it
 // is), and whether out_accp of the walk's rows holds the sums of the others
-// (without G, each as an FP32 (hi, lo) pair: far_sum) for the pair kernels to
+// (load_pairs) for the pair kernels to
 // add.
 struct __align__(32) SpjNear {
     int32_t n[4];
@@ -144,6 +208,7 @@ struct __align__(32) SpjNear {
 
 struct Params {
     const EpiDev* epi;
+    const EpiRel* epi_rel;  // of the same rows (launch_epi_rel or the walk gather)
     const EpjMix* epj;
     const double* epj_m64;
     const double* epj_rs64;
@@ -253,8 +318,9 @@ __device__ __forceinline__ void co_pair_diff(const EpiDev& ei, const CoRec& ci, 
 }
 
 // A walk whose list was split into n_parts parts (small dispatches, to spread
-// the largest walks over several CTAs): part 0 writes the walk's own EPI rows
-// from row0, part k >= 1 a copy of them from rows1 + (k - 1) n_i.
+// the largest walks over several CTAs): every part reads the walk's EPI rows;
+// part 0 writes the walk's own result rows from row0, part k >= 1 rows of its
+// own from rows1 + (k - 1) n_i.
 struct SplitRec {
     int32_t row0, rows1, n_i, n_parts;
 };
@@ -270,7 +336,7 @@ struct WalkSrc {
     const int32_t* id_epj;  // the caller's id lists of the walk
     const int32_t* id_spj;
     int64_t i_off, e_off, s_off;  // first EPI row and list entries in the device arrays
-    int64_t rows1;          // split walks: first EPI row of part 1's copy
+    int64_t rows1;          // split walks: first result row of part 1
     double rcut2;           // r_out^2 of the walk
     int32_t n_i, n_epj, n_spj;
     int32_t walk;           // the caller's walk index (error reports)
@@ -323,6 +389,8 @@ struct HdWalkArgs {
     size_t co_epi_off_id, co_epi_off_r_in, co_epi_off_r_out, co_epi_off_self_mass;  // changeover (out_epi_co)
     int64_t n_epj_tot, n_spj_tot;
     EpiDev* out_epi;
+    EpiRel* out_epi_rel;
+    float eps2;  // of the kernels' neighbour test (guard bands)
     Accp* out_epi_acc;
     CoRec* out_epi_co;
     int32_t* out_id_epj;
@@ -374,15 +442,22 @@ inline cudaError_t reset_counters(const Params& p, cudaStream_t s) {
 constexpr int64_t kFarMinRows = 8192;
 inline bool far_applies(double eps2, int64_t n_i) { return eps2 == 0.0 && n_i >= kFarMinRows; }
 
-// The far-field sums in row gi: acceleration x, y, z and potential.
-__device__ __forceinline__ void far_sum(const Params& p, int gi, double f[4]) {
-    const float4* r = reinterpret_cast<const float4*>(p.out_accp + gi);
+// A result row as four (hi, lo) FP32 pairs, without G: the far-field sums
+// (acceleration x, y, z and potential) and the sums of a split walk's parts.
+__device__ __forceinline__ void load_pairs(const Accp* row, float2 f[4]) {
+    const float4* r = reinterpret_cast<const float4*>(row);
     const float4 a = r[0], b = r[1];
-    f[0] = (double)a.x + (double)a.y;
-    f[1] = (double)a.z + (double)a.w;
-    f[2] = (double)b.x + (double)b.y;
-    f[3] = (double)b.z + (double)b.w;
+    f[0] = make_float2(a.x, a.y);
+    f[1] = make_float2(a.z, a.w);
+    f[2] = make_float2(b.x, b.y);
+    f[3] = make_float2(b.z, b.w);
 }
+__device__ __forceinline__ void store_pairs(Accp* row, const float2 f[4]) {
+    float4* r = reinterpret_cast<float4*>(row);
+    r[0] = make_float4(f[0].x, f[0].y, f[1].x, f[1].y);
+    r[1] = make_float4(f[2].x, f[2].y, f[3].x, f[3].y);
+}
+__device__ __forceinline__ double pair_value(float2 v) { return (double)v.x + (double)v.y; }
 
 // The superparticle list the pair kernels run for one descriptor: entries
 // [begin, begin + n) of the walk's own list, or of its compacted one, whose
@@ -439,12 +514,13 @@ cudaError_t launch_mixed(const Params& p, cudaStream_t s, int num_sms);
 cudaError_t launch_retest(const Params& p, cudaStream_t s, int num_sms);
 // Adds the results of every split walk's parts into its own rows, parts in
 // order (deterministic).
-// pot_soft and acorr (optional) are the changeover and gradient modes' outputs.
+// pot_soft and acorr (optional) are the changeover and gradient modes'
+// outputs.  pairs: the parts' rows are (hi, lo) pairs without G (the
+// warp-specialised kernels), else FP64 with G applied.
 cudaError_t launch_combine_parts(const SplitRec* recs, int n_recs, Accp* accp, int32_t* nnb, double* pot_soft,
-                                 Accp* acorr, cudaStream_t s);
-// Copies every split walk's EPI rows (and its changeover / gradient records,
-// when given) from row0 to the rows of parts 1 .. n_parts-1.
-cudaError_t launch_split_rows(const SplitRec* recs, int n_recs, EpiDev* epi, CoRec* co, Accp* acc, cudaStream_t s);
+                                 Accp* acorr, bool pairs, double G, cudaStream_t s);
+// EpiRel rows of every walk of a launch (its roots).
+cudaError_t launch_epi_rel(const Params& p, EpiRel* out, cudaStream_t s, int num_sms);
 // Builds the (hi, lo) FP32 copies of the EPJ / SPJ arrays.
 cudaError_t launch_split_j(const EpjMix* epj, int64_t n_epj, EpjF32* epj32, const SpjMix* spj, int64_t n_spj,
                            SpjF32* spj32, cudaStream_t s);

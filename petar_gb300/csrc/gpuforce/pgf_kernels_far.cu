@@ -48,14 +48,12 @@ constexpr int kRing = 64;      // per warp: 32 sources arrive while fewer than 3
 constexpr int kMinI = 32;      // fewer i: direct pairs (33 n_i operations) cost about as much
 constexpr float kRhoMax = 0.14f;
 constexpr float kQuadTol = 2e-6f / 84.f;
-constexpr int kKeptI = 512;  // i whose coordinates stay in shared memory
 constexpr int kPad = 96;  // coefficients padded to 3 per lane
 
 struct FarSmem {
     float src[kWarps][9][kRing];  // x, y, z, m, and the five quadrupole moments (QuadOp), scaled
     float red[kWarps][kPad];
     float2 lead[kWarps][4];  // rows 0 and 1 as (hi, lo)
-    float xi[3][kKeptI];      // the first i's coordinates, scaled
     float c[2][3];            // walk centre (hi, lo)
     float L[kFarCoefs + 3];
     float4 ev[kFarCoefs + 3];  // phi and gradient coefficients
@@ -63,12 +61,6 @@ struct FarSmem {
     int n_near[kWarps], n_far[kWarps];
     int w;
 };
-
-__device__ __forceinline__ float rsqrt_approx_f(float x) {
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 
 struct SpjRec {
     float4 a, b, c;
@@ -84,13 +76,6 @@ __device__ __forceinline__ SpjRec load_spj(const SpjF32* __restrict__ spj, int i
         r.d = __ldg(reinterpret_cast<const float2*>(src + 3));
     }
     return r;
-}
-
-// Sum of two (hi, lo) pairs.
-__device__ __forceinline__ float2 add_pair(float2 a, float2 b) {
-    float s, e;
-    two_sum_le(a.x, b.x, s, e);
-    return make_float2(s, e + (a.y + b.y));
 }
 
 // A shared-memory load that keeps its place: hoisted to the front, the 80
@@ -159,14 +144,8 @@ __global__ __launch_bounds__(kT, 3) void far_kernel(Params p) {
         // Radius of the walk's particles.
         float r2m = 0.f;
         for (int i = t; i < wd.n_i; i += kT) {
-            const EpiDev e = p.epi[wd.i_begin + i];
-            const float x = (float)(e.x - wd.cx), y = (float)(e.y - wd.cy), z = (float)(e.z - wd.cz);
-            if (i < kKeptI) {
-                s.xi[0][i] = x;
-                s.xi[1][i] = y;
-                s.xi[2][i] = z;
-            }
-            r2m = fmaxf(r2m, fmaf(x, x, fmaf(y, y, z * z)));
+            const float4 e = __ldg(reinterpret_cast<const float4*>(p.epi_rel + wd.i_root + i));
+            r2m = fmaxf(r2m, fmaf(e.x, e.x, fmaf(e.y, e.y, e.z * e.z)));
         }
         if (t < 3) {
             const double c = t == 0 ? wd.cx : (t == 1 ? wd.cy : wd.cz);
@@ -269,7 +248,7 @@ __global__ __launch_bounds__(kT, 3) void far_kernel(Params p) {
             const int take = min(32, waiting);
             head = (head + take) & (kRing - 1);
             waiting -= take;
-            const float ri = rsqrt_approx_f(fmaf(hx, hx, fmaf(hy, hy, hz * hz)));
+            const float ri = rsqrt_approx(fmaf(hx, hx, fmaf(hy, hy, hz * hz)));
             add_source(hx, hy, hz, ri, m, q, L, lo);
         }
         if (lane == 0) {
@@ -325,31 +304,41 @@ __global__ __launch_bounds__(kT, 3) void far_kernel(Params p) {
 #pragma unroll 1
         for (int i = t; i < wd.n_i; i += kT) {
             const int gi = wd.i_begin + i;
-            float x, y, z;
-            if (i < kKeptI) {
-                x = s.xi[0][i] * inv;
-                y = s.xi[1][i] * inv;
-                z = s.xi[2][i] * inv;
-            } else {
-                const EpiDev e = p.epi[gi];
-                x = (float)(e.x - wd.cx) * inv;
-                y = (float)(e.y - wd.cy) * inv;
-                z = (float)(e.z - wd.cz) * inv;
-            }
+            const float4 e = __ldg(reinterpret_cast<const float4*>(p.epi_rel + wd.i_root + i));
+            const float x = e.x * inv, y = e.y * inv, z = e.z * inv;
             float r0[2 * kFarOrder + 1] = {1.f}, rz[2 * kFarOrder + 1] = {};
             float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
             eval_rows<1>(r0, rz, x, y, z, fmaf(x, x, fmaf(y, y, z * z)), s.ev, o);
             // rows 0: phi = L_00, gradient (Re L_11, Im L_11, L_10)
             const float2 ax = add_pair(lead[2], make_float2(o.x, 0.f)), ay = add_pair(lead[3], make_float2(o.y, 0.f));
             const float2 az = add_pair(lead[1], make_float2(o.z, 0.f)), ph = add_pair(lead[0], make_float2(o.w, 0.f));
-            float4* out = reinterpret_cast<float4*>(p.out_accp + gi);
-            out[0] = make_float4(ax.x * inv2, ax.y * inv2, ay.x * inv2, ay.y * inv2);
-            out[1] = make_float4(az.x * inv2, az.y * inv2, -ph.x * inv, -ph.y * inv);
+            const float2 f[4] = {make_float2(ax.x * inv2, ax.y * inv2), make_float2(ay.x * inv2, ay.y * inv2),
+                                 make_float2(az.x * inv2, az.y * inv2), make_float2(-ph.x * inv, -ph.y * inv)};
+            store_pairs(p.out_accp + gi, f);
         }
     }
 }
 
+// EPI rows about their walk's centre, one warp per walk.
+__global__ __launch_bounds__(256) void epi_rel_kernel(Params p, EpiRel* __restrict__ out) {
+    const int n_walk = p.n_root < p.n_walk ? p.n_root : walk_count(p);
+    const int lane = threadIdx.x & 31;
+    for (int k = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); k < n_walk; k += (int)((gridDim.x * blockDim.x) >> 5)) {
+        const WalkDesc wd = p.walks[p.n_root < p.n_walk ? k : p.order[k]];
+        for (int i = lane; i < wd.n_i; i += 32)
+            out[wd.i_root + i] = make_epi_rel(p.epi[wd.i_root + i], wd.cx, wd.cy, wd.cz, (float)p.eps2);
+    }
+}
+
 }  // namespace
+
+cudaError_t launch_epi_rel(const Params& p, EpiRel* out, cudaStream_t s, int num_sms) {
+    if (p.n_walk <= 0) return cudaSuccess;
+    const int64_t want = ((int64_t)(p.n_root < p.n_walk ? p.n_root : p.n_walk) + 7) / 8;
+    const int grid = (int)(want < num_sms * 8 ? want : num_sms * 8);
+    epi_rel_kernel<<<grid, 256, 0, s>>>(p, out);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_far(const Params& p, cudaStream_t s, int num_sms) {
     if (!p.spj_near || p.n_walk <= 0) return cudaSuccess;

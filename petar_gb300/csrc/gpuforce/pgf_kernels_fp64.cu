@@ -35,7 +35,7 @@ __global__ __launch_bounds__(kT) void fp64_kernel(Params p) {
             const bool valid = li < wd.n_i;
             double xi = 0, yi = 0, zi = 0, rsi = 0;
             if (valid) {
-                const EpiDev e = p.epi[wd.i_begin + li];
+                const EpiDev e = p.epi[wd.i_root + li];
                 xi = e.x;
                 yi = e.y;
                 zi = e.z;

@@ -171,7 +171,7 @@ __global__ __launch_bounds__(kThreadsG, 2) void gradient_kernel_pk(Params p) {
                 float v[12] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
                 const int ii = li + k * S;
                 if (active && ii < nip) {
-                    const int gi = wd.i_begin + ipass + ii;
+                    const int gi = wd.i_root + ipass + ii;
                     const EpiDev e = p.epi[gi];
                     const double d[3] = {e.x - wd.cx, e.y - wd.cy, e.z - wd.cz};
                     const Accp a = p.epi_acc64[gi];
@@ -501,12 +501,12 @@ __global__ __launch_bounds__(kThreadsG, 2) void gradient_kernel_pk(Params p) {
                         for (int c = 0; c < 7; ++c) r[c] += (double)s.acc[k][c][src].x + (double)s.acc[k][c][src].y;
                     }
                     if (spj.add_far) {  // the far-field pass's sums
-                        double f[4];
-                        far_sum(p, gi, f);
-                        for (int c = 0; c < 4; ++c) r[3 + c] += f[c];
+                        float2 f[4];
+                        load_pairs(p.out_accp + gi, f);
+                        for (int c = 0; c < 4; ++c) r[3 + c] += pair_value(f[c]);
                     }
                     // a_i once: parts of a split walk add their pairs only
-                    const Accp a = wd.part == 0 ? p.epi_acc64[gi] : Accp{0.0, 0.0, 0.0, 0.0};
+                    const Accp a = wd.part == 0 ? p.epi_acc64[wd.i_root + ipass + ii] : Accp{0.0, 0.0, 0.0, 0.0};
                     const double G = p.G;
                     p.out_acorr[gi] = Accp{2.0 * r[0], 2.0 * r[1], 2.0 * r[2], 0.0};
                     p.out_accp[gi] = Accp{a.x + G * r[3], a.y + G * r[4], a.z + G * r[5], G * r[6]};

@@ -23,7 +23,7 @@
 //     a walk 0.1 wide; these pairs get the cutoff and the neighbour test.
 // Exact neighbour counts
 //   The FP32 test r2 < max(rs_i, rs_j)^2 is done on float bit patterns with a
-//   per-i guard band of K ulps that bounds the FP32 error (kband_near).  Pairs
+//   per-i guard band of K ulps that bounds the FP32 error (kband_near64).  Pairs
 //   more than K ulps below rs2 are counted, pairs more than K ulps above are
 //   not.  If any pair of (i, tile) falls inside the band, every thread drops
 //   its count of that (i, tile) and one thread pushes a Retest record: the
@@ -71,16 +71,9 @@ constexpr int kMaxPass = kThreads * kI;  // i-particles per pass
 constexpr int kTileEP = kThreads;        // one EPJ per thread per tile
 constexpr int kTileSP = kThreads / 2;    // two threads stage one SPJ
 constexpr int kFlush = 256;              // pairs per thread between FP64 flushes
-constexpr int kKMax = 1 << 22;
 constexpr int kNearUnroll = PGF_NEAR_UNROLL;
 constexpr int kFarUnroll = PGF_FAR_UNROLL;
 constexpr int kSpUnroll = PGF_SP_UNROLL;
-
-__device__ __forceinline__ float rsqrt_approx(float x) {
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 
 // Guard band, in float ulps of rs2, for the near-pair neighbour test of one
 // i-particle at distance D (max norm) from the walk centre.  With u = 2^-24
@@ -89,7 +82,7 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
 // r2 + eps2 near the threshold, r >= r_ref = sqrt(rs_i^2 - eps2); rounding
 // rs2 to float adds u.  One ulp of x is at least u x: the bound is below
 // 8 + 1.3e-6 D / r_ref ulps.  K is more than twice that.
-__device__ __forceinline__ int kband_near(double D, double rs, double eps2) {
+__device__ __forceinline__ int kband_near64(double D, double rs, double eps2) {
     const double r2ref = rs * rs - eps2;
     if (!(r2ref > 0.0)) return kKMax;
     const double k = 48.0 + 1e-5 * D / sqrt(r2ref);
@@ -202,7 +195,7 @@ __global__ __launch_bounds__(kThreads, PGF_MINB) void mixed_kernel(Params p) {
             const bool active = js < n_js;
 
             float xih[kI], yih[kI], zih[kI], xil[kI], yil[kI], zil[kI], rsi2[kI];
-            int kb[kI], gi[kI], li[kI], cnt[kI];
+            int kb[kI], gi[kI], ri[kI], li[kI], cnt[kI];  // gi: result row, ri: EPI row
             bool valid[kI];
             float a[kI][4];
 #pragma unroll
@@ -210,12 +203,13 @@ __global__ __launch_bounds__(kThreads, PGF_MINB) void mixed_kernel(Params p) {
                 li[k] = slot + k * S;
                 valid[k] = active && li[k] < nip;
                 gi[k] = wd.i_begin + ipass + li[k];
+                ri[k] = wd.i_root + ipass + li[k];
                 xih[k] = yih[k] = zih[k] = xil[k] = yil[k] = zil[k] = 0.f;
                 rsi2[k] = 0.f;
                 kb[k] = 0;
                 cnt[k] = 0;
                 if (valid[k]) {
-                    const EpiDev e = p.epi[gi[k]];
+                    const EpiDev e = p.epi[ri[k]];
                     const double dx = e.x - cx, dy = e.y - cy, dz = e.z - cz;
                     xih[k] = (float)dx;
                     yih[k] = (float)dy;
@@ -224,7 +218,7 @@ __global__ __launch_bounds__(kThreads, PGF_MINB) void mixed_kernel(Params p) {
                     yil[k] = (float)(dy - (double)yih[k]);
                     zil[k] = (float)(dz - (double)zih[k]);
                     rsi2[k] = (float)(e.rs * e.rs);
-                    kb[k] = kband_near(fmax(fabs(dx), fmax(fabs(dy), fabs(dz))), e.rs, eps2d);
+                    kb[k] = kband_near64(fmax(fabs(dx), fmax(fabs(dy), fabs(dz))), e.rs, eps2d);
                 }
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
@@ -469,13 +463,13 @@ __global__ __launch_bounds__(kThreads, PGF_MINB) void mixed_kernel(Params p) {
                             if (slot_r < p.retest_cap) {
                                 Retest rr;
                                 rr.j_begin = rt.base;
-                                rr.i = gi[k];
+                                rr.i = ri[k];
+                                rr.row = gi[k];
                                 rr.n = rt.nt;
                                 rr.walk = widx;
-                                rr.pad = 0;
                                 p.retest[slot_r] = rr;
                             } else {
-                                cnt[k] += exact_count(p, gi[k], rt.base, rt.nt);
+                                cnt[k] += exact_count(p, ri[k], rt.base, rt.nt);
                             }
                         }
                     }
@@ -535,26 +529,11 @@ __global__ __launch_bounds__(256) void retest_kernel(Params p) {
         for (int k = lane; k < rec.n; k += 32) {
             const int id = p.id_epj[rec.j_begin + k];
             const EpjMix e = p.epj[id];
-            const int nb = exact_neighbour(ei.x, ei.y, ei.z, ei.rs, e.x, e.y, e.z, p.epj_rs64[id], p.eps2);
-            c += nb;
-            if (p.epi_co && nb) {
-                // Fused changeover mode: the interaction kernel used the linear
-                // cutoff for this pair; replace it by the changeover terms.
-                const CoRec ci = p.epi_co[rec.i], cj = p.epj_co[id];
-                if (ci.id != cj.id) {
-                    double d[5];
-                    co_pair_diff(ei, ci, e, e.m, cj, p.eps2, p.walks[rec.walk].rcut2, d);
-                    atomicAdd(&p.out_accp[rec.i].x, p.G * d[0]);
-                    atomicAdd(&p.out_accp[rec.i].y, p.G * d[1]);
-                    atomicAdd(&p.out_accp[rec.i].z, p.G * d[2]);
-                    atomicAdd(&p.out_accp[rec.i].w, p.G * d[3]);
-                    atomicAdd(&p.out_pot_soft[rec.i], p.G * d[4]);
-                }
-            }
+            c += exact_neighbour(ei.x, ei.y, ei.z, ei.rs, e.x, e.y, e.z, p.epj_rs64[id], p.eps2);
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-        if (lane == 0 && c) atomicAdd(&p.out_nnb[rec.i], c);
+        if (lane == 0 && c) atomicAdd(&p.out_nnb[rec.row], c);
     }
 }
 
@@ -577,61 +556,68 @@ cudaError_t launch_mixed(const Params& p, cudaStream_t s, int num_sms) {
     return cudaGetLastError();
 }
 
-__global__ __launch_bounds__(256) void combine_parts_kernel(const SplitRec* __restrict__ recs, Accp* accp,
-                                                            int32_t* nnb, double* pot_soft, Accp* acorr) {
+// One thread per result row of a split walk: gridDim.y CTAs share a walk's
+// rows, and the loads of four parts are in flight at once.
+template <bool PAIRS>
+__global__ __launch_bounds__(128) void combine_parts_kernel(const SplitRec* __restrict__ recs, Accp* accp,
+                                                            int32_t* nnb, double* pot_soft, Accp* acorr, double G) {
     const SplitRec r = recs[blockIdx.x];
-    for (int i = threadIdx.x; i < r.n_i; i += blockDim.x) {
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < r.n_i; i += gridDim.y * blockDim.x) {
         const int64_t r0 = (int64_t)r.row0 + i;
-        Accp a = accp[r0];
-        int c = nnb[r0];
-        double ps = pot_soft ? pot_soft[r0] : 0.0;
-        Accp g = acorr ? acorr[r0] : Accp{0.0, 0.0, 0.0, 0.0};
-        for (int k = 1; k < r.n_parts; ++k) {
-            const int64_t row = (int64_t)r.rows1 + (int64_t)(k - 1) * r.n_i + i;
-            const Accp b = accp[row];
-            a.x += b.x;
-            a.y += b.y;
-            a.z += b.z;
-            a.w += b.w;
-            c += nnb[row];
-            if (pot_soft) ps += pot_soft[row];
-            if (acorr) {
-                const Accp h = acorr[row];
-                g.x += h.x;
-                g.y += h.y;
-                g.z += h.z;
+        if constexpr (PAIRS) {
+            float2 a[4], ps = make_float2(0.f, 0.f);
+            load_pairs(accp + r0, a);
+            int c = nnb[r0];
+            const float2* soft = reinterpret_cast<const float2*>(pot_soft);
+            if (pot_soft) ps = soft[r0];
+#pragma unroll 4
+            for (int k = 1; k < r.n_parts; ++k) {
+                const int64_t row = (int64_t)r.rows1 + (int64_t)(k - 1) * r.n_i + i;
+                float2 b[4];
+                load_pairs(accp + row, b);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) a[q] = add_pair(a[q], b[q]);
+                c += nnb[row];
+                if (pot_soft) ps = add_pair(ps, soft[row]);
             }
+            accp[r0] = Accp{G * pair_value(a[0]), G * pair_value(a[1]), G * pair_value(a[2]), G * pair_value(a[3])};
+            nnb[r0] = c;
+            if (pot_soft) pot_soft[r0] = G * pair_value(ps);
+        } else {
+            Accp a = accp[r0];
+            int c = nnb[r0];
+            Accp g = acorr ? acorr[r0] : Accp{0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+            for (int k = 1; k < r.n_parts; ++k) {
+                const int64_t row = (int64_t)r.rows1 + (int64_t)(k - 1) * r.n_i + i;
+                const Accp b = accp[row];
+                a.x += b.x;
+                a.y += b.y;
+                a.z += b.z;
+                a.w += b.w;
+                c += nnb[row];
+                if (acorr) {
+                    const Accp h = acorr[row];
+                    g.x += h.x;
+                    g.y += h.y;
+                    g.z += h.z;
+                }
+            }
+            accp[r0] = a;
+            nnb[r0] = c;
+            if (acorr) acorr[r0] = g;
         }
-        accp[r0] = a;
-        nnb[r0] = c;
-        if (pot_soft) pot_soft[r0] = ps;
-        if (acorr) acorr[r0] = g;
     }
 }
 
 cudaError_t launch_combine_parts(const SplitRec* recs, int n_recs, Accp* accp, int32_t* nnb, double* pot_soft,
-                                 Accp* acorr, cudaStream_t s) {
+                                 Accp* acorr, bool pairs, double G, cudaStream_t s) {
     if (n_recs <= 0) return cudaSuccess;
-    combine_parts_kernel<<<n_recs, 256, 0, s>>>(recs, accp, nnb, pot_soft, acorr);
-    return cudaGetLastError();
-}
-
-__global__ __launch_bounds__(256) void split_rows_kernel(const SplitRec* __restrict__ recs, EpiDev* epi, CoRec* co,
-                                                         Accp* acc) {
-    const SplitRec r = recs[blockIdx.x];
-    const int64_t total = (int64_t)(r.n_parts - 1) * r.n_i;
-    for (int64_t k = threadIdx.x; k < total; k += blockDim.x) {
-        const int64_t i = k % r.n_i;
-        const int64_t src = (int64_t)r.row0 + i, dst = (int64_t)r.rows1 + k;
-        epi[dst] = epi[src];
-        if (co) co[dst] = co[src];
-        if (acc) acc[dst] = acc[src];
-    }
-}
-
-cudaError_t launch_split_rows(const SplitRec* recs, int n_recs, EpiDev* epi, CoRec* co, Accp* acc, cudaStream_t s) {
-    if (n_recs <= 0) return cudaSuccess;
-    split_rows_kernel<<<n_recs, 256, 0, s>>>(recs, epi, co, acc);
+    const dim3 grid(n_recs, 2);
+    if (pairs)
+        combine_parts_kernel<true><<<grid, 128, 0, s>>>(recs, accp, nnb, pot_soft, acorr, G);
+    else
+        combine_parts_kernel<false><<<grid, 128, 0, s>>>(recs, accp, nnb, pot_soft, acorr, G);
     return cudaGetLastError();
 }
 

@@ -24,10 +24,11 @@
 //   producer would throttle it on small walks.
 // * Consumers flush their FP32 partial sums into (hi, lo) FP32 accumulators
 //   in shared memory with a two-sum (no FP64 in the pair loops either); the
-//   j-slices are combined in FP64 once per pass.
-// * Ambiguous neighbour pairs (within the guard band of r_search) are pushed
-//   one by one as Retest records with their own list index, so no thread has
-//   to coordinate its counts with another.
+//   j-slices are combined as (hi, lo) pairs once per pass, and the i set up
+//   from EpiRel rows, so that a pass issues FP64 only to write its results
+//   (parts of split walks: not even there).
+// * Ambiguous neighbour pairs (within the guard band of r_search; a few per
+//   evaluation) are tested exactly in FP64 where they are met.
 // * Every mbarrier wait is bounded by 1 s of %globaltimer; on expiry the thread
 //   sets the device error word and returns.  The host reports PGF_ERR_DEVICE.
 #include "pgf_internal.cuh"
@@ -41,32 +42,10 @@ namespace {
 // EP tile (TE / 32 per producer lane), TE SPJ entries per SP tile (TE / 2
 // with TMA staging), NS ring slots.
 constexpr int kFlush = 256;   // pairs per consumer thread between FP64 flushes
-constexpr int kKMax = 1 << 22;
 constexpr unsigned long long kWaitLimitNs = 1000000000ull;
 constexpr int kErrWaitTimeout = 1;
 
 enum : int { kItemEP = 0, kItemSP = 1, kItemBegin = 2, kItemEnd = 3, kItemExit = 4 };
-
-__device__ __forceinline__ float rsqrt_approx(float x) {
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-// Guard band in ulps of rs2 for the near-pair neighbour test of one i at
-// distance D (max norm) from the walk centre; see kband_near in
-// pgf_kernels_mixed.cu for the derivation: the FP32 test is off by less than
-// 8 + 1.3e-6 D / r_ref ulps, r_ref = sqrt(rs^2 - eps2), and the band is
-// 48 + 1e-5 D / r_ref.  Evaluated here in FP32 (GB300's FP64 pipe runs at
-// 1/64 of the FP32 rate and this runs for every i of every pass); the few
-// ulps of rounding of the FP32 form are far inside the factor of six between
-// the band and the bound, and a larger band only adds FP64 re-tests.
-__device__ __forceinline__ int kband_near(float D, float rs2, float eps2) {
-    const float r2ref = rs2 - eps2;
-    if (!(r2ref > 0.f)) return kKMax;
-    const float k = 48.f + 1e-5f * D * rsqrt_approx(r2ref) * 1.001f;
-    return k >= float(kKMax) ? kKMax : int(k) + 1;
-}
 
 // L2 policy for data read once per launch (the id lists): evicted before
 // lines loaded with the default policy, so the streamed ids do not push the
@@ -81,13 +60,6 @@ __device__ __forceinline__ int ld_streamed(const int32_t* a, uint64_t pol) {
     int v;
     asm volatile("ld.global.nc.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(v) : "l"(a), "l"(pol));
     return v;
-}
-
-// Error-free sum: s + e == a + b exactly (round-to-nearest, no reassociation).
-__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
-    s = a + b;
-    const float bb = s - a;
-    e = (a - (s - bb)) + (b - bb);
 }
 
 __device__ __forceinline__ unsigned long long globaltimer() {
@@ -690,7 +662,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
     // Pass state.  A pass runs ku (KA or KI) i-particles per thread, whichever
     // leaves fewer lanes idle; the tile bodies are instantiated for both.
     float rcut2 = 0.f;
-    int nip = 0, S = 1, n_js = 1, js = 0, slot = 0, ku = KI, gbase = 0;
+    int nip = 0, S = 1, n_js = 1, js = 0, slot = 0, ku = KI, gbase = 0, ibase = 0;
     bool active = false, add_far = false;
     // Scalar path: i coordinates and accumulators a[0..2] acceleration, a[3]
     // potential.  Packed path: (-x_i, -x_i) operands and pair accumulators
@@ -702,8 +674,8 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
     // Changeover: pot_tot and pot_soft partials of neighbour pairs (all other
     // pairs add the same term to both, in a[k][3]).
     float dt[CO ? KI : 1], ds[CO ? KI : 1];
-    double r_out_walk = 0.0, rcut2d = 0.0, self_scale = 1.0;
-    int walk_cur = 0;
+    double rcut2d = 0.0;
+    bool add_self = true, parts = false;
     int since = 0;
 #pragma unroll
     for (int k = 0; k < (CO ? KI : 1); ++k) dt[k] = ds[k] = 0.f;
@@ -800,25 +772,16 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
         clear_acc();
         since = 0;
     };
-    auto push_retest = [&](int k, int64_t jidx) -> int {
-        const int gi = gbase + k * S;
-        const int r = atomicAdd(p.n_retest, 1);
-        if (r < p.retest_cap) {
-            Retest rr;
-            rr.j_begin = jidx;
-            rr.i = gi;
-            rr.n = 1;
-            rr.walk = CO ? walk_cur : 0;  // only the changeover re-test reads it
-            rr.pad = 0;
-            p.retest[r] = rr;
-            return 0;
-        }
+    // Exact FP64 neighbour test of a pair inside the guard band (a few pairs per
+    // evaluation); the changeover mode adds the pair's difference when it is one.
+    auto retest = [&](int k, int64_t jidx) -> int {
+        const int gi = ibase + k * S;
+        if (p.retest_total) atomicAdd(p.retest_total, 1);
         const EpiDev ei = p.epi[gi];
         const int id = p.id_epj[jidx];
         const EpjMix e = p.epj[id];
         const int nb = exact_neighbour(ei.x, ei.y, ei.z, ei.rs, e.x, e.y, e.z, p.epj_rs64[id], p.eps2);
         if constexpr (CO) {
-            // Capacity overflow: apply the changeover difference here.
             const CoRec ci = p.epi_co[gi], cj = p.epj_co[id];
             if (nb && ci.id != cj.id) {
                 double d[5];
@@ -867,7 +830,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
                     const float rs2 = fmaxf(lo[k].w, ll.w);
                     const int e = __float_as_int(r2) - __float_as_int(rs2) + kb[k];
                     c[k] += (int)((unsigned)e >> 31);
-                    if ((unsigned)e < (unsigned)(2 * kb[k]) && vk[k]) c[k] += push_retest(k, h.base + T.nidx[j]);
+                    if ((unsigned)e < (unsigned)(2 * kb[k]) && vk[k]) c[k] += retest(k, h.base + T.nidx[j]);
                     if constexpr (CO) {
                         const CoRec& cj = T.nco[j];
                         if ((e < 0) && cj.id != ci[k].id) {
@@ -1071,29 +1034,26 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
             slot = ct - js * S;
             active = js < n_js;
             gbase = wd.i_begin + h.ipass + slot;
+            ibase = wd.i_root + h.ipass + slot;
+            parts = wd.n_parts > 1;
             if constexpr (!SR) add_far = spj_list(p, wd).add_far;
             if constexpr (CO) {
-                r_out_walk = sqrt(wd.rcut2);
                 rcut2d = wd.rcut2;
-                walk_cur = h.walk;
-                self_scale = wd.part == 0 ? 1.0 : 0.0;  // parts of a split walk add it once
+                add_self = wd.part == 0;  // parts of a split walk add it once
             }
 #pragma unroll
             for (int k = 0; k < KI; ++k) {
                 const bool valid = active && k < ku && slot + k * S < nip;
-                float hx = 0.f, hy = 0.f, hz = 0.f;
-                float4 lo = make_float4(0.f, 0.f, 0.f, 0.f);
+                float4 hi = make_float4(0.f, 0.f, 0.f, 0.f), lo = hi;
                 int kb = 0;
                 if (valid) {
-                    const EpiDev e = p.epi[gbase + k * S];
-                    const double dx = e.x - wd.cx, dy = e.y - wd.cy, dz = e.z - wd.cz;
-                    hx = (float)dx;
-                    hy = (float)dy;
-                    hz = (float)dz;
-                    lo = make_float4((float)(dx - (double)hx), (float)(dy - (double)hy), (float)(dz - (double)hz),
-                                     (float)(e.rs * e.rs));
-                    kb = kband_near(fmaxf(fabsf(hx), fmaxf(fabsf(hy), fabsf(hz))), lo.w, eps2);
+                    const float4* e = reinterpret_cast<const float4*>(p.epi_rel + ibase + k * S);
+                    hi = __ldg(e);
+                    lo = __ldg(e + 1);
+                    kb = __float_as_int(lo.w);
+                    lo.w = hi.w;  // r_search^2
                 }
+                const float hx = hi.x, hy = hi.y, hz = hi.z;
                 if constexpr (PK) {
                     nx2[k] = make_float2(-hx, -hx);
                     ny2[k] = make_float2(-hy, -hy);
@@ -1108,7 +1068,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
                 if constexpr (CO) {
                     CoRec cr{};
                     cr.id = -1;
-                    if (valid) cr = p.epi_co[gbase + k * S];
+                    if (valid) cr = p.epi_co[ibase + k * S];
                     s.co.coi[k][ct] = cr;
                     s.co.dtot[k][ct] = make_float2(0.f, 0.f);
                     s.co.dsoft[k][ct] = make_float2(0.f, 0.f);
@@ -1143,35 +1103,48 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
 #pragma unroll
                 for (int k = 0; k < KI; ++k) {
                     if (!(k < ku && slot + k * S < nip)) continue;
-                    double r[4] = {0.0, 0.0, 0.0, 0.0}, rt = 0.0, rs = 0.0;
+                    // (hi, lo) FP32 pairs; FP64 once per result at the end
+                    float2 r[4], rt = make_float2(0.f, 0.f), rs = rt;
+                    const int gi = gbase + k * S;
+                    if (!SR && add_far) {
+                        load_pairs(p.out_accp + gi, r);  // the far-field pass's sums
+                    } else {
+                        r[0] = r[1] = r[2] = r[3] = rt;
+                    }
                     int n = 0;
                     for (int q = 0; q < n_js; ++q) {
                         const int src = q * S + slot;
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            const float2 v = s.acc[k][c][src];
-                            r[c] += (double)v.x + (double)v.y;
-                        }
+                        for (int c = 0; c < 4; ++c) r[c] = add_pair(r[c], s.acc[k][c][src]);
                         if constexpr (CO) {
-                            const float2 v = s.co.dtot[k][src], w = s.co.dsoft[k][src];
-                            rt += (double)v.x + (double)v.y;
-                            rs += (double)w.x + (double)w.y;
+                            rt = add_pair(rt, s.co.dtot[k][src]);
+                            rs = add_pair(rs, s.co.dsoft[k][src]);
                         }
                         n += s.cnt[k][src];
                     }
-                    const int gi = gbase + k * S;
-                    if (!SR && add_far) {  // the far-field pass's sums
-                        double f[4];
-                        far_sum(p, gi, f);
-                        for (int c = 0; c < 4; ++c) r[c] += f[c];
-                    }
                     if constexpr (CO) {
-                        // self-potential G m / r_out removed (src/hard.hpp:1663-1674)
-                        const double self = self_scale * (double)s.co.coi[k][slot].mass / r_out_walk;
-                        p.out_accp[gi] = Accp{G * r[0], G * r[1], G * r[2], G * ((r[3] + rt) + self)};
-                        p.out_pot_soft[gi] = G * ((r[3] + rs) + self);
-                    } else if constexpr (!SR) {
-                        p.out_accp[gi] = Accp{G * r[0], G * r[1], G * r[2], G * r[3]};
+                        rt = add_pair(r[3], rt);
+                        rs = add_pair(r[3], rs);
+                        if (add_self) {
+                            // self-potential G m / r_out removed (src/hard.hpp:1663-1674)
+                            const double self = (double)s.co.coi[k][slot].mass / sqrt(rcut2d);
+                            const float sh = (float)self;
+                            const float2 sp = make_float2(sh, (float)(self - (double)sh));
+                            rt = add_pair(rt, sp);
+                            rs = add_pair(rs, sp);
+                        }
+                        r[3] = rt;
+                        if (parts)
+                            reinterpret_cast<float2*>(p.out_pot_soft)[gi] = rs;
+                        else
+                            p.out_pot_soft[gi] = G * pair_value(rs);
+                    }
+                    if constexpr (!SR) {
+                        if (parts)
+                            store_pairs(p.out_accp + gi, r);
+                        else
+                            p.out_accp[gi] = Accp{G * pair_value(r[0]), G * pair_value(r[1]), G * pair_value(r[2]),
+                                                  G * pair_value(r[3])};
                     }
                     p.out_nnb[gi] = n;
                 }

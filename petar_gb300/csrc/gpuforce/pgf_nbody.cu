@@ -1081,6 +1081,7 @@ __global__ __launch_bounds__(128) void group_reduce_kernel(TreeHdr* h, const TCe
         d.rcut2 = rcut2;
         d.part = 0;
         d.n_parts = 1;
+        d.i_root = d.i_begin;
         d.root = (int32_t)g;
         d.n_spj_all = ns;
         walks[g] = d;
@@ -1435,6 +1436,7 @@ struct pgf_nbody {
     DArr<int32_t> val_in, order;
     // sorted copies
     DArr<EpiDev> epi;
+    DArr<EpiRel> epi_rel;
     DArr<EpjMix> epj;
     DArr<double> epj_m64, epj_rs64;
     DArr<EpjF32> epj32;
@@ -1575,10 +1577,11 @@ cudaError_t enqueue_force(pgf_nbody* h) {
     if (h->variant == 0) {
         e = launch_mixed(h->p, h->stream, h->num_sms);
     } else {
-        e = launch_far(h->p, h->stream, h->num_sms);
+        e = launch_epi_rel(h->p, h->epi_rel.d, h->stream, h->num_sms);
+        if (e == cudaSuccess) e = launch_far(h->p, h->stream, h->num_sms);
         if (e == cudaSuccess) e = launch_ws(h->p, h->stream, h->num_sms, h->variant - 1, nullptr);
     }
-    if (e == cudaSuccess) e = launch_retest(h->p, h->stream, h->num_sms);
+    if (e == cudaSuccess && h->variant == 0) e = launch_retest(h->p, h->stream, h->num_sms);
     return e;
 }
 
@@ -1627,6 +1630,7 @@ void bind_params(pgf_nbody* h) {
     Params& p = h->p;
     p = Params{};
     p.epi = h->epi.d;
+    p.epi_rel = h->epi_rel.d;
     p.epj = h->epj.d;
     p.epj_m64 = h->epj_m64.d;
     p.epj_rs64 = h->epj_rs64.d;
@@ -1813,6 +1817,7 @@ int pgf_nbody_create(const pgf_nbody_config* cfg, int64_t n, const double* pos, 
     NB_TRY(h->val_in.alloc(n));
     NB_TRY(h->order.alloc(n));
     NB_TRY(h->epi.alloc(n));
+    NB_TRY(h->epi_rel.alloc(n));
     NB_TRY(h->epj.alloc(n));
     NB_TRY(h->epj_m64.alloc(n));
     NB_TRY(h->epj_rs64.alloc(n));

@@ -138,6 +138,7 @@ __global__ __launch_bounds__(128) void walk_prep_kernel(int n_walk, const int64_
         }
         d.part = 0;
         d.n_parts = 1;
+        d.i_root = d.i_begin;
         d.root = w;
         d.n_spj_all = d.n_spj;
         d.rcut2 = rcut2;
