@@ -206,7 +206,7 @@ int pgf_set_dispatch_stages(int stages);
 
 /* Walk splitting in single-launch dispatches (1, the default, or 0 = off).
  * When a dispatch has few walks for the GPU's CTAs, each walk costing more
- * than a sixteenth of one SM's even share runs as up to 16 parts over slices
+ * than a sixteenth of one SM's even share runs as up to 32 parts over slices
  * of its EPJ and SPJ lists, and the parts are added in a fixed order; results then differ
  * from an unsplit launch by FP32 summation order only (counts are exact).
  * All modes; no counterpart in the reference. */

@@ -1026,13 +1026,16 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
     // Split plan.  In a single launch the most expensive walks bound the
     // launch time when there are few walks per CTA.  The unit is a sixteenth
     // of one SM's even share of the dispatch's cost; each walk that costs
-    // more than a unit runs as parts of at most a unit (at most 16 parts, at
-    // least 256 list entries each), each with a slice of its EPJ and SPJ
+    // more than a unit runs as parts of at most a unit (at most 32 parts, at
+    // least 128 list entries each, or 64 when 128 would leave CTAs without
+    // work), each with a slice of its EPJ and SPJ
     // lists and result rows of its own, and a combine kernel adds the parts up.  The kernels add per-i terms
     // (changeover self-potential, the gradient pass's a_i) in part 0 only.
     // On 200-walk batches of the 1M binary Plummer workload an eighth ran
     // the kernels 24% faster than parts of a quarter share split only above
-    // two units, and a sixteenth another 5% faster than an eighth.
+    // two units, and a sixteenth another 5% faster than an eighth.  At most
+    // 16 parts of at least 256 entries ran 700 stars in 90 us (40 us now) and
+    // 10,000 in 159 us (130 us); more and smaller parts gained nothing at 65k.
     std::vector<SplitPlan> plan;
     int64_t ni_all = ni;
     int n_desc = n_walk;
@@ -1040,12 +1043,13 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
         double total = 0.0;
         for (int k = 0; k < n_walk; ++k) total += cost(ord[k]);
         const double target = total / ((double)g.split_div * (double)g.num_sms);
+        const int64_t min_entries = (ne + ns) / 128 < 3 * (int64_t)g.num_sms ? 64 : 128;
         for (int k = 0; k < n_walk; ++k) {
             const int w = ord[k];
             const double c = cost(w);
             if (!(c > target)) break;  // the layout is sorted by cost
             const int64_t entries = (int64_t)n_epj[w] + n_spj[w];
-            const int parts = (int)std::min<double>({16.0, std::ceil(c / target), (double)(entries / 256)});
+            const int parts = (int)std::min<double>({32.0, std::ceil(c / target), (double)(entries / min_entries)});
             if (parts < 2) continue;
             plan.push_back(SplitPlan{k, parts, ni_all, n_desc});
             ni_all += (int64_t)(parts - 1) * n_epi[w];
