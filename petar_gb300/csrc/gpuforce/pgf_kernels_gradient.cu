@@ -336,7 +336,10 @@ __global__ __launch_bounds__(kThreadsG, 2) void gradient_kernel_pk(Params p) {
                         }
                     }
                     since += 2 * (j1 - j0);
-                    // Near entries, each handled by slice (index mod n_js).
+                    // Near entries, each handled by slice (index mod n_js).  A close
+                    // companion's term can exceed the rest of the sum, so it is
+                    // flushed before other pairs are rounded against it.
+                    bool any_near = false;
                     for (int wv = 0; wv < kTileEPG / 32; ++wv) {
                         unsigned m = s.nmask[wv];
                         while (m) {
@@ -410,10 +413,10 @@ __global__ __launch_bounds__(kThreadsG, 2) void gradient_kernel_pk(Params p) {
                                 g[k][1].x = fmaf(mr3, v[1], g[k][1].x);
                                 g[k][2].x = fmaf(mr3, v[2], g[k][2].x);
                             }
-                            ++since;
+                            any_near = true;
                         }
                     }
-                    if (since >= kFlushG) flush();
+                    if (any_near || since >= kFlushG) flush();
                 }
             }
             // SPJ tiles: the quadrupole force.
