@@ -32,7 +32,8 @@ using namespace pgf;
 
 constexpr int kMaxTags = 16;
 constexpr int kMaxChunks = 8;                       // pipeline stages of a large dispatch
-constexpr int64_t kChunkIdEntries = 12 << 20;       // about 48 MB of id lists per stage
+constexpr int64_t kPipelineEntries = 12 << 20;      // list entries from which a dispatch runs in stages
+constexpr int64_t kChunkIdEntries = 2 << 20;        // least list entries per stage
 constexpr int kScratchInts = 8 + kLaunchCounters * kMaxChunks;
 constexpr int kHdErrWords = 4;  // HdWalkArgs::err
 static_assert(PGF_NUM_KERNEL_VARIANTS == 1 + kNumWsVariants, "variant 0 plus the warp-specialised variants");
@@ -1018,10 +1019,20 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
     // Stages: contiguous ranges of the sorted layout.  The first has a quarter
     // of the list entries of the others, so the GPU starts sooner; the rest
     // share the remainder equally.
-    int n_chunks = g.stages > 0 ? g.stages : (int)std::min<int64_t>(kMaxChunks, (ne + ns) / kChunkIdEntries + 1);
+    // Force modes: from 12 M entries the overlap pays for the stages' copies
+    // (131k binaries, 16 M entries: 2.92 ms in one launch, 3.04 in two stages,
+    // 2.71 in eight; 65k, 5 M: 1.13 against 1.51 in four).  A neighbour search
+    // has little to overlap with: its lists are gathered from host memory
+    // faster than the host packs them (200k binaries, 27 M entries: 1.54 ms in
+    // one launch, 2.2 to 2.7 in stages), so it runs in one where that works.
+    const bool hd_walks = use_hd() && hd_walks_ok(n_walk, epi, n_epi, il, id_epj, n_epj, id_spj, n_spj, t.mode);
+    int n_chunks = g.stages;
+    if (n_chunks == 0) {
+        const bool one = ne + ns < kPipelineEntries || (t.mode == PGF_MODE_NEIGHBOR_SEARCH && hd_walks);
+        n_chunks = one ? 1 : (int)std::min<int64_t>(kMaxChunks, (ne + ns) / kChunkIdEntries + 1);
+    }
     if (n_walk < 8 * n_chunks) n_chunks = 1;
-    const bool hd_single =
-        n_chunks == 1 && use_hd() && hd_walks_ok(n_walk, epi, n_epi, il, id_epj, n_epj, id_spj, n_spj, t.mode);
+    const bool hd_single = n_chunks == 1 && hd_walks;
 
     // Split plan.  In a single launch the most expensive walks bound the
     // launch time when there are few walks per CTA.  The unit is a sixteenth
