@@ -114,6 +114,7 @@ struct TagState {
     std::vector<int64_t> epi_disp;
     DevBuf<EpiDev> epi;
     DevBuf<EpiRel> epi_rel;
+    DevBuf<AccF32> epi_acc32;
     DevBuf<int32_t> id_epj, id_spj, order;
     DevBuf<int32_t> id_spj_near;  // far-field pass: Params::id_spj_near, spj_near
     DevBuf<SpjNear> spj_near;
@@ -678,10 +679,10 @@ int launch_tag(TagState& t) {
     bind_scratch(t.params);
     if (int r = launch_kernels(t, t.params, g.stream, t.ev[1], t.ev[2])) return r;
     if (t.n_split > 0) {
-        const bool pairs = t.mode == PGF_MODE_FORCE_CHANGEOVER || t.mode == PGF_MODE_NEIGHBOR_SEARCH ||
-                           (t.mode == PGF_MODE_FORCE && t.precision == PGF_PRECISION_MIXED && t.variant != 0);
+        const bool pairs = t.mode != PGF_MODE_FORCE || (t.precision == PGF_PRECISION_MIXED && t.variant != 0);
         const cudaError_t e = launch_combine_parts(t.splits.d, t.n_split, t.params.out_accp, t.params.out_nnb,
-                                                   t.params.out_pot_soft, t.params.out_acorr, pairs, t.params.G, g.stream);
+                                                   t.params.out_pot_soft, t.params.out_acorr, t.params.epi_acc64, pairs,
+                                                   t.params.G, g.stream);
         if (e != cudaSuccess) return fail(PGF_ERR_CUDA, "combine kernel failed: %s", cudaGetErrorString(e));
     }
     PGF_CUDA(cudaEventRecord(t.ev[3], g.stream));
@@ -802,6 +803,7 @@ bool pack_walk(TagState& t, int k, int w, const Slot3& o, const void* const* epi
     d.root = k;
     d.n_spj_all = n_spj[w];
     d.rcut2 = g.walk_rcut2.empty() ? g.rcut2 : g.walk_rcut2[w];
+    set_walk_f32(d, t.mode == PGF_MODE_GRADIENT);
     t.h_walks.h[k] = d;
     t.h_order.h[k] = k;
     return bad == 0;
@@ -917,6 +919,7 @@ int dispatch_host_direct(TagState& t, int n_walk, const std::vector<int32_t>& or
     if (gr_mode) {
         a.gr_epi_off_acc = g.gr.epi_off_acc;
         a.out_epi_acc = t.epi_acc.d;
+        a.out_epi_acc32 = t.epi_acc32.d;
     }
     if (co_mode) {
         a.co_epi_off_id = g.co.epi_off_id;
@@ -1076,6 +1079,7 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
     if (gr_mode) {
         if (!hd_single) PGF_CUDA(t.h_epi_acc.ensure(ni));
         PGF_CUDA(t.epi_acc.ensure(ni));
+        PGF_CUDA(t.epi_acc32.ensure(ni));
         PGF_CUDA(t.acorr.ensure(ni_all));
     }
     if (co_mode) {
@@ -1131,6 +1135,7 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
     if (gr_mode) {
         p.epj_acc32 = g.epj_acc32.d;
         p.epi_acc64 = t.epi_acc.d;
+        p.epi_acc32 = t.epi_acc32.d;
         p.out_acorr = t.acorr.d;
     }
     if (co_mode) {
@@ -1260,7 +1265,7 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
             t.n_split = (int)plan.size();
         }
         {
-            const cudaError_t e = launch_epi_rel(t.params, t.epi_rel.d, g.stream, g.num_sms);
+            const cudaError_t e = launch_epi_rel(t.params, t.epi_rel.d, gr_mode ? t.epi_acc32.d : nullptr, g.stream, g.num_sms);
             if (e != cudaSuccess) return fail(PGF_ERR_CUDA, "EPI row kernel failed: %s", cudaGetErrorString(e));
         }
         return launch_tag(t);
@@ -1300,7 +1305,7 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
         pc.order = t.order.d + k0;
         pc.n_walk = pc.n_root = k1 - k0;
         bind_scratch(pc, c, n_chunks);
-        if (launch_epi_rel(pc, t.epi_rel.d, sc, g.num_sms) != cudaSuccess) {
+        if (launch_epi_rel(pc, t.epi_rel.d, gr_mode ? t.epi_acc32.d : nullptr, sc, g.num_sms) != cudaSuccess) {
             drain();
             return fail(PGF_ERR_CUDA, "EPI row kernel of stage %d failed", c);
         }
@@ -1834,6 +1839,7 @@ int pgf_finalize(void) {
     for (auto& t : g.tags) {
         t.epi.release();
         t.epi_rel.release();
+        t.epi_acc32.release();
         t.id_epj.release();
         t.id_spj.release();
         t.id_spj_near.release();

@@ -71,15 +71,7 @@ __global__ __launch_bounds__(256) void gather_j_kernel(HdSendArgs a) {
         a.out_epj32[j] = o;
         if (a.out_epj_acc32) {
             const double* ac = dptr(r, a.gr_epj_off_acc);
-            AccF32 g;
-            g.xh = __double2float_rn(ac[0]);
-            g.yh = __double2float_rn(ac[1]);
-            g.zh = __double2float_rn(ac[2]);
-            g.xl = __double2float_rn(__dsub_rn(ac[0], (double)g.xh));
-            g.yl = __double2float_rn(__dsub_rn(ac[1], (double)g.yh));
-            g.zl = __double2float_rn(__dsub_rn(ac[2], (double)g.zh));
-            g.pad0 = g.pad1 = 0.f;
-            a.out_epj_acc32[j] = g;
+            a.out_epj_acc32[j] = make_acc32(ac[0], ac[1], ac[2]);
         }
         if (a.out_epj_co) {
             const double status = *dptr(r, a.co_epj_off_status), mbk = *dptr(r, a.co_epj_off_mass_backup);
@@ -313,6 +305,7 @@ __global__ __launch_bounds__(kGatherThreads) void gather_walks_kernel(HdWalkArgs
             d.root = k;
             d.n_spj_all = w.n_spj;
             d.rcut2 = w.rcut2;
+            set_walk_f32(d, a.out_epi_acc != nullptr);
             // A split walk: part j takes a slice of both lists; parts >= 1
             // write result rows of their own at rows1 + (j - 1) n_i.
             for (int j = 0; j < w.parts; ++j) {
@@ -340,7 +333,9 @@ __global__ __launch_bounds__(kGatherThreads) void gather_walks_kernel(HdWalkArgs
             const double cx = __dmul_rn(0.5, __dadd_rn(red[0][0], red[3][0]));
             const double cy = __dmul_rn(0.5, __dadd_rn(red[1][0], red[4][0]));
             const double cz = __dmul_rn(0.5, __dadd_rn(red[2][0], red[5][0]));
-            a.out_epi_rel[w.i_off + i] = make_epi_rel(a.out_epi[w.i_off + i], cx, cy, cz, a.eps2);
+            const int64_t r = w.i_off + i;
+            a.out_epi_rel[r] = make_epi_rel(a.out_epi[r], cx, cy, cz, a.eps2);
+            if (a.out_epi_acc) a.out_epi_acc32[r] = make_acc32(a.out_epi_acc[r].x, a.out_epi_acc[r].y, a.out_epi_acc[r].z);
         }
         __syncthreads();
     }

@@ -13,7 +13,7 @@
 //                              traceless quadrupole and tr(q)
 //   EpiDev[ni_tot]       32 B: FP64 position and r_search
 //   id_epj / id_spj      int32 per list entry, walks concatenated
-//   WalkDesc[n_walk]     96 B: list offsets, walk centre (FP64), box
+//   WalkDesc[n_walk]    160 B: list offsets, walk centre (FP64 and FP32), box
 //                              half-extents, largest i r_search, r_out^2
 //   order[n_walk]        walks sorted by descending work (the work queue)
 //   EpiRel[ni_tot]       32 B: FP32 (hi, lo) position about the walk centre,
@@ -65,7 +65,7 @@ struct __align__(32) SpjF32 {
 };
 static_assert(sizeof(SpjF32) == 64, "SpjF32 layout");
 
-// Acceleration of one EPJ as an FP32 (hi, lo) pair (KDKDK_4TH gradient mode):
+// Acceleration of one particle as an FP32 (hi, lo) pair (KDKDK_4TH gradient mode):
 // differences a_j - a_i are formed from both halves, accurate to an ulp of
 // the difference itself.
 struct __align__(32) AccF32 {
@@ -132,6 +132,18 @@ __device__ __forceinline__ int kband_near(float D, float rs2, float eps2) {
     return k >= float(kKMax) ? kKMax : int(k) + 1;
 }
 
+__device__ __forceinline__ AccF32 make_acc32(double x, double y, double z) {
+    AccF32 g;
+    g.xh = __double2float_rn(x);
+    g.yh = __double2float_rn(y);
+    g.zh = __double2float_rn(z);
+    g.xl = __double2float_rn(__dsub_rn(x, (double)g.xh));
+    g.yl = __double2float_rn(__dsub_rn(y, (double)g.yh));
+    g.zl = __double2float_rn(__dsub_rn(z, (double)g.zh));
+    g.pad0 = g.pad1 = 0.f;
+    return g;
+}
+
 __device__ __forceinline__ EpiRel make_epi_rel(const EpiDev& e, double cx, double cy, double cz, float eps2) {
     const double dx = __dsub_rn(e.x, cx), dy = __dsub_rn(e.y, cy), dz = __dsub_rn(e.z, cz);
     EpiRel r;
@@ -176,8 +188,31 @@ struct __align__(32) WalkDesc {
     int32_t root;       // descriptor of part 0 (this one when not split)
     int32_t n_spj_all;  // SPJ of the whole walk
     int32_t i_root;     // first EPI row of the walk; i_begin is the first result row
+    // FP32 forms of the above for the kernels' passes (set_walk_f32).
+    float ch[3], cl[3];      // walk centre, hi and lo
+    float rcut2f;
+    float gr_kh, gr_kl;      // 3 / r_out^2, hi and lo (gradient mode)
+    float gr_r3;             // r_out^-3 (gradient mode)
+    float pad[6];
 };
-static_assert(sizeof(WalkDesc) == 96, "WalkDesc layout");
+static_assert(sizeof(WalkDesc) == 160, "WalkDesc layout");
+
+__host__ __device__ inline void set_walk_f32(WalkDesc& d, bool gradient) {
+    const double c[3] = {d.cx, d.cy, d.cz};
+    for (int k = 0; k < 3; ++k) {
+        d.ch[k] = (float)c[k];
+        d.cl[k] = (float)(c[k] - (double)d.ch[k]);
+    }
+    d.rcut2f = (float)d.rcut2;
+    d.gr_kh = d.gr_kl = d.gr_r3 = 0.f;
+    if (gradient) {
+        const double kd = 3.0 / d.rcut2;
+        d.gr_kh = (float)kd;
+        d.gr_kl = (float)(kd - (double)d.gr_kh);
+        d.gr_r3 = (float)(1.0 / (d.rcut2 * sqrt(d.rcut2)));
+    }
+    for (int k = 0; k < 6; ++k) d.pad[k] = 0.f;
+}
 
 // Result of one i-particle: acceleration and potential with G applied.
 struct __align__(32) Accp {
@@ -221,6 +256,7 @@ struct Params {
     double* out_pot_soft;  // fused changeover mode: soft potential (G applied)
     const AccF32* epj_acc32;  // gradient mode: EPJ accelerations (hi, lo)
     const Accp* epi_acc64;    // gradient mode: EPI accelerations (x, y, z; w unused)
+    const AccF32* epi_acc32;  // and as (hi, lo) pairs
     Accp* out_acorr;          // gradient mode: acorr (no G; w unused)
     const int32_t* id_epj;
     const int32_t* id_spj;
@@ -391,6 +427,7 @@ struct HdWalkArgs {
     EpiDev* out_epi;
     EpiRel* out_epi_rel;
     float eps2;  // of the kernels' neighbour test (guard bands)
+    AccF32* out_epi_acc32;
     Accp* out_epi_acc;
     CoRec* out_epi_co;
     int32_t* out_id_epj;
@@ -516,11 +553,13 @@ cudaError_t launch_retest(const Params& p, cudaStream_t s, int num_sms);
 // order (deterministic).
 // pot_soft and acorr (optional) are the changeover and gradient modes'
 // outputs.  pairs: the parts' rows are (hi, lo) pairs without G (the
-// warp-specialised kernels), else FP64 with G applied.
+// warp-specialised and gradient kernels; epi_acc: the latter's a_i, added
+// here), else FP64 with G applied.
 cudaError_t launch_combine_parts(const SplitRec* recs, int n_recs, Accp* accp, int32_t* nnb, double* pot_soft,
-                                 Accp* acorr, bool pairs, double G, cudaStream_t s);
-// EpiRel rows of every walk of a launch (its roots).
-cudaError_t launch_epi_rel(const Params& p, EpiRel* out, cudaStream_t s, int num_sms);
+                                 Accp* acorr, const Accp* epi_acc, bool pairs, double G, cudaStream_t s);
+// EpiRel rows of every walk of a launch (its roots), and the AccF32 forms of
+// epi_acc64 (gradient mode; null otherwise).
+cudaError_t launch_epi_rel(const Params& p, EpiRel* out, AccF32* out_acc, cudaStream_t s, int num_sms);
 // Builds the (hi, lo) FP32 copies of the EPJ / SPJ arrays.
 cudaError_t launch_split_j(const EpjMix* epj, int64_t n_epj, EpjF32* epj32, const SpjMix* spj, int64_t n_spj,
                            SpjF32* spj32, cudaStream_t s);

@@ -54,7 +54,6 @@ struct FarSmem {
     float src[kWarps][9][kRing];  // x, y, z, m, and the five quadrupole moments (QuadOp), scaled
     float red[kWarps][kPad];
     float2 lead[kWarps][4];  // rows 0 and 1 as (hi, lo)
-    float c[2][3];            // walk centre (hi, lo)
     float L[kFarCoefs + 3];
     float4 ev[kFarCoefs + 3];  // phi and gradient coefficients
     float rmax[kWarps];
@@ -147,12 +146,6 @@ __global__ __launch_bounds__(kT, 3) void far_kernel(Params p) {
             const float4 e = __ldg(reinterpret_cast<const float4*>(p.epi_rel + wd.i_root + i));
             r2m = fmaxf(r2m, fmaf(e.x, e.x, fmaf(e.y, e.y, e.z * e.z)));
         }
-        if (t < 3) {
-            const double c = t == 0 ? wd.cx : (t == 1 ? wd.cy : wd.cz);
-            const float h = (float)c;
-            s.c[0][t] = h;
-            s.c[1][t] = (float)(c - (double)h);
-        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) r2m = fmaxf(r2m, __shfl_xor_sync(0xffffffffu, r2m, o));
         if (lane == 0) s.rmax[warp] = r2m;
@@ -171,8 +164,8 @@ __global__ __launch_bounds__(kT, 3) void far_kernel(Params p) {
         const float Rs = R * inv;  // in (0.07, 0.14]
         const float lim2 = (Rs / kRhoMax) * (Rs / kRhoMax);
         const float kq = (Rs * Rs * Rs) * (Rs * Rs * Rs) / kQuadTol;
-        const float chx = s.c[0][0], chy = s.c[0][1], chz = s.c[0][2];
-        const float clx = s.c[1][0], cly = s.c[1][1], clz = s.c[1][2];
+        const float chx = wd.ch[0], chy = wd.ch[1], chz = wd.ch[2];
+        const float clx = wd.cl[0], cly = wd.cl[1], clz = wd.cl[2];
 
         float L[kFarCoefs], lo[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -320,23 +313,26 @@ __global__ __launch_bounds__(kT, 3) void far_kernel(Params p) {
 }
 
 // EPI rows about their walk's centre, one warp per walk.
-__global__ __launch_bounds__(256) void epi_rel_kernel(Params p, EpiRel* __restrict__ out) {
+__global__ __launch_bounds__(256) void epi_rel_kernel(Params p, EpiRel* __restrict__ out, AccF32* __restrict__ out_acc) {
     const int n_walk = p.n_root < p.n_walk ? p.n_root : walk_count(p);
     const int lane = threadIdx.x & 31;
     for (int k = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); k < n_walk; k += (int)((gridDim.x * blockDim.x) >> 5)) {
         const WalkDesc wd = p.walks[p.n_root < p.n_walk ? k : p.order[k]];
-        for (int i = lane; i < wd.n_i; i += 32)
-            out[wd.i_root + i] = make_epi_rel(p.epi[wd.i_root + i], wd.cx, wd.cy, wd.cz, (float)p.eps2);
+        for (int i = lane; i < wd.n_i; i += 32) {
+            const int r = wd.i_root + i;
+            out[r] = make_epi_rel(p.epi[r], wd.cx, wd.cy, wd.cz, (float)p.eps2);
+            if (out_acc) out_acc[r] = make_acc32(p.epi_acc64[r].x, p.epi_acc64[r].y, p.epi_acc64[r].z);
+        }
     }
 }
 
 }  // namespace
 
-cudaError_t launch_epi_rel(const Params& p, EpiRel* out, cudaStream_t s, int num_sms) {
+cudaError_t launch_epi_rel(const Params& p, EpiRel* out, AccF32* out_acc, cudaStream_t s, int num_sms) {
     if (p.n_walk <= 0) return cudaSuccess;
     const int64_t want = ((int64_t)(p.n_root < p.n_walk ? p.n_root : p.n_walk) + 7) / 8;
     const int grid = (int)(want < num_sms * 8 ? want : num_sms * 8);
-    epi_rel_kernel<<<grid, 256, 0, s>>>(p, out);
+    epi_rel_kernel<<<grid, 256, 0, s>>>(p, out, out_acc);
     return cudaGetLastError();
 }
 

@@ -75,7 +75,7 @@ __global__ __launch_bounds__(kT, 2) void fp64_kernel(Params p) {
         const WalkDesc wd = p.walks[p.order[wq]];
         const double rcut2 = wd.rcut2;
         const float rc2 = __double2float_ru(rcut2), rsmax2 = wd.rs_max * wd.rs_max * 1.000001f;
-        const float chx = (float)wd.cx, chy = (float)wd.cy, chz = (float)wd.cz;
+        const float chx = wd.ch[0], chy = wd.ch[1], chz = wd.ch[2];
         const float hmax = fmaxf(wd.hx, fmaxf(wd.hy, wd.hz));
         const float cmax = fmaxf(fabsf(chx), fmaxf(fabsf(chy), fabsf(chz)));
         const int n_pass = (wd.n_i + kT - 1) / kT, per_pass = n_pass ? (wd.n_i + n_pass - 1) / n_pass : 0;

@@ -18,7 +18,8 @@
 // arrays, accelerations as (hi, lo) pairs) and 256-entry SPJ tiles in shared
 // memory.  Pair arithmetic is FP32 with both halves, so dr and da are accurate
 // to an ulp of themselves for close pairs; partial sums are flushed into
-// (hi, lo) FP32 accumulators and the slices are combined in FP64.
+// (hi, lo) FP32 accumulators, and the slices are combined as such pairs: a pass
+// issues FP64 only to write its results.
 #include "pgf_internal.cuh"
 
 namespace pgf {
@@ -141,21 +142,18 @@ __global__ __launch_bounds__(kThreadsG, 2) void gradient_kernel_pk(Params p) {
         if (wq >= n_walk) break;
         const WalkDesc wd = p.walks[p.order[wq]];
         const SpjList spj = spj_list(p, wd);
-        const float chx = (float)wd.cx, chy = (float)wd.cy, chz = (float)wd.cz;
-        const float clx = (float)(wd.cx - (double)chx), cly = (float)(wd.cy - (double)chy),
-                    clz = (float)(wd.cz - (double)chz);
-        const float rcut2 = (float)wd.rcut2;
+        const float chx = wd.ch[0], chy = wd.ch[1], chz = wd.ch[2];
+        const float clx = wd.cl[0], cly = wd.cl[1], clz = wd.cl[2];
+        const float rcut2 = wd.rcut2f;
         // Near entries (possibly within r_out of an i of the walk's box):
         // their pairs run in the near loop below.  Inside r_out the distance
         // is clamped to r_out, and da - 3 (dr.da) / r_out^2 dr cancels for
         // pairs at r_out / sqrt(3) with da along dr (close binary companions);
         // those pairs are evaluated in double-float arithmetic with
-        // kdf = 3 / r_out^2 and r3c = r_out^-3 formed in FP64 here.
+        // kd = 3 / r_out^2 and r3c = r_out^-3 from the descriptor.
         const float rc = sqrtf(rcut2);
         const float hmax = fmaxf(wd.hx, fmaxf(wd.hy, wd.hz));
-        const double kd = 3.0 / wd.rcut2;
-        const float kdh = (float)kd, kdl = (float)(kd - (double)kdh);
-        const float r3c = (float)(1.0 / (wd.rcut2 * sqrt(wd.rcut2)));
+        const float kdh = wd.gr_kh, kdl = wd.gr_kl, r3c = wd.gr_r3;
         for (int ipass = 0; ipass < wd.n_i; ipass += kThreadsG * KU) {
             const int nip = min(kThreadsG * KU, wd.n_i - ipass);
             const int S = (nip + KU - 1) / KU;
@@ -172,16 +170,14 @@ __global__ __launch_bounds__(kThreadsG, 2) void gradient_kernel_pk(Params p) {
                 const int ii = li + k * S;
                 if (active && ii < nip) {
                     const int gi = wd.i_root + ipass + ii;
-                    const EpiDev e = p.epi[gi];
-                    const double d[3] = {e.x - wd.cx, e.y - wd.cy, e.z - wd.cz};
-                    const Accp a = p.epi_acc64[gi];
-                    const double aa[3] = {a.x, a.y, a.z};
+                    const float4* e = reinterpret_cast<const float4*>(p.epi_rel + gi);
+                    const float4* a = reinterpret_cast<const float4*>(p.epi_acc32 + gi);
+                    const float4 f[4] = {__ldg(e), __ldg(e + 1), __ldg(a), __ldg(a + 1)};
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        v[c] = (float)d[c];
-                        v[3 + c] = (float)(d[c] - (double)v[c]);
-                        v[6 + c] = (float)aa[c];
-                        v[9 + c] = (float)(aa[c] - (double)v[6 + c]);
+                    for (int c = 0; c < 4; ++c) {
+                        v[3 * c] = f[c].x;
+                        v[3 * c + 1] = f[c].y;
+                        v[3 * c + 2] = f[c].z;
                     }
                 }
                 nxh[k] = make_float2(-v[0], -v[0]);
@@ -265,11 +261,11 @@ __global__ __launch_bounds__(kThreadsG, 2) void gradient_kernel_pk(Params p) {
                     P[0] = hx;
                     P[2] = hy;
                     P[4] = hz;
-                    P[6] = near ? 0.f : r.m;  // near pairs run in the near loop
+                    P[6] = r.m;
                     P[8] = lx;
                     P[10] = ly;
                     P[12] = lz;
-                    P[14] = 0.f;
+                    P[14] = near ? 1.f : 0.f;
                     float* A = reinterpret_cast<float*>(&s.A[tid >> 1][0]) + (tid & 1);
                     A[0] = a.xh;
                     A[2] = a.yh;
@@ -300,6 +296,7 @@ __global__ __launch_bounds__(kThreadsG, 2) void gradient_kernel_pk(Params p) {
                         const float2 Zh = make_float2(p1.x, p1.y), M = make_float2(p1.z, p1.w);
                         const float2 Xl = make_float2(p2.x, p2.y), Yl = make_float2(p2.z, p2.w);
                         const float2 Zl = make_float2(p3.x, p3.y);
+                        const bool near2 = (p3.z != 0.f) | (p3.w != 0.f);  // same for all threads of a slice
                         const float2 AXh = make_float2(a0.x, a0.y), AYh = make_float2(a0.z, a0.w);
                         const float2 AZh = make_float2(a1.x, a1.y), AXl = make_float2(a1.z, a1.w);
                         const float2 AYl = make_float2(a2.x, a2.y), AZl = make_float2(a2.z, a2.w);
@@ -324,6 +321,14 @@ __global__ __launch_bounds__(kThreadsG, 2) void gradient_kernel_pk(Params p) {
                                 ri2 = __fmul2_rn(ri, ri);
                                 mr3 = __fmul2_rn(__fmul2_rn(M, ri), ri2);
                             }
+                            if (near2) {
+                                // pairs inside r_out run in the near loop (the same test there)
+                                float2 r2 = __ffma2_rn(dx, dx, e2);
+                                r2 = __ffma2_rn(dy, dy, r2);
+                                r2 = __ffma2_rn(dz, dz, r2);
+                                if (p3.z != 0.f && r2.x < rcut2) mr3.x = 0.f;
+                                if (p3.w != 0.f && r2.y < rcut2) mr3.y = 0.f;
+                            }
                             const float2 drda = __ffma2_rn(dx, dax, __ffma2_rn(dy, day, __fmul2_rn(dz, daz)));
                             // -alpha = -3 (dr.da) / r^2
                             const float2 nal_ = __fmul2_rn(__fmul2_rn(drda, ri2), make_float2(-3.f, -3.f));
@@ -336,9 +341,10 @@ __global__ __launch_bounds__(kThreadsG, 2) void gradient_kernel_pk(Params p) {
                         }
                     }
                     since += 2 * (j1 - j0);
-                    // Near entries, each handled by slice (index mod n_js).  A close
-                    // companion's term can exceed the rest of the sum, so it is
-                    // flushed before other pairs are rounded against it.
+                    // Near entries, each handled by slice (index mod n_js): their
+                    // pairs inside r_out.  A close companion's term can exceed
+                    // the rest of the sum, so it is flushed before other pairs
+                    // are rounded against it.
                     bool any_near = false;
                     for (int wv = 0; wv < kTileEPG / 32; ++wv) {
                         unsigned m = s.nmask[wv];
@@ -354,66 +360,44 @@ __global__ __launch_bounds__(kThreadsG, 2) void gradient_kernel_pk(Params p) {
                                 const float d0 = (q0.x + nxh[k].x) + (q1.x + nxl[k].x);
                                 const float d1 = (q0.y + nyh[k].x) + (q1.y + nyl[k].x);
                                 const float d2 = (q0.z + nzh[k].x) + (q1.z + nzl[k].x);
-                                const float r2 = fmaf(d0, d0, fmaf(d1, d1, fmaf(d2, d2, eps2)));
-                                float v[3], mr3;
-                                if (r2 < rcut2) {
-                                    // clamped: v = da - (3 / r_out^2)(dr.da) dr in double-float
-                                    float dh[3], dl[3], ah[3], al[3];
-                                    df_diff(q0.x, q1.x, nxh[k].x, nxl[k].x, dh[0], dl[0]);
-                                    df_diff(q0.y, q1.y, nyh[k].x, nyl[k].x, dh[1], dl[1]);
-                                    df_diff(q0.z, q1.z, nzh[k].x, nzl[k].x, dh[2], dl[2]);
-                                    df_diff(q2.x, q3.x, nah[k][0].x, nal[k][0].x, ah[0], al[0]);
-                                    df_diff(q2.y, q3.y, nah[k][1].x, nal[k][1].x, ah[1], al[1]);
-                                    df_diff(q2.z, q3.z, nah[k][2].x, nal[k][2].x, ah[2], al[2]);
-                                    float sh = 0.f, sl = 0.f;
+                                const float r2 = fmaf(d2, d2, fmaf(d1, d1, fmaf(d0, d0, eps2)));
+                                if (!(r2 < rcut2)) continue;  // done in the packed loop
+                                float v[3];
+                                // clamped: v = da - (3 / r_out^2)(dr.da) dr in double-float
+                                float dh[3], dl[3], ah[3], al[3];
+                                df_diff(q0.x, q1.x, nxh[k].x, nxl[k].x, dh[0], dl[0]);
+                                df_diff(q0.y, q1.y, nyh[k].x, nyl[k].x, dh[1], dl[1]);
+                                df_diff(q0.z, q1.z, nzh[k].x, nzl[k].x, dh[2], dl[2]);
+                                df_diff(q2.x, q3.x, nah[k][0].x, nal[k][0].x, ah[0], al[0]);
+                                df_diff(q2.y, q3.y, nah[k][1].x, nal[k][1].x, ah[1], al[1]);
+                                df_diff(q2.z, q3.z, nah[k][2].x, nal[k][2].x, ah[2], al[2]);
+                                float sh = 0.f, sl = 0.f;
 #pragma unroll
-                                    for (int c = 0; c < 3; ++c) {
-                                        float pp, pe, t1, t2;
-                                        two_prod_g(dh[c], ah[c], pp, pe);
-                                        pe = fmaf(dh[c], al[c], fmaf(dl[c], ah[c], pe));
-                                        two_sum_g(sh, pp, t1, t2);
-                                        sh = t1;
-                                        sl += t2 + pe;
-                                    }
-                                    float alh, ale;
-                                    two_prod_g(kdh, sh, alh, ale);
-                                    ale = fmaf(kdh, sl, fmaf(kdl, sh, ale));
-#pragma unroll
-                                    for (int c = 0; c < 3; ++c) {
-                                        float qh, qe, vh, ve;
-                                        two_prod_g(alh, dh[c], qh, qe);
-                                        qe = fmaf(alh, dl[c], fmaf(ale, dh[c], qe));
-                                        two_sum_g(ah[c], -qh, vh, ve);
-                                        v[c] = vh + (ve + (al[c] - qe));
-                                    }
-                                    mr3 = q0.w * r3c;
-                                } else {
-                                    const float e0 = (q2.x + nah[k][0].x) + (q3.x + nal[k][0].x);
-                                    const float e1 = (q2.y + nah[k][1].x) + (q3.y + nal[k][1].x);
-                                    const float e2_ = (q2.z + nah[k][2].x) + (q3.z + nal[k][2].x);
-                                    float ri2;
-                                    if constexpr (CMP) {
-                                        float2 m2, r22;
-                                        far_r3_compensated(make_float2(d0, d0), make_float2(d1, d1),
-                                                           make_float2(d2, d2), make_float2(eps2, eps2),
-                                                           make_float2(q0.w, q0.w), rcut2, m2, r22);
-                                        mr3 = m2.x;
-                                        ri2 = r22.x;
-                                    } else {
-                                        const float ri = rsqrt_approx_g(r2);
-                                        ri2 = ri * ri;
-                                        mr3 = (q0.w * ri) * ri2;
-                                    }
-                                    const float nl3 = -3.f * (fmaf(d0, e0, fmaf(d1, e1, d2 * e2_)) * ri2);
-                                    v[0] = fmaf(nl3, d0, e0);
-                                    v[1] = fmaf(nl3, d1, e1);
-                                    v[2] = fmaf(nl3, d2, e2_);
+                                for (int c = 0; c < 3; ++c) {
+                                    float pp, pe, t1, t2;
+                                    two_prod_g(dh[c], ah[c], pp, pe);
+                                    pe = fmaf(dh[c], al[c], fmaf(dl[c], ah[c], pe));
+                                    two_sum_g(sh, pp, t1, t2);
+                                    sh = t1;
+                                    sl += t2 + pe;
                                 }
+                                float alh, ale;
+                                two_prod_g(kdh, sh, alh, ale);
+                                ale = fmaf(kdh, sl, fmaf(kdl, sh, ale));
+#pragma unroll
+                                for (int c = 0; c < 3; ++c) {
+                                    float qh, qe, vh, ve;
+                                    two_prod_g(alh, dh[c], qh, qe);
+                                    qe = fmaf(alh, dl[c], fmaf(ale, dh[c], qe));
+                                    two_sum_g(ah[c], -qh, vh, ve);
+                                    v[c] = vh + (ve + (al[c] - qe));
+                                }
+                                const float mr3 = q0.w * r3c;
                                 g[k][0].x = fmaf(mr3, v[0], g[k][0].x);
                                 g[k][1].x = fmaf(mr3, v[1], g[k][1].x);
                                 g[k][2].x = fmaf(mr3, v[2], g[k][2].x);
+                                any_near = true;
                             }
-                            any_near = true;
                         }
                     }
                     if (any_near || since >= kFlushG) flush();
@@ -497,22 +481,28 @@ __global__ __launch_bounds__(kThreadsG, 2) void gradient_kernel_pk(Params p) {
                     const int ii = li + k * S;
                     if (ii >= nip) continue;
                     const int gi = wd.i_begin + ipass + ii;
-                    double r[7] = {0, 0, 0, 0, 0, 0, 0};
+                    // (hi, lo) FP32 pairs; FP64 once per result at the end, and
+                    // for a split walk's parts only where they are combined
+                    float2 r[7];
+#pragma unroll
+                    for (int c = 0; c < 7; ++c) r[c] = make_float2(0.f, 0.f);
+                    if (spj.add_far) load_pairs(p.out_accp + gi, r + 3);  // the far-field pass's sums
                     for (int q = 0; q < n_js; ++q) {
                         const int src = q * S + li;
 #pragma unroll
-                        for (int c = 0; c < 7; ++c) r[c] += (double)s.acc[k][c][src].x + (double)s.acc[k][c][src].y;
+                        for (int c = 0; c < 7; ++c) r[c] = add_pair(r[c], s.acc[k][c][src]);
                     }
-                    if (spj.add_far) {  // the far-field pass's sums
-                        float2 f[4];
-                        load_pairs(p.out_accp + gi, f);
-                        for (int c = 0; c < 4; ++c) r[3 + c] += pair_value(f[c]);
+                    if (wd.n_parts > 1) {
+                        const float2 ac[4] = {r[0], r[1], r[2], make_float2(0.f, 0.f)};
+                        store_pairs(p.out_acorr + gi, ac);
+                        store_pairs(p.out_accp + gi, r + 3);
+                    } else {
+                        const Accp a = p.epi_acc64[gi];
+                        const double G = p.G;
+                        p.out_acorr[gi] = Accp{2.0 * pair_value(r[0]), 2.0 * pair_value(r[1]), 2.0 * pair_value(r[2]), 0.0};
+                        p.out_accp[gi] = Accp{a.x + G * pair_value(r[3]), a.y + G * pair_value(r[4]),
+                                              a.z + G * pair_value(r[5]), G * pair_value(r[6])};
                     }
-                    // a_i once: parts of a split walk add their pairs only
-                    const Accp a = wd.part == 0 ? p.epi_acc64[wd.i_root + ipass + ii] : Accp{0.0, 0.0, 0.0, 0.0};
-                    const double G = p.G;
-                    p.out_acorr[gi] = Accp{2.0 * r[0], 2.0 * r[1], 2.0 * r[2], 0.0};
-                    p.out_accp[gi] = Accp{a.x + G * r[3], a.y + G * r[4], a.z + G * r[5], G * r[6]};
                     p.out_nnb[gi] = 0;
                 }
             }

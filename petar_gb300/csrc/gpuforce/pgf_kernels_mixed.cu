@@ -560,13 +560,15 @@ cudaError_t launch_mixed(const Params& p, cudaStream_t s, int num_sms) {
 // rows, and the loads of four parts are in flight at once.
 template <bool PAIRS>
 __global__ __launch_bounds__(128) void combine_parts_kernel(const SplitRec* __restrict__ recs, Accp* accp,
-                                                            int32_t* nnb, double* pot_soft, Accp* acorr, double G) {
+                                                            int32_t* nnb, double* pot_soft, Accp* acorr,
+                                                            const Accp* __restrict__ epi_acc, double G) {
     const SplitRec r = recs[blockIdx.x];
     for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < r.n_i; i += gridDim.y * blockDim.x) {
         const int64_t r0 = (int64_t)r.row0 + i;
         if constexpr (PAIRS) {
-            float2 a[4], ps = make_float2(0.f, 0.f);
+            float2 a[4], g[4], ps = make_float2(0.f, 0.f);
             load_pairs(accp + r0, a);
+            if (acorr) load_pairs(acorr + r0, g);
             int c = nnb[r0];
             const float2* soft = reinterpret_cast<const float2*>(pot_soft);
             if (pot_soft) ps = soft[r0];
@@ -579,14 +581,26 @@ __global__ __launch_bounds__(128) void combine_parts_kernel(const SplitRec* __re
                 for (int q = 0; q < 4; ++q) a[q] = add_pair(a[q], b[q]);
                 c += nnb[row];
                 if (pot_soft) ps = add_pair(ps, soft[row]);
+                if (acorr) {
+                    load_pairs(acorr + row, b);
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) g[q] = add_pair(g[q], b[q]);
+                }
             }
-            accp[r0] = Accp{G * pair_value(a[0]), G * pair_value(a[1]), G * pair_value(a[2]), G * pair_value(a[3])};
+            Accp v{G * pair_value(a[0]), G * pair_value(a[1]), G * pair_value(a[2]), G * pair_value(a[3])};
+            if (acorr) {  // gradient mode: a_i once
+                const Accp e = epi_acc[r0];
+                v.x += e.x;
+                v.y += e.y;
+                v.z += e.z;
+                acorr[r0] = Accp{2.0 * pair_value(g[0]), 2.0 * pair_value(g[1]), 2.0 * pair_value(g[2]), 0.0};
+            }
+            accp[r0] = v;
             nnb[r0] = c;
             if (pot_soft) pot_soft[r0] = G * pair_value(ps);
         } else {
             Accp a = accp[r0];
             int c = nnb[r0];
-            Accp g = acorr ? acorr[r0] : Accp{0.0, 0.0, 0.0, 0.0};
 #pragma unroll 4
             for (int k = 1; k < r.n_parts; ++k) {
                 const int64_t row = (int64_t)r.rows1 + (int64_t)(k - 1) * r.n_i + i;
@@ -596,28 +610,21 @@ __global__ __launch_bounds__(128) void combine_parts_kernel(const SplitRec* __re
                 a.z += b.z;
                 a.w += b.w;
                 c += nnb[row];
-                if (acorr) {
-                    const Accp h = acorr[row];
-                    g.x += h.x;
-                    g.y += h.y;
-                    g.z += h.z;
-                }
             }
             accp[r0] = a;
             nnb[r0] = c;
-            if (acorr) acorr[r0] = g;
         }
     }
 }
 
 cudaError_t launch_combine_parts(const SplitRec* recs, int n_recs, Accp* accp, int32_t* nnb, double* pot_soft,
-                                 Accp* acorr, bool pairs, double G, cudaStream_t s) {
+                                 Accp* acorr, const Accp* epi_acc, bool pairs, double G, cudaStream_t s) {
     if (n_recs <= 0) return cudaSuccess;
     const dim3 grid(n_recs, 2);
     if (pairs)
-        combine_parts_kernel<true><<<grid, 128, 0, s>>>(recs, accp, nnb, pot_soft, acorr, G);
+        combine_parts_kernel<true><<<grid, 128, 0, s>>>(recs, accp, nnb, pot_soft, acorr, epi_acc, G);
     else
-        combine_parts_kernel<false><<<grid, 128, 0, s>>>(recs, accp, nnb, pot_soft, acorr, G);
+        combine_parts_kernel<false><<<grid, 128, 0, s>>>(recs, accp, nnb, pot_soft, acorr, epi_acc, G);
     return cudaGetLastError();
 }
 

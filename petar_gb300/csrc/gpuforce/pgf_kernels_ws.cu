@@ -348,10 +348,9 @@ __device__ void producer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
         const int widx = p.order[w_q];
         const WalkDesc wd = p.walks[widx];
         // Walk centre as an FP32 (hi, lo) pair.
-        const float chx = (float)wd.cx, chy = (float)wd.cy, chz = (float)wd.cz;
-        const float clx = (float)(wd.cx - (double)chx), cly = (float)(wd.cy - (double)chy),
-                    clz = (float)(wd.cz - (double)chz);
-        const float rcut2 = (float)wd.rcut2;
+        const float chx = wd.ch[0], chy = wd.ch[1], chz = wd.ch[2];
+        const float clx = wd.cl[0], cly = wd.cl[1], clz = wd.cl[2];
+        const float rcut2 = wd.rcut2f;
         const float rsmax2 = wd.rs_max * wd.rs_max;
         const float hmax = fmaxf(wd.hx, fmaxf(wd.hy, wd.hz));
         const int n_ept = (wd.n_epj + kTileEP - 1) / kTileEP;
@@ -1022,7 +1021,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
         if (h.kind == kItemExit) return;
         if (h.kind == kItemBegin) {
             const WalkDesc wd = p.walks[h.walk];
-            rcut2 = (float)wd.rcut2;
+            rcut2 = wd.rcut2f;
             nip = min(kMaxPass, wd.n_i - h.ipass);
             ku = KI;
             if constexpr (KA < KI) {

@@ -1084,6 +1084,7 @@ __global__ __launch_bounds__(128) void group_reduce_kernel(TreeHdr* h, const TCe
         d.i_root = d.i_begin;
         d.root = (int32_t)g;
         d.n_spj_all = ns;
+        set_walk_f32(d, false);
         walks[g] = d;
         cnt_e[g] = ne;
         cnt_s[g] = ns;
@@ -1577,7 +1578,7 @@ cudaError_t enqueue_force(pgf_nbody* h) {
     if (h->variant == 0) {
         e = launch_mixed(h->p, h->stream, h->num_sms);
     } else {
-        e = launch_epi_rel(h->p, h->epi_rel.d, h->stream, h->num_sms);
+        e = launch_epi_rel(h->p, h->epi_rel.d, nullptr, h->stream, h->num_sms);
         if (e == cudaSuccess) e = launch_far(h->p, h->stream, h->num_sms);
         if (e == cudaSuccess) e = launch_ws(h->p, h->stream, h->num_sms, h->variant - 1, nullptr);
     }

@@ -142,6 +142,7 @@ __global__ __launch_bounds__(128) void walk_prep_kernel(int n_walk, const int64_
         d.root = w;
         d.n_spj_all = d.n_spj;
         d.rcut2 = rcut2;
+        set_walk_f32(d, false);
         desc[w] = d;
         order[w] = w;
     }
