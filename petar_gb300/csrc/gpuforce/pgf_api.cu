@@ -1153,6 +1153,7 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
     p.order = t.order.d;
     p.n_walk = n_desc;
     p.n_root = n_walk;
+    p.flush_tiles = !g.walk_split && ni <= kPlanRows ? 1 : 0;
     p.gr_compensated = g.gr_compensated;
     // The neighbour search tests r^2 < max(rs_i, rs_j)^2 without softening
     // (src/soft_force.hpp:11-34); the force kernels include eps^2.

@@ -295,6 +295,12 @@ struct Params {
     // per walk (by root descriptor) what they hold.
     int32_t* id_spj_near;
     SpjNear* spj_near;
+    // Parts of split walks start at multiples of this many entries of the
+    // compacted list (0: 1).
+    int32_t part_align;
+    // Partial sums are flushed at every tile's end, so that whole walks and
+    // walks in parts of whole tiles add the same FP32 terms.
+    int32_t flush_tiles;
     // Walks without their further parts: when some are split (n_root <
     // n_walk) the roots are descriptors 0 .. n_root - 1 by descending cost.
     int32_t n_root;
@@ -479,6 +485,20 @@ inline cudaError_t reset_counters(const Params& p, cudaStream_t s) {
 constexpr int64_t kFarMinRows = 8192;
 inline bool far_applies(double eps2, int64_t n_i) { return eps2 == 0.0 && n_i >= kFarMinRows; }
 
+// Tile of the default pair kernel: the parts of a device plan start at
+// multiples of it.
+constexpr int kPartAlign = 256;
+// Launches with more i-particles than this run their walks whole in the
+// device-resident step (they have enough of them: a King model of 1M has
+// 7,000 walks for 456 CTAs); up to it, whole walks flush at tile ends.
+constexpr int64_t kPlanRows = 400000;
+
+// First entry of part j of n entries in n_parts parts.
+__host__ __device__ inline int part_begin(int64_t n, int j, int n_parts, int align) {
+    const int64_t units = (n + align - 1) / align, b = units * j / n_parts * align;
+    return (int)(b < n ? b : n);
+}
+
 // A result row as four (hi, lo) FP32 pairs, without G: the far-field sums
 // (acceleration x, y, z and potential) and the sums of a split walk's parts.
 __device__ __forceinline__ void load_pairs(const Accp* row, float2 f[4]) {
@@ -519,7 +539,8 @@ __device__ __forceinline__ SpjList spj_list(const Params& p, const WalkDesc& wd)
         const SpjNear c = p.spj_near[wd.root];
         if (c.n[0] >= 0) {
             const int64_t all = wd.n_spj_all;
-            l.ids = p.id_spj_near + (wd.spj_begin - (int)(all * wd.part / wd.n_parts));
+            const int align = p.part_align ? p.part_align : 1;
+            l.ids = p.id_spj_near + (wd.spj_begin - part_begin(all, wd.part, wd.n_parts, align));
             l.after1 = c.n[0];
             l.after2 = l.after1 + c.n[1];
             l.after3 = l.after2 + c.n[2];
@@ -527,8 +548,8 @@ __device__ __forceinline__ SpjList spj_list(const Params& p, const WalkDesc& wd)
             l.gap2 = (int)(all * 2 / 4) - l.after2;
             l.gap3 = (int)(all * 3 / 4) - l.after3;
             const int64_t total = l.after3 + c.n[3];
-            l.begin = (int)(total * wd.part / wd.n_parts);
-            l.n = (int)(total * (wd.part + 1) / wd.n_parts) - l.begin;
+            l.begin = part_begin(total, wd.part, wd.n_parts, align);
+            l.n = part_begin(total, wd.part + 1, wd.n_parts, align) - l.begin;
             l.add_far = c.add_far != 0 && wd.part == 0;
             return l;
         }
@@ -549,6 +570,24 @@ cudaError_t launch_far(const Params& p, cudaStream_t s, int num_sms);
 cudaError_t launch_fp64(const Params& p, cudaStream_t s, int num_sms);
 cudaError_t launch_mixed(const Params& p, cudaStream_t s, int num_sms);
 cudaError_t launch_retest(const Params& p, cudaStream_t s, int num_sms);
+// Split plan made on the device (pgf_plan.cu).  cap_splits bounds the further
+// parts, row0 is the first of cap_rows result rows for them.
+struct PlanArgs {
+    const WalkDesc* roots;
+    int n_root;
+    const int32_t* n_root_dev;  // walk count on the device (at most n_root), or null
+    const SpjNear* spj_near;    // far-field pass, or null
+    int num_sms;
+    WalkDesc* walks;
+    int32_t* order;
+    SplitRec* splits;
+    int32_t* n_desc;
+    int32_t* n_split;
+    int cap_desc, cap_splits, row0;
+    int64_t cap_rows;
+};
+cudaError_t launch_plan(const PlanArgs& a, cudaStream_t s);
+cudaError_t launch_combine_plan(const PlanArgs& a, Accp* accp, int32_t* nnb, double G, cudaStream_t s);
 // Adds the results of every split walk's parts into its own rows, parts in
 // order (deterministic).
 // pot_soft and acorr (optional) are the changeover and gradient modes'

@@ -656,6 +656,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
     constexpr int kMaxPass = CT * KI;
     constexpr int KA = KI > 1 ? KI - 1 : 1;  // the other i-per-thread count a pass may use
     const float eps2 = (float)p.eps2;
+    const bool flush_tiles = p.flush_tiles != 0;
     unsigned item = 0;
 
     // Pass state.  A pass runs ku (KA or KI) i-particles per thread, whichever
@@ -1084,7 +1085,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
                     ep_tile(IntC<KI>{}, h, sl);
                 else if constexpr (KA < KI)
                     ep_tile(IntC<KA>{}, h, sl);
-                if (since >= kFlush) flush();
+                if (since >= kFlush || flush_tiles) flush();
             }
         } else if (h.kind == kItemSP) {
             if (active) {
@@ -1092,7 +1093,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
                     sp_tile(IntC<KI>{}, h, sl);
                 else if constexpr (KA < KI)
                     sp_tile(IntC<KA>{}, h, sl);
-                if (since >= kFlush) flush();
+                if (since >= kFlush || flush_tiles) flush();
             }
         } else {  // kItemEnd: reduce the j-slices of the pass and write
             if (active) flush();

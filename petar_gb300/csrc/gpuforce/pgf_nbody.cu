@@ -1469,9 +1469,15 @@ struct pgf_nbody {
     DArr<int32_t> id_spj_near;  // far-field pass (far_applies): the compacted lists and their lengths
     DArr<SpjNear> spj_near;
     // force scratch and results
+    // split plan of launches with few walks (kPlanRows)
+    DArr<WalkDesc> plan_walks;
+    DArr<int32_t> plan_order;
+    DArr<SplitRec> splits;
+    int64_t plan_rows = 0;  // result rows beyond n
+    bool planned() const { return plan_rows > 0; }
     DArr<Accp> out_accp;
     DArr<int32_t> out_nnb;
-    DArr<int32_t> flags;  // [2] kernel error word, [4..6] launch counters
+    DArr<int32_t> flags;  // [0], [1] descriptors and split walks of the plan, [2] kernel error word, [4..6] launch counters
     DArr<Retest> retest;
     int retest_cap = 1 << 20;
     DArr<TreeHdr> hdr;
@@ -1571,6 +1577,25 @@ cudaError_t enqueue_build(pgf_nbody* h) {
     return cudaGetLastError();
 }
 
+PlanArgs plan_args(pgf_nbody* h) {
+    PlanArgs a{};
+    a.roots = h->walks.d;
+    a.n_root = (int)h->n;
+    a.n_root_dev = &h->hdr.d->n_walk;
+    a.spj_near = h->p.spj_near;
+    a.num_sms = h->num_sms;
+    a.walks = h->plan_walks.d;
+    a.order = h->plan_order.d;
+    a.splits = h->splits.d;
+    a.n_desc = h->flags.d;
+    a.n_split = h->flags.d + 1;
+    a.cap_desc = (int)h->plan_walks.n;
+    a.cap_splits = (int)h->splits.n;
+    a.row0 = (int)h->n;
+    a.cap_rows = h->plan_rows;
+    return a;
+}
+
 cudaError_t enqueue_force(pgf_nbody* h) {
     cudaError_t e = reset_counters(h->p, h->stream);
     if (e != cudaSuccess) return e;
@@ -1580,7 +1605,19 @@ cudaError_t enqueue_force(pgf_nbody* h) {
     } else {
         e = launch_epi_rel(h->p, h->epi_rel.d, nullptr, h->stream, h->num_sms);
         if (e == cudaSuccess) e = launch_far(h->p, h->stream, h->num_sms);
-        if (e == cudaSuccess) e = launch_ws(h->p, h->stream, h->num_sms, h->variant - 1, nullptr);
+        if (e == cudaSuccess && h->planned()) {
+            const PlanArgs a = plan_args(h);
+            Params p = h->p;
+            p.walks = h->plan_walks.d;
+            p.order = h->plan_order.d;
+            p.n_walk = a.cap_desc;
+            p.n_walk_dev = a.n_desc;
+            e = launch_plan(a, h->stream);
+            if (e == cudaSuccess) e = launch_ws(p, h->stream, h->num_sms, h->variant - 1, nullptr);
+            if (e == cudaSuccess) e = launch_combine_plan(a, p.out_accp, p.out_nnb, p.G, h->stream);
+        } else if (e == cudaSuccess) {
+            e = launch_ws(h->p, h->stream, h->num_sms, h->variant - 1, nullptr);
+        }
     }
     if (e == cudaSuccess && h->variant == 0) e = launch_retest(h->p, h->stream, h->num_sms);
     return e;
@@ -1651,6 +1688,8 @@ void bind_params(pgf_nbody* h) {
     p.out_accp = h->out_accp.d;
     p.out_nnb = h->out_nnb.d;
     bind_counters(p, h->flags.d + 4);
+    p.part_align = kPartAlign;
+    p.flush_tiles = h->planned() ? 1 : 0;
     if (far_applies(h->cfg.eps2, h->n)) {
         p.id_spj_near = h->id_spj_near.d;
         p.spj_near = h->spj_near.d;
@@ -1836,8 +1875,17 @@ int pgf_nbody_create(const pgf_nbody_config* cfg, int64_t n, const double* pos, 
     NB_TRY(alloc_spj(h));
     if (far_applies(cfg->eps2, n)) NB_TRY(h->spj_near.alloc(n));
     NB_TRY(h->blocksum.alloc(kLevelBlocks));
-    NB_TRY(h->out_accp.alloc(n));
-    NB_TRY(h->out_nnb.alloc(n));
+    if (n <= kPlanRows) {
+        // Parts cost at most a sixteenth of an SM's share each beyond one per
+        // walk, so there are at most 16 num_sms further ones.
+        const int64_t extra = 16 * (int64_t)h->num_sms;
+        h->plan_rows = std::min<int64_t>(extra * std::max(cfg->n_group_limit, cfg->n_leaf_limit), 4 << 20);
+        NB_TRY(h->plan_walks.alloc(n + extra));
+        NB_TRY(h->plan_order.alloc(n + extra));
+        NB_TRY(h->splits.alloc(extra));
+    }
+    NB_TRY(h->out_accp.alloc(n + h->plan_rows));
+    NB_TRY(h->out_nnb.alloc(n + h->plan_rows));
     NB_TRY(h->flags.alloc(8));
     NB_TRY(h->retest.alloc(h->retest_cap));
     NB_TRY(h->hdr.alloc(1));
