@@ -331,8 +331,8 @@ const char *pgf_last_error(void);
  * other allocating routine.
  *
  * The mixed-precision kernels still need scratch (walk descriptors, work
- * order, queue cursor, FP64 re-test records).  It lives in one static device
- * array of about 2.6 MB that every GPU loading the library keeps until the
+ * order, queue cursor, result rows of the parts that expensive walks are
+ * split into).  It lives in one static device array of about 15 MB that every GPU loading the library keeps until the
  * process exits, sized for at most PGF_NOALLOC_MAX_WALKS walks per call;
  * larger calls return PGF_ERR_CAPACITY.  The first call on each device looks
  * up that array's device address (with the device current) and keeps it; make
@@ -346,8 +346,9 @@ const char *pgf_last_error(void);
  * device first, and the call copies the check's result to the host and waits
  * on the stream for it (so it also waits for the work queued on the stream
  * before it) before it launches the force kernels.  Those are then left
- * running on the stream.  They contain no waits and report no device errors,
- * so the check is the only device-side failure the call can report.
+ * running on the stream.  Their waits are bounded (1 s); should one run out,
+ * the next call reports it as PGF_ERR_DEVICE, and the results of the call that
+ * it happened in are not complete.
  *
  * walk_table: 6 int64 per walk: i_begin, n_i, epj_begin, n_epj, spj_begin,
  *   n_spj (rows of epi; offsets into id_epj / id_spj).

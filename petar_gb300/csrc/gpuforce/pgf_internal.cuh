@@ -158,6 +158,25 @@ __device__ __forceinline__ EpiRel make_epi_rel(const EpiDev& e, double cx, doubl
     return r;
 }
 
+// An FP64 value as FP32 (hi, lo) without the FP64 pipe: hi the leading 24 bits,
+// lo the other 29 rounded to 24 (hi + lo to 2^-48 of it).  Values below 2^-74
+// lose lo, values below 2^-126 are 0, those beyond FP32's range infinite.
+__device__ __forceinline__ void split_f64(unsigned blo, unsigned bhi, float& h, float& l) {
+    const int e = (int)((bhi >> 20) & 0x7ffu);
+    const unsigned sign = bhi & 0x80000000u;
+    const unsigned m23 = ((bhi & 0xfffffu) << 3) | (blo >> 29);
+    unsigned hb = sign | ((unsigned)(e - 896) << 23) | m23;
+    float scale = __uint_as_float(sign | ((unsigned)(e - 948) << 23));
+    if (e < 949) scale = 0.f;
+    if (e < 897) hb = sign;
+    if (e > 1150) {  // infinities and NaN included
+        hb = sign | 0x7f800000u | ((e == 0x7ff && (m23 | blo)) ? 0x400000u : 0u);
+        scale = 0.f;
+    }
+    h = __uint_as_float(hb);
+    l = scale * (float)(blo & 0x1fffffffu);
+}
+
 // Error-free sum: s + e == a + b exactly (round-to-nearest, no reassociation).
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
     s = a + b;
@@ -268,6 +287,10 @@ struct Params {
     double G;
     Accp* out_accp;
     int32_t* out_nnb;
+    // Bases of the result rows of parts >= 1 of split walks (null: out_accp,
+    // out_nnb).
+    Accp* part_accp;
+    int32_t* part_nnb;
     // scratch
     // Launch counters, kLaunchCounters ints that lie together and are zeroed
     // before each launch (reset_counters): the work-queue cursor, the number
@@ -571,7 +594,7 @@ cudaError_t launch_fp64(const Params& p, cudaStream_t s, int num_sms);
 cudaError_t launch_mixed(const Params& p, cudaStream_t s, int num_sms);
 cudaError_t launch_retest(const Params& p, cudaStream_t s, int num_sms);
 // Split plan made on the device (pgf_plan.cu).  cap_splits bounds the further
-// parts, row0 is the first of cap_rows result rows for them.
+// parts, row0 is the first of cap_rows result rows for them (in part_accp).
 struct PlanArgs {
     const WalkDesc* roots;
     int n_root;
@@ -587,7 +610,7 @@ struct PlanArgs {
     int64_t cap_rows;
 };
 cudaError_t launch_plan(const PlanArgs& a, cudaStream_t s);
-cudaError_t launch_combine_plan(const PlanArgs& a, Accp* accp, int32_t* nnb, double G, cudaStream_t s);
+cudaError_t launch_combine_plan(const PlanArgs& a, const Params& p, cudaStream_t s);
 // Adds the results of every split walk's parts into its own rows, parts in
 // order (deterministic).
 // pot_soft and acorr (optional) are the changeover and gradient modes'
@@ -612,6 +635,9 @@ struct TensorMaps {
     bool valid = false;
 };
 cudaError_t launch_ws(const Params& p, cudaStream_t s, int num_sms, int variant, const TensorMaps* tm);
+// The default variant on FP64 records alone (epi, EpjMix, SpjMix), for callers
+// whose data has no FP32 forms.
+cudaError_t launch_ws_fp64_records(const Params& p, cudaStream_t s, int num_sms);
 // Whether warp-specialised variant v stages its tiles with TMA (needs TensorMaps).
 bool ws_variant_uses_tma(int variant);
 // Neighbour search (counts only, SPJ lists ignored) with the warp-specialised kernel.

@@ -292,11 +292,53 @@ __device__ __forceinline__ void co_k_f32(float r, float r_in, float norm, float 
     }
 }
 
+// FP64 records in the forms of EpjF32 and SpjF32 (split on the integer pipe).
+__device__ __forceinline__ void load_epj_mix(const EpjMix* e, float4& r0, float4& r1) {
+    const uint4 a = __ldg(reinterpret_cast<const uint4*>(e)), b = __ldg(reinterpret_cast<const uint4*>(e) + 1);
+    split_f64(a.x, a.y, r0.x, r1.x);
+    split_f64(a.z, a.w, r0.y, r1.y);
+    split_f64(b.x, b.y, r0.z, r1.z);
+    r0.w = __uint_as_float(b.z);
+    r1.w = __uint_as_float(b.w);
+}
+
+__device__ __forceinline__ void load_spj_mix(const SpjMix* e, float4 (&r)[4]) {
+    const uint4* src = reinterpret_cast<const uint4*>(e);
+    const uint4 a = __ldg(src), b = __ldg(src + 1);
+    const float4 c = __ldg(reinterpret_cast<const float4*>(src + 2)), d = __ldg(reinterpret_cast<const float4*>(src + 3));
+    split_f64(a.x, a.y, r[0].x, r[1].x);
+    split_f64(a.z, a.w, r[0].y, r[1].y);
+    split_f64(b.x, b.y, r[0].z, r[1].z);
+    r[0].w = __uint_as_float(b.z);
+    r[1].w = d.z;  // tr
+    r[2] = c;
+    r[3] = d;
+}
+
+// An EpiRel row from the FP64 one: x - c from both (hi, lo) pairs.
+__device__ __forceinline__ void load_epi_mix(const EpiDev* e, const WalkDesc& wd, float eps2, float4& hi, float4& lo) {
+    const uint4 a = __ldg(reinterpret_cast<const uint4*>(e)), b = __ldg(reinterpret_cast<const uint4*>(e) + 1);
+    float xh, xl, s, t;
+    split_f64(a.x, a.y, xh, xl);
+    two_sum(xh, -wd.ch[0], s, t);
+    two_sum(s, t + (xl - wd.cl[0]), hi.x, lo.x);
+    split_f64(a.z, a.w, xh, xl);
+    two_sum(xh, -wd.ch[1], s, t);
+    two_sum(s, t + (xl - wd.cl[1]), hi.y, lo.y);
+    split_f64(b.x, b.y, xh, xl);
+    two_sum(xh, -wd.ch[2], s, t);
+    two_sum(s, t + (xl - wd.cl[2]), hi.z, lo.z);
+    split_f64(b.z, b.w, xh, xl);
+    const float p = xh * xh;
+    hi.w = p + fmaf(2.f * xh, xl, fmaf(xh, xh, -p));
+    lo.w = __int_as_float(kband_near(fmaxf(fabsf(hi.x), fmaxf(fabsf(hi.y), fabsf(hi.z))), hi.w, eps2));
+}
+
 // ---------------------------------------------------------------- producer
 
 // SR (neighbour search): EPJ tiles only, near entries only; far entries can
 // hold no neighbour and SPJ lists are skipped.
-template <int CW, int KI, bool PK, int MD, int TE, int NS, bool TM>
+template <int CW, int KI, bool PK, int MD, int TE, int NS, bool TM, bool MX>
 __device__ void producer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, int lane, const CUtensorMap& tme,
                          const CUtensorMap& tms) {
     constexpr bool SR = MD == kModeSearch, CO = MD == kModeChangeover;
@@ -445,9 +487,13 @@ __device__ void producer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
 #pragma unroll
                     for (int qq = 0; qq < QB; ++qq) {
                         if (id[qq] >= 0) {
-                            const float4* src = reinterpret_cast<const float4*>(p.epj32 + id[qq]);
-                            r0[qq] = __ldg(src);
-                            r1[qq] = __ldg(src + 1);
+                            if constexpr (MX) {
+                                load_epj_mix(p.epj + id[qq], r0[qq], r1[qq]);
+                            } else {
+                                const float4* src = reinterpret_cast<const float4*>(p.epj32 + id[qq]);
+                                r0[qq] = __ldg(src);
+                                r1[qq] = __ldg(src + 1);
+                            }
                         } else {
                             r0[qq] = r1[qq] = make_float4(0.f, 0.f, 0.f, 0.f);
                         }
@@ -562,9 +608,13 @@ __device__ void producer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
 #pragma unroll
                     for (int qq = 0; qq < QSB; ++qq) {
                         if (id[qq] >= 0) {
-                            const float4* src = reinterpret_cast<const float4*>(p.spj32 + id[qq]);
+                            if constexpr (MX) {
+                                load_spj_mix(p.spj + id[qq], r[qq]);
+                            } else {
+                                const float4* src = reinterpret_cast<const float4*>(p.spj32 + id[qq]);
 #pragma unroll
-                            for (int u = 0; u < 4; ++u) r[qq][u] = __ldg(src + u);
+                                for (int u = 0; u < 4; ++u) r[qq][u] = __ldg(src + u);
+                            }
                         }
                     }
                 }
@@ -648,7 +698,7 @@ __device__ __forceinline__ float pass_cost(int nip, int ku, int ct_threads) {
 // coordinates and the pair accumulators.  The near-only data of each i (lo
 // coordinates, r_search^2, guard band) and the neighbour counts live in
 // shared memory and are read once per tile that has near entries.
-template <int CW, int KI, bool PK, int MD, int TE, int NS, bool TM>
+template <int CW, int KI, bool PK, int MD, int TE, int NS, bool TM, bool MX>
 __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, int ct) {
     constexpr bool SR = MD == kModeSearch, CO = MD == kModeChangeover;
     constexpr int kSlots = NS;
@@ -675,7 +725,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
     // pairs add the same term to both, in a[k][3]).
     float dt[CO ? KI : 1], ds[CO ? KI : 1];
     double rcut2d = 0.0;
-    bool add_self = true, parts = false;
+    bool add_self = true, parts = false, further = false;  // further: a part >= 1
     int since = 0;
 #pragma unroll
     for (int k = 0; k < (CO ? KI : 1); ++k) dt[k] = ds[k] = 0.f;
@@ -1036,6 +1086,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
             gbase = wd.i_begin + h.ipass + slot;
             ibase = wd.i_root + h.ipass + slot;
             parts = wd.n_parts > 1;
+            further = wd.part != 0;
             if constexpr (!SR) add_far = spj_list(p, wd).add_far;
             if constexpr (CO) {
                 rcut2d = wd.rcut2;
@@ -1047,9 +1098,13 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
                 float4 hi = make_float4(0.f, 0.f, 0.f, 0.f), lo = hi;
                 int kb = 0;
                 if (valid) {
-                    const float4* e = reinterpret_cast<const float4*>(p.epi_rel + ibase + k * S);
-                    hi = __ldg(e);
-                    lo = __ldg(e + 1);
+                    if constexpr (MX) {
+                        load_epi_mix(p.epi + ibase + k * S, wd, eps2, hi, lo);
+                    } else {
+                        const float4* e = reinterpret_cast<const float4*>(p.epi_rel + ibase + k * S);
+                        hi = __ldg(e);
+                        lo = __ldg(e + 1);
+                    }
                     kb = __float_as_int(lo.w);
                     lo.w = hi.w;  // r_search^2
                 }
@@ -1100,6 +1155,8 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
             consumers_sync(CT);
             if (active && js == 0) {
                 const double G = p.G;
+                Accp* const out = further && p.part_accp ? p.part_accp : p.out_accp;
+                int32_t* const out_n = further && p.part_nnb ? p.part_nnb : p.out_nnb;
 #pragma unroll
                 for (int k = 0; k < KI; ++k) {
                     if (!(k < ku && slot + k * S < nip)) continue;
@@ -1107,7 +1164,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
                     float2 r[4], rt = make_float2(0.f, 0.f), rs = rt;
                     const int gi = gbase + k * S;
                     if (!SR && add_far) {
-                        load_pairs(p.out_accp + gi, r);  // the far-field pass's sums
+                        load_pairs(out + gi, r);  // the far-field pass's sums
                     } else {
                         r[0] = r[1] = r[2] = r[3] = rt;
                     }
@@ -1141,12 +1198,12 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
                     }
                     if constexpr (!SR) {
                         if (parts)
-                            store_pairs(p.out_accp + gi, r);
+                            store_pairs(out + gi, r);
                         else
-                            p.out_accp[gi] = Accp{G * pair_value(r[0]), G * pair_value(r[1]), G * pair_value(r[2]),
+                            out[gi] = Accp{G * pair_value(r[0]), G * pair_value(r[1]), G * pair_value(r[2]),
                                                   G * pair_value(r[3])};
                     }
-                    p.out_nnb[gi] = n;
+                    out_n[gi] = n;
                 }
             }
             consumers_sync(CT);
@@ -1156,7 +1213,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
     }
 }
 
-template <int CW, int KI, int MINB, bool PK, int MD, int TE, int NS, bool TM>
+template <int CW, int KI, int MINB, bool PK, int MD, int TE, int NS, bool TM, bool MX>
 __global__ __launch_bounds__((CW + 1) * 32, MINB) void ws_kernel(Params p, const __grid_constant__ CUtensorMap tme,
                                                                  const __grid_constant__ CUtensorMap tms) {
     if (p.input_err && *p.input_err) return;  // the inputs failed their check: run nothing
@@ -1177,30 +1234,37 @@ __global__ __launch_bounds__((CW + 1) * 32, MINB) void ws_kernel(Params p, const
     }
     __syncthreads();
     if (tid >= CW * 32)
-        producer<CW, KI, PK, MD, TE, NS, TM>(p, s, tid - CW * 32, tme, tms);
+        producer<CW, KI, PK, MD, TE, NS, TM, MX>(p, s, tid - CW * 32, tme, tms);
     else
-        consumer<CW, KI, PK, MD, TE, NS, TM>(p, s, tid);
+        consumer<CW, KI, PK, MD, TE, NS, TM, MX>(p, s, tid);
 }
 
-template <int CW, int KI, int MINB, bool PK, int MD = kModeForce, int TE = 128, int NS = 4, bool TM = false>
+template <int CW, int KI, int MINB, bool PK, int MD = kModeForce, int TE = 128, int NS = 4, bool TM = false, bool MX = false>
 cudaError_t launch_ws_t(const Params& p, cudaStream_t st, int num_sms, const TensorMaps* tm = nullptr) {
     if (p.n_walk <= 0) return cudaSuccess;
     cudaError_t e;
-    static int per_sm = 0;
+    // Per device: the attribute and the occupancy belong to its context.
+    constexpr int kMaxDevices = 64;
+    static int per_sm_of[kMaxDevices] = {};
+    int dev = 0;
+    e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    int per_sm = dev < kMaxDevices ? per_sm_of[dev] : 0;
     const size_t smem = sizeof(Smem<CW, KI, PK, TE, NS, MD, TM>);
     static const CUtensorMap none{};
     if (TM && (!tm || !tm->valid)) return cudaErrorInvalidValue;
     if (per_sm == 0) {
-        e = cudaFuncSetAttribute(ws_kernel<CW, KI, MINB, PK, MD, TE, NS, TM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        e = cudaFuncSetAttribute(ws_kernel<CW, KI, MINB, PK, MD, TE, NS, TM, MX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem);
         if (e != cudaSuccess) return e;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ws_kernel<CW, KI, MINB, PK, MD, TE, NS, TM>, (CW + 1) * 32, smem);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ws_kernel<CW, KI, MINB, PK, MD, TE, NS, TM, MX>, (CW + 1) * 32, smem);
         if (e != cudaSuccess) return e;
         if (per_sm < 1) per_sm = 1;
+        if (dev < kMaxDevices) per_sm_of[dev] = per_sm;
     }
     int grid = num_sms * per_sm;
     if (grid > p.n_walk) grid = p.n_walk;
-    ws_kernel<CW, KI, MINB, PK, MD, TE, NS, TM><<<grid, (CW + 1) * 32, smem, st>>>(p, TM ? tm->epj : none,
+    ws_kernel<CW, KI, MINB, PK, MD, TE, NS, TM, MX><<<grid, (CW + 1) * 32, smem, st>>>(p, TM ? tm->epj : none,
                                                                                   TM ? tm->spj : none);
     return cudaGetLastError();
 }
@@ -1267,6 +1331,10 @@ cudaError_t launch_ws(const Params& p, cudaStream_t s, int num_sms, int variant,
         case 7: return launch_ws_t<4, 3, 3, true, kModeForce, 128, 6>(p, s, num_sms);
         default: return cudaErrorInvalidValue;
     }
+}
+
+cudaError_t launch_ws_fp64_records(const Params& p, cudaStream_t s, int num_sms) {
+    return launch_ws_t<4, 3, 3, true, kModeForce, 256, 4, false, true>(p, s, num_sms);
 }
 
 bool ws_variant_uses_tma(int variant) { return variant == 1; }

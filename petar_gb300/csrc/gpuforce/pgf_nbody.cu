@@ -1614,7 +1614,7 @@ cudaError_t enqueue_force(pgf_nbody* h) {
             p.n_walk_dev = a.n_desc;
             e = launch_plan(a, h->stream);
             if (e == cudaSuccess) e = launch_ws(p, h->stream, h->num_sms, h->variant - 1, nullptr);
-            if (e == cudaSuccess) e = launch_combine_plan(a, p.out_accp, p.out_nnb, p.G, h->stream);
+            if (e == cudaSuccess) e = launch_combine_plan(a, p, h->stream);
         } else if (e == cudaSuccess) {
             e = launch_ws(h->p, h->stream, h->num_sms, h->variant - 1, nullptr);
         }

@@ -9,12 +9,17 @@
 //
 // The interaction kernels need some scratch besides their inputs and outputs:
 // per-walk descriptors (centre, box, largest r_search), the work-queue order,
-// the queue cursor and the FP64 re-test records.  Here that scratch is the
-// file-scope array g_noalloc_scratch, sized for PGF_NOALLOC_MAX_WALKS walks
-// (about 2.6 MB); every GPU that loads the library keeps it until the process
+// the queue cursor, and the result rows of the parts that expensive walks are
+// split into.  Here that scratch is the file-scope array g_noalloc_scratch,
+// sized for PGF_NOALLOC_MAX_WALKS walks (about 15 MB); every GPU that loads the library keeps it until the process
 // exits.  Host code cannot use the array's name as a device address: the first
 // call on each device looks the address up with cudaGetSymbolAddress while
 // that device is current, and later calls reuse it.
+//
+// The pair kernel is the default warp-specialised one, reading the caller's
+// FP64 records (split into FP32 pairs on the integer pipe), with its walks
+// split on the device (pgf_plan.cu).  Measured on GB300, 33,333 stars: one
+// call 1.35 -> 0.46 ms (before: the CTA-synchronous kernel, walks whole).
 #include "petar_gpuforce.h"
 #include "pgf_internal.cuh"
 
@@ -27,14 +32,21 @@ namespace {
 using namespace pgf;
 
 constexpr int kMaxWalks = PGF_NOALLOC_MAX_WALKS;
-constexpr int kRetestCap = 1 << 16;
+// Parts of split walks: at most 16 per SM beyond one per walk, and their
+// result rows (33,333 stars want 150,000 in quarters of an SM's share).
+constexpr int kMaxParts = 2560;
+constexpr int kMaxDescs = kMaxWalks + kMaxParts;
+constexpr int kPartRows = 1 << 18;
 constexpr int kMaxDevices = 64;
 constexpr size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
-constexpr size_t kFlagsOff = 0;  // [2] error bits, [4..6] launch counters
+constexpr size_t kFlagsOff = 0;  // [0], [1] descriptors and split walks of the plan, [2] input error bits, [3] the kernels' error word, [4..6] launch counters
 constexpr size_t kDescOff = 256;
-constexpr size_t kOrderOff = align256(kDescOff + sizeof(WalkDesc) * kMaxWalks);
-constexpr size_t kRetestOff = align256(kOrderOff + sizeof(int32_t) * kMaxWalks);
-constexpr size_t kScratchBytes = kRetestOff + sizeof(Retest) * kRetestCap;
+constexpr size_t kPlanOff = align256(kDescOff + sizeof(WalkDesc) * kMaxWalks);
+constexpr size_t kOrderOff = align256(kPlanOff + sizeof(WalkDesc) * kMaxDescs);
+constexpr size_t kSplitOff = align256(kOrderOff + sizeof(int32_t) * kMaxDescs);
+constexpr size_t kRowsOff = align256(kSplitOff + sizeof(SplitRec) * kMaxParts);
+constexpr size_t kRowNnbOff = align256(kRowsOff + sizeof(Accp) * kPartRows);
+constexpr size_t kScratchBytes = kRowNnbOff + sizeof(int32_t) * kPartRows;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -68,7 +80,7 @@ __global__ __launch_bounds__(128) void walk_prep_kernel(int n_walk, const int64_
                                                         int64_t n_epi, int64_t n_epj, int64_t n_spj,
                                                         const int32_t* id_epj, int64_t n_id_epj,
                                                         const int32_t* id_spj, int64_t n_id_spj, double rcut2,
-                                                        WalkDesc* desc, int32_t* order, int32_t* err) {
+                                                        WalkDesc* desc, int32_t* err) {
     __shared__ double red[7][128];
     __shared__ int bad;
     const int w = blockIdx.x;
@@ -144,7 +156,6 @@ __global__ __launch_bounds__(128) void walk_prep_kernel(int n_walk, const int64_
         d.rcut2 = rcut2;
         set_walk_f32(d, false);
         desc[w] = d;
-        order[w] = w;
     }
 }
 
@@ -205,21 +216,25 @@ extern "C" int pgf_force_device_noalloc(int n_walk, const int64_t* walk_table, c
     unsigned char* base = g_scratch_addr[dev];
     int32_t* flags = reinterpret_cast<int32_t*>(base + kFlagsOff);
     WalkDesc* desc = reinterpret_cast<WalkDesc*>(base + kDescOff);
-    int32_t* order = reinterpret_cast<int32_t*>(base + kOrderOff);
-    Retest* retest = reinterpret_cast<Retest*>(base + kRetestOff);
 
     e = cudaMemsetAsync(flags, 0, 3 * sizeof(int32_t), s);
     if (e != cudaSuccess) return fail(errbuf, errbuf_len, PGF_ERR_CUDA, "pgf_force_device_noalloc: %s", cudaGetErrorString(e));
     walk_prep_kernel<<<n_walk, 128, 0, s>>>(n_walk, walk_table, epi, n_epi_total, n_epj_total, n_spj_total, id_epj,
-                                            n_id_epj, id_spj, n_id_spj, rcut2, desc, order, flags + 2);
+                                            n_id_epj, id_spj, n_id_spj, rcut2, desc, flags + 2);
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail(errbuf, errbuf_len, PGF_ERR_CUDA, "pgf_force_device_noalloc: prep: %s", cudaGetErrorString(e));
     // The interaction kernels trust the lists, so the validation result is
     // read back (into this stack variable) before they are launched.
-    int32_t err_bits = 0;
-    e = cudaMemcpyAsync(&err_bits, flags + 2, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
+    int32_t err[2] = {0, 0};
+    e = cudaMemcpyAsync(err, flags + 2, sizeof(err), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(errbuf, errbuf_len, PGF_ERR_CUDA, "pgf_force_device_noalloc: %s", cudaGetErrorString(e));
+    const int32_t err_bits = err[0];
+    if (err[1]) {
+        (void)cudaMemsetAsync(flags + 3, 0, sizeof(int32_t), s);
+        return fail(errbuf, errbuf_len, PGF_ERR_DEVICE,
+                    "pgf_force_device_noalloc: a wait in an earlier call's kernels ran out (its results are not complete)");
+    }
     if (err_bits)
         return fail(errbuf, errbuf_len, PGF_ERR_ARG, "pgf_force_device_noalloc: %s%s%s", (err_bits & kBadWalk) ? "walk table row out of range; " : "",
                     (err_bits & kBadEpjId) ? "EPJ id out of range; " : "", (err_bits & kBadSpjId) ? "SPJ id out of range" : "");
@@ -233,20 +248,36 @@ extern "C" int pgf_force_device_noalloc(int n_walk, const int64_t* walk_table, c
     p.spj_q64 = nullptr;
     p.id_epj = id_epj;
     p.id_spj = id_spj;
-    p.walks = desc;
-    p.order = order;
-    p.n_walk = n_walk;
+    PlanArgs a{};
+    a.roots = desc;
+    a.n_root = n_walk;
+    a.num_sms = g_num_sms[dev];
+    a.walks = reinterpret_cast<WalkDesc*>(base + kPlanOff);
+    a.order = reinterpret_cast<int32_t*>(base + kOrderOff);
+    a.splits = reinterpret_cast<SplitRec*>(base + kSplitOff);
+    a.n_desc = flags;
+    a.n_split = flags + 1;
+    a.cap_desc = kMaxDescs;
+    a.cap_splits = kMaxParts;
+    a.row0 = 0;
+    a.cap_rows = kPartRows;
+    p.walks = a.walks;
+    p.order = a.order;
+    p.n_walk = p.n_root = kMaxDescs;
+    p.n_walk_dev = a.n_desc;
+    p.part_align = kPartAlign;
+    p.part_accp = reinterpret_cast<Accp*>(base + kRowsOff);
+    p.part_nnb = reinterpret_cast<int32_t*>(base + kRowNnbOff);
     p.eps2 = eps2;
     p.G = G;
     p.out_accp = reinterpret_cast<Accp*>(accp);
     p.out_nnb = n_ngb;
     bind_counters(p, flags + 4);
-    p.retest = retest;
-    p.retest_cap = kRetestCap;
-    p.err = flags + 2;
+    p.err = flags + 3;
     e = reset_counters(p, s);
-    if (e == cudaSuccess) e = launch_mixed(p, s, g_num_sms[dev]);
-    if (e == cudaSuccess) e = launch_retest(p, s, g_num_sms[dev]);
+    if (e == cudaSuccess) e = launch_plan(a, s);
+    if (e == cudaSuccess) e = launch_ws_fp64_records(p, s, g_num_sms[dev]);
+    if (e == cudaSuccess) e = launch_combine_plan(a, p, s);
     if (e != cudaSuccess) return fail(errbuf, errbuf_len, PGF_ERR_CUDA, "pgf_force_device_noalloc: launch: %s", cudaGetErrorString(e));
     return PGF_OK;
 }

@@ -4,7 +4,7 @@
 //
 // Few walks leave the GPU waiting for the most expensive one.  One CTA reads
 // the walks, gives each that costs more than a sixteenth of one SM's even
-// share up to 32 parts, and writes the descriptors, the work-queue order and
+// share (more where the result rows would not fit) up to 32 parts, and writes the descriptors, the work-queue order and
 // the records of what to add up.  Parts are cut at multiples of 256 list
 // entries, the pair kernel's tile: with partial sums flushed at every tile's
 // end (Params::flush_tiles) a split walk adds the same FP32 terms as a whole
@@ -75,40 +75,47 @@ __global__ __launch_bounds__(kPlanThreads) void plan_kernel(PlanArgs a) {
         s.total = v;
     }
     __syncthreads();
-    const unsigned long long target = s.total / (16ull * (unsigned long long)a.num_sms) + 1;
-    // Further parts and their result rows, scanned over the walks.
+    // Further parts and their result rows, scanned over the walks.  A plan
+    // that does not fit its arrays is tried again with larger parts, down to
+    // half an SM's share; then no walk is split.
+    unsigned long long target = 0;
     long long parts = 0, rows = 0;
-    for (int k = b; k < e; ++k) {
-        const WalkDesc d = a.roots[k];
-        const int p = walk_parts(d, walk_cost(a, k, d), target) - 1;
-        parts += p;
-        rows += (long long)p * d.n_i;
-    }
-    longlong2 v = make_longlong2(parts, rows);
+    longlong2 v = make_longlong2(0, 0);
+    bool fits = false;
+    for (int div = 16; div >= 2 && !fits; div >>= 1) {
+        target = s.total / ((unsigned long long)div * (unsigned long long)a.num_sms) + 1;
+        parts = rows = 0;
+        for (int k = b; k < e; ++k) {
+            const WalkDesc d = a.roots[k];
+            const int p = walk_parts(d, walk_cost(a, k, d), target) - 1;
+            parts += p;
+            rows += (long long)p * d.n_i;
+        }
+        v = make_longlong2(parts, rows);
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const long long px = __shfl_up_sync(0xffffffffu, v.x, o), py = __shfl_up_sync(0xffffffffu, v.y, o);
-        if (lane >= o) {
-            v.x += px;
-            v.y += py;
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long px = __shfl_up_sync(0xffffffffu, v.x, o), py = __shfl_up_sync(0xffffffffu, v.y, o);
+            if (lane >= o) {
+                v.x += px;
+                v.y += py;
+            }
         }
-    }
-    if (lane == 31) s.warp_scan[warp] = v;
-    __syncthreads();
-    if (t == 0) {
-        longlong2 run = make_longlong2(0, 0);
-        for (int k = 0; k < kPlanThreads / 32; ++k) {
-            const longlong2 x = s.warp_scan[k];
-            s.warp_scan[k] = run;
-            run.x += x.x;
-            run.y += x.y;
+        __syncthreads();
+        if (lane == 31) s.warp_scan[warp] = v;
+        __syncthreads();
+        if (t == 0) {
+            longlong2 run = make_longlong2(0, 0);
+            for (int k = 0; k < kPlanThreads / 32; ++k) {
+                const longlong2 x = s.warp_scan[k];
+                s.warp_scan[k] = run;
+                run.x += x.x;
+                run.y += x.y;
+            }
+            s.all = run;
         }
-        s.all = run;
+        __syncthreads();
+        fits = n_root + s.all.x <= a.cap_desc && s.all.x <= a.cap_splits && s.all.y <= a.cap_rows;
     }
-    __syncthreads();
-    const longlong2 all = s.all;
-    // All or nothing: a plan that does not fit its arrays splits no walk.
-    const bool fits = n_root + all.x <= a.cap_desc && all.x <= a.cap_splits && all.y <= a.cap_rows;
     const int desc = (int)(n_root + s.warp_scan[warp].x + v.x - parts);
     int row = (int)(s.warp_scan[warp].y + v.y - rows);  // used only when the plan fits
     for (int pass = 0; pass < 2; ++pass) {
@@ -172,7 +179,8 @@ __global__ __launch_bounds__(kPlanThreads) void plan_kernel(PlanArgs a) {
 // Adds up the parts of every split walk of a device plan: as
 // combine_parts_kernel, the number of records read on the device.
 __global__ __launch_bounds__(128) void combine_plan_kernel(const SplitRec* __restrict__ recs, const int32_t* n_split,
-                                                           Accp* accp, int32_t* nnb, double G) {
+                                                           Accp* accp, int32_t* nnb, const Accp* part_accp,
+                                                           const int32_t* part_nnb, double G) {
     const int n = *n_split;
     for (int q = blockIdx.x; q < n; q += gridDim.x) {
         const SplitRec r = recs[q];
@@ -185,10 +193,10 @@ __global__ __launch_bounds__(128) void combine_plan_kernel(const SplitRec* __res
             for (int k = 1; k < r.n_parts; ++k) {
                 const int64_t row = (int64_t)r.rows1 + (int64_t)(k - 1) * r.n_i + i;
                 float2 b[4];
-                load_pairs(accp + row, b);
+                load_pairs(part_accp + row, b);
 #pragma unroll
                 for (int u = 0; u < 4; ++u) a[u] = add_pair(a[u], b[u]);
-                c += nnb[row];
+                c += part_nnb[row];
             }
             accp[r0] = Accp{G * pair_value(a[0]), G * pair_value(a[1]), G * pair_value(a[2]), G * pair_value(a[3])};
             nnb[r0] = c;
@@ -205,8 +213,10 @@ cudaError_t launch_plan(const PlanArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_combine_plan(const PlanArgs& a, Accp* accp, int32_t* nnb, double G, cudaStream_t s) {
-    combine_plan_kernel<<<a.num_sms * 4, 128, 0, s>>>(a.splits, a.n_split, accp, nnb, G);
+cudaError_t launch_combine_plan(const PlanArgs& a, const Params& p, cudaStream_t s) {
+    combine_plan_kernel<<<a.num_sms * 4, 128, 0, s>>>(a.splits, a.n_split, p.out_accp, p.out_nnb,
+                                                      p.part_accp ? p.part_accp : p.out_accp,
+                                                      p.part_nnb ? p.part_nnb : p.out_nnb, p.G);
     return cudaGetLastError();
 }
 
