@@ -1148,6 +1148,7 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
     if (far) {
         p.id_spj_near = t.id_spj_near.d;
         p.spj_near = t.spj_near.d;
+        p.far_wide = ni <= kFarWideRows ? 1 : 0;
     }
     p.walks = t.walks.d;
     p.order = t.order.d;

@@ -327,7 +327,7 @@ struct Params {
     // Walks without their further parts: when some are split (n_root <
     // n_walk) the roots are descriptors 0 .. n_root - 1 by descending cost.
     int32_t n_root;
-    int32_t pad1;
+    int32_t far_wide;  // far-field pass with eight warps per walk (kFarWideRows)
     // Result of the device-side check of a host-direct dispatch's ids, or
     // null: when it is non-zero the force kernels run nothing.
     const int32_t* input_err;
@@ -506,6 +506,7 @@ inline cudaError_t reset_counters(const Params& p, cudaStream_t s) {
 // its launch costs more than the pairs it saves.  It expands unsoftened
 // gravity only.
 constexpr int64_t kFarMinRows = 8192;
+constexpr int64_t kFarWideRows = 40000;
 inline bool far_applies(double eps2, int64_t n_i) { return eps2 == 0.0 && n_i >= kFarMinRows; }
 
 // Tile of the default pair kernel: the parts of a device plan start at

@@ -19,9 +19,9 @@
 // of the force on Plummer and King models, against 7e-8).  The leading terms
 // (potential and uniform force) are summed as (hi, lo) FP32 pairs.
 //
-// One CTA of four warps per walk, from the same queue order as the
-// interaction kernel (a split walk is handled whole; its parts share the
-// compacted list).  Each warp takes a quarter of the list by itself: the near
+// One CTA per walk, from the same queue order as the interaction kernel (a
+// split walk is handled whole; its parts share the compacted list).  Each of
+// its four or eight warps takes a quarter of the list, or half of one, by itself: the near
 // ids are appended to the compacted list that the interaction kernel reads
 // instead, the far sources go to a ring in shared memory, and whenever 32 are
 // there every lane expands one into 81 coefficients in its registers.  The
@@ -42,22 +42,24 @@
 namespace pgf {
 namespace {
 
-constexpr int kWarps = 4;      // quarters of a list (SpjNear)
-constexpr int kT = kWarps * 32;
 constexpr int kRing = 64;      // per warp: 32 sources arrive while fewer than 32 wait
 constexpr int kMinI = 32;      // fewer i: direct pairs (33 n_i operations) cost about as much
 constexpr float kRhoMax = 0.14f;
 constexpr float kQuadTol = 2e-6f / 84.f;
 constexpr int kPad = 96;  // coefficients padded to 3 per lane
 
+constexpr int kStage = 2048;  // list entries of half a quarter
+
+template <int W>
 struct FarSmem {
-    float src[kWarps][9][kRing];  // x, y, z, m, and the five quadrupole moments (QuadOp), scaled
-    float red[kWarps][kPad];
-    float2 lead[kWarps][4];  // rows 0 and 1 as (hi, lo)
+    float src[W][9][kRing];  // x, y, z, m, and the five quadrupole moments (QuadOp), scaled
+    float red[W][kPad];
+    float2 lead[W][4];  // rows 0 and 1 as (hi, lo)
     float L[kFarCoefs + 3];
     float4 ev[kFarCoefs + 3];  // phi and gradient coefficients
-    float rmax[kWarps];
-    int n_near[kWarps], n_far[kWarps];
+    float rmax[W];
+    int n_near[W], n_far[W];
+    int32_t stage[W == 8 ? 4 : 1][W == 8 ? kStage : 1];  // near ids of a quarter's second half
     int w;
 };
 
@@ -122,9 +124,12 @@ __device__ __forceinline__ void halve(float (&v)[kPad], int lane, int bit) {
     }
 }
 
-__global__ __launch_bounds__(kT, 3) void far_kernel(Params p) {
+template <int W>
+__global__ __launch_bounds__(W * 32, W == 4 ? 3 : 1) void far_kernel(Params p) {
+    constexpr int kT = W * 32;
+    static_assert(W == 4 || W == 8, "a quarter of the list, or half of one, per warp");
     if (p.input_err && *p.input_err) return;  // the inputs failed their check: run nothing
-    __shared__ FarSmem s;
+    __shared__ FarSmem<W> s;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const unsigned lane_lt = (1u << lane) - 1u;
     const int n_walk = p.n_root < p.n_walk ? p.n_root : walk_count(p);
@@ -137,7 +142,7 @@ __global__ __launch_bounds__(kT, 3) void far_kernel(Params p) {
         const WalkDesc wd = p.walks[w];
         const int n_spj = wd.n_spj_all;
         if (wd.n_i < kMinI || n_spj == 0) {
-            if (t == 0) p.spj_near[w] = SpjNear{{-1, 0, 0, 0}, 0, {0, 0, 0}};
+            if (t == 0) p.spj_near[w].n[0] = -1;
             continue;
         }
         // Radius of the walk's particles.
@@ -150,10 +155,11 @@ __global__ __launch_bounds__(kT, 3) void far_kernel(Params p) {
         for (int o = 16; o > 0; o >>= 1) r2m = fmaxf(r2m, __shfl_xor_sync(0xffffffffu, r2m, o));
         if (lane == 0) s.rmax[warp] = r2m;
         __syncthreads();
-        r2m = fmaxf(fmaxf(s.rmax[0], s.rmax[1]), fmaxf(s.rmax[2], s.rmax[3]));
+#pragma unroll
+        for (int k = 0; k < W; ++k) r2m = fmaxf(r2m, s.rmax[k]);
         const float R = sqrtf(r2m) * 1.00001f;
         if (!(R > 1e-18f && R < 1e18f)) {
-            if (t == 0) p.spj_near[w] = SpjNear{{-1, 0, 0, 0}, 0, {0, 0, 0}};
+            if (t == 0) p.spj_near[w].n[0] = -1;
             continue;
         }
         // Lengths in units of a power of two at the nearest distance expanded,
@@ -170,13 +176,23 @@ __global__ __launch_bounds__(kT, 3) void far_kernel(Params p) {
         float L[kFarCoefs], lo[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int k = 0; k < kFarCoefs; ++k) L[k] = 0.f;
-        // Each warp takes a quarter of the list by itself: 32 entries at a
-        // time, with the records loaded one chunk ahead and the ids two.
-        const int b0 = (int)((int64_t)n_spj * warp / kWarps), n_w = (int)((int64_t)n_spj * (warp + 1) / kWarps) - b0;
-        const int32_t* __restrict__ ids = p.id_spj + wd.spj_begin + b0;
-        int32_t* __restrict__ near_out = p.id_spj_near + wd.spj_begin + b0;
+        // Each warp takes its quarter of the list, or half of it, by itself: 32
+        // entries at a time, with the records loaded one chunk ahead and the
+        // ids two.  The near ids of a second half wait in shared memory for
+        // the number of those before them; quarters too long for that are
+        // left to the first warp.
+        const int quarter = W == 8 ? warp >> 1 : warp, half = W == 8 ? warp & 1 : 0;
+        int b0 = (int)((int64_t)n_spj * quarter / 4), n_w = (int)((int64_t)n_spj * (quarter + 1) / 4) - b0;
+        int32_t* const quarter_out = p.id_spj_near + wd.spj_begin + b0;
+        if (W == 8) {
+            const int first = n_w <= 2 * kStage ? (n_w + 1) >> 1 : n_w;
+            if (half) b0 += first;
+            n_w = half ? n_w - first : first;
+        }
+        int32_t* __restrict__ const near_out = half ? s.stage[W == 8 ? quarter : 0] : quarter_out;
         float (*const src)[kRing] = s.src[warp];
         int head = 0, waiting = 0, n_near = 0, n_far = 0;
+        const int32_t* __restrict__ ids = p.id_spj + wd.spj_begin + b0;
         int id = lane < n_w ? __ldg(ids + lane) : -1;
         int id_next = 32 + lane < n_w ? __ldg(ids + 32 + lane) : -1;
         SpjRec rec = load_spj(p.spj32, id);
@@ -249,9 +265,20 @@ __global__ __launch_bounds__(kT, 3) void far_kernel(Params p) {
             s.n_far[warp] = n_far;
         }
         __syncthreads();
-        n_far = (s.n_far[0] + s.n_far[1]) + (s.n_far[2] + s.n_far[3]);
-        if (t == 0)
-            p.spj_near[w] = SpjNear{{s.n_near[0], s.n_near[1], s.n_near[2], s.n_near[3]}, n_far > 0 ? 1 : 0, {0, 0, 0}};
+        n_far = 0;
+#pragma unroll
+        for (int k = 0; k < W; ++k) n_far += s.n_far[k];
+        if (half) {
+            const int before = s.n_near[warp - 1], n = s.n_near[warp];
+            for (int k = lane; k < n; k += 32) quarter_out[before + k] = near_out[k];
+        }
+        if (t == 0) {
+            SpjNear r{};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) r.n[q] = W == 8 ? s.n_near[(2 * q) % W] + s.n_near[(2 * q + 1) % W] : s.n_near[q];
+            r.add_far = n_far > 0 ? 1 : 0;
+            p.spj_near[w] = r;
+        }
         if (n_far == 0) continue;
 
         // Sum over the threads: rows 0 and 1 in FP64, the others by a
@@ -279,7 +306,12 @@ __global__ __launch_bounds__(kT, 3) void far_kernel(Params p) {
             for (int k = 0; k < 3; ++k) s.red[warp][b + k] = v[k];
         }
         __syncthreads();
-        if (t < kFarCoefs) s.L[t] = (s.red[0][t] + s.red[1][t]) + (s.red[2][t] + s.red[3][t]);
+        if (t < kFarCoefs) {
+            float v = 0.f;
+#pragma unroll
+            for (int k = 0; k < W; k += 2) v += s.red[k][t] + s.red[k + 1][t];
+            s.L[t] = v;
+        }
         __syncthreads();
         if (t < kFarCoefs) {
             int n = 0;
@@ -291,7 +323,11 @@ __global__ __launch_bounds__(kT, 3) void far_kernel(Params p) {
         float2 lead[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            lead[k] = add_pair(add_pair(s.lead[0][k], s.lead[1][k]), add_pair(s.lead[2][k], s.lead[3][k]));
+        {
+            lead[k] = s.lead[0][k];
+#pragma unroll
+            for (int q = 1; q < W; ++q) lead[k] = add_pair(lead[k], s.lead[q][k]);
+        }
         __syncthreads();
         const float inv2 = inv * inv;  // powers of two: scaling the results is exact
 #pragma unroll 1
@@ -336,18 +372,31 @@ cudaError_t launch_epi_rel(const Params& p, EpiRel* out, AccF32* out_acc, cudaSt
     return cudaGetLastError();
 }
 
-cudaError_t launch_far(const Params& p, cudaStream_t s, int num_sms) {
-    if (!p.spj_near || p.n_walk <= 0) return cudaSuccess;
+namespace {
+
+template <int W>
+cudaError_t launch_far_t(const Params& p, cudaStream_t s, int num_sms) {
     static int per_sm = 0;
     if (per_sm == 0) {
-        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, far_kernel, kT, 0);
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, far_kernel<W>, W * 32, 0);
         if (e != cudaSuccess) return e;
         if (per_sm < 1) per_sm = 1;
     }
     int grid = num_sms * per_sm;
     if (grid > p.n_walk) grid = p.n_walk;
-    far_kernel<<<grid, kT, 0, s>>>(p);
+    far_kernel<W><<<grid, W * 32, 0, s>>>(p);
     return cudaGetLastError();
+}
+
+}  // namespace
+
+// Eight warps per walk where the walks leave SMs with one or none (200-walk
+// calls on 262,144 binary stars: kernels of a call 433 -> 410 us), else four.  The rule looks
+// at the dispatch's i-particles, not at the launch, so that results do not
+// depend on the pipeline stages.
+cudaError_t launch_far(const Params& p, cudaStream_t s, int num_sms) {
+    if (!p.spj_near || p.n_walk <= 0) return cudaSuccess;
+    return p.far_wide ? launch_far_t<8>(p, s, num_sms) : launch_far_t<4>(p, s, num_sms);
 }
 
 }  // namespace pgf

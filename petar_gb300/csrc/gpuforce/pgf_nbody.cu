@@ -1693,6 +1693,7 @@ void bind_params(pgf_nbody* h) {
     if (far_applies(h->cfg.eps2, h->n)) {
         p.id_spj_near = h->id_spj_near.d;
         p.spj_near = h->spj_near.d;
+        p.far_wide = h->n <= kFarWideRows ? 1 : 0;
     }
     p.err = h->flags.d + 2;
     p.retest = h->retest.d;

@@ -69,6 +69,8 @@ CASES = {
     "empty": dict(n_i=[40, 100], n_spj=[0, 0], near=1.0, far=2.0),
     # more i than one pass and than the coordinates kept in shared memory
     "large": dict(n_i=[511, 512, 513, 1500], n_spj=[700, 701, 702, 703], near=0.5, far=50.0),
+    # lists whose half quarters are longer than the pass keeps in shared memory
+    "long": dict(n_i=[64, 100], n_spj=[16390, 17000], near=0.5, far=50.0),
     # walks away from the origin (x - c cancels), large moments
     "offset": dict(n_i=[64, 200], n_spj=[400, 3000], near=0.5, far=20.0, centre=300.0),
     "moments": dict(n_i=[64, 200], n_spj=[400, 3000], near=0.5, far=20.0, quad=2.0),
