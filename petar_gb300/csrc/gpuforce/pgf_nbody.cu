@@ -38,7 +38,7 @@
 //
 // The walks run as one thread per (group, pair of frontier cells), taken a
 // warp at a time from a counter.  The frontier cells are the topmost cells
-// with at most n / 512 particles (at least n_group_limit) (or
+// with at most n / 512 particles (or 64) (or
 // leaves); they partition the particles in Morton order, so the depth-first
 // list of a group is the concatenation, in frontier order, of the lists of
 // the frontier subtrees (a cell above the frontier that the group does not
@@ -118,7 +118,12 @@ struct __align__(16) TCellW {
     float in_lo[3], in_hi[3];
     float out_lo[3], out_hi[3];
     int32_t begin, end, first_child, n_child;
-    int32_t leaf, parent, level, pad1;
+    int32_t leaf, parent, level;
+    // A group whose largest r_search is below this cannot have boxes that
+    // meet this cell's once the cell is closed by distance: the centre of mass
+    // is then side / theta away, the cell's particles within sqrt(3) side of
+    // it, and boxes that meet within sqrt(3) of the larger r_search.
+    float apart;
 };
 static_assert(sizeof(TCellW) == 96, "TCellW layout");
 
@@ -681,7 +686,10 @@ __global__ __launch_bounds__(256) void moments_kernel(const TreeHdr* h, TCell* c
         w.leaf = cc.leaf;
         w.parent = cc.parent;
         w.level = cc.level;
-        w.pad1 = 0;
+        {
+            const float a = 0.5772f * ((float)sqrt(cc.crit) * 0.9999f - 1.7322f * (float)side);
+            w.apart = a > cc.rs_max ? a : 0.f;
+        }
         cw[c] = w;
         CMom& o = mom[c];
         o.m = m;
@@ -811,6 +819,7 @@ struct WalkCtx {
     int gcell;
     float in_lo[3], in_hi[3], out_lo[3], out_hi[3];
     float X;
+    float rs;  // largest r_search of the group
     bool open_all;
 };
 
@@ -827,6 +836,7 @@ __device__ __forceinline__ void load_ctx(WalkCtx& x, const TCellW* cw, const TCe
         x.out_hi[d] = g.out_hi[d];
     }
     x.X = X;
+    x.rs = cells[gcell].rs_max;
     x.open_all = open_all;
 }
 
@@ -835,6 +845,8 @@ __device__ __forceinline__ bool open_cell(const WalkCtx& x, int c, const TCellW&
     if (x.open_all) return true;
     const int d = dist3(x.in_lo, x.in_hi, w, x.X);
     if (d == 1) return true;
+    // Closed by distance, and too far for the r_search boxes to meet.
+    if (d == 0 && w.apart > x.rs) return false;
     const int o1 = overlap3(x.out_lo, x.out_hi, w.in_lo, w.in_hi);
     if (o1 == 1) return true;
     const int o2 = overlap3(x.in_lo, x.in_hi, w.out_lo, w.out_hi);
@@ -982,6 +994,7 @@ __device__ __forceinline__ int cost_bucket(float cost) {
 }
 
 constexpr int kChunk = 2;  // frontier cells per task
+constexpr int kWalkWarps = 4;  // per CTA
 
 __device__ __forceinline__ int64_t n_chunks(const TreeHdr* h) { return (h->n_fronts + kChunk - 1) / kChunk; }
 
@@ -992,41 +1005,79 @@ __global__ void task_check_kernel(TreeHdr* h, int64_t cap_tasks) {
     if ((int64_t)h->n_groups * n_chunks(h) > cap_tasks) h->err |= kErrTasks;
 }
 
-// The walk passes take tasks a warp at a time from a counter: task costs
-// differ by orders of magnitude (a chunk next to the group against one whose
-// ancestors the group closes), so a static split leaves SMs idle at the end.
-// Lane l of a warp takes task base + l, so a warp walks one chunk for 32
-// neighbouring groups.
-__device__ __forceinline__ int64_t next_tasks(unsigned long long* cursor) {
-    unsigned long long base = 0;
-    if ((threadIdx.x & 31) == 0) base = atomicAdd(cursor, 32ull);
-    return (int64_t)__shfl_sync(0xffffffffu, base, 0);
+// A task is (chunk q of frontier cells, block b of 32 groups), walked by one
+// warp, a lane per group: its threads walk the same subtrees for neighbouring
+// groups.  Warps take tasks from a counter, as their costs differ by orders of
+// magnitude: a chunk next to the groups against one whose ancestors they
+// close.  The tasks of every block run outwards from the chunk that holds its
+// own particles, so the expensive ones come first and the launch ends on
+// cheap ones (King 1M: tree and lists 3.36 -> 2.92 ms with this order and
+// the early exit in open_cell).
+__device__ __forceinline__ int64_t next_task(unsigned long long* cursor) {
+    unsigned long long t = 0;
+    if ((threadIdx.x & 31) == 0) t = atomicAdd(cursor, 1ull);
+    return (int64_t)__shfl_sync(0xffffffffu, t, 0);
 }
 
-// Task t = (chunk q = t / n_groups, group g = t % n_groups) walks frontier
-// cells kChunk q .. kChunk q + kChunk - 1 for group g: the threads of a warp
-// walk the same subtrees for neighbouring groups.  Counts are stored at t.
-__global__ __launch_bounds__(128) void walk_task_count_kernel(TreeHdr* h, const TCellW* __restrict__ cw,
-                                                              const TCell* __restrict__ cells,
-                                                              const int32_t* __restrict__ groups,
-                                                              const int32_t* __restrict__ fronts, int32_t* task_e,
-                                                              int32_t* task_s, bool open_all) {
+// Frontier cell holding particle row i: the last one that begins at or before
+// it, by a 32-way search.
+__device__ __forceinline__ int front_of(const TCellW* __restrict__ cw, const int32_t* __restrict__ fronts, int nf, int i) {
+    int lo = 0, n = nf;  // the answer is in [lo, lo + n)
+    while (n > 1) {
+        const int step = (n + 31) / 32;
+        const int k = lo + (int)(threadIdx.x & 31) * step;
+        const bool le = k < lo + n && cw[fronts[k]].begin <= i;
+        const unsigned m = __ballot_sync(0xffffffffu, le) | 1u;
+        const int j = 31 - __clz(m);
+        n = min(step, n - j * step);
+        lo += j * step;
+    }
+    return lo;
+}
+
+template <bool FILL>
+__device__ __forceinline__ void walk_tasks(TreeHdr* h, const TCellW* __restrict__ cw, const TCell* __restrict__ cells,
+                                           const int32_t* __restrict__ groups, const int32_t* __restrict__ fronts,
+                                           const WalkDesc* __restrict__ walks, int32_t* task_e, int32_t* task_s,
+                                           int32_t* id_epj, int32_t* id_spj, bool open_all) {
     if (h->err) return;
-    const int64_t ng = h->n_groups, nf = h->n_fronts, T = ng * n_chunks(h);
+    const int lane = threadIdx.x & 31;
+    const int64_t ng = h->n_groups, nf = h->n_fronts, nb = (ng + 31) / 32, T = nb * n_chunks(h);
     const float X = h->xmax;
     for (;;) {
-        const int64_t t = next_tasks(&h->walk_cursor[0]) + (threadIdx.x & 31);
-        if (t - (threadIdx.x & 31) >= T) break;
-        if (t >= T) continue;
-        const int q = (int)(t / ng), g = (int)(t - (int64_t)q * ng);
+        const int64_t t = next_task(&h->walk_cursor[FILL ? 1 : 0]);
+        if (t >= T) break;
+        const int64_t nq = n_chunks(h);
+        const int o = (int)(t / nb), b = (int)(t - (int64_t)o * nb);
+        const int g = b * 32 + lane;
+        const bool valid = g < ng;
+        const int mid = groups[min((int)ng - 1, b * 32 + 16)];
+        // own chunk, then 1 after, 1 before, 2 after, ... (wrapping around)
+        const int own = front_of(cw, fronts, (int)nf, cw[mid].begin) / kChunk;
+        int q = (int)((own + ((o & 1) ? (o + 1) / 2 : -(o / 2))) % nq);
+        if (q < 0) q += (int)nq;
         WalkCtx x;
-        load_ctx(x, cw, cells, groups[g], X, open_all);
+        load_ctx(x, cw, cells, groups[valid ? g : (int)ng - 1], X, open_all);
+        const int64_t slot = (int64_t)q * ng + g;
+        if (!valid) continue;
         int ne, ns;
-        walk_chunk<false>(x, fronts, q * kChunk, (int)min(nf, (int64_t)(q + 1) * kChunk), ne, ns, nullptr,
-                          nullptr);
-        task_e[t] = ne;
-        task_s[t] = ns;
+        walk_chunk<FILL>(x, fronts, q * kChunk, (int)min(nf, (int64_t)(q + 1) * kChunk), ne, ns,
+                         FILL ? id_epj + walks[g].epj_begin + task_e[slot] : nullptr,
+                         FILL ? id_spj + walks[g].spj_begin + task_s[slot] : nullptr);
+        if (!FILL) {
+            task_e[slot] = ne;
+            task_s[slot] = ns;
+        }
     }
+}
+
+// Counts of every (chunk, group), stored at q * n_groups + g.
+__global__ __launch_bounds__(kWalkWarps * 32) void walk_task_count_kernel(TreeHdr* h, const TCellW* __restrict__ cw,
+                                                                          const TCell* __restrict__ cells,
+                                                                          const int32_t* __restrict__ groups,
+                                                                          const int32_t* __restrict__ fronts,
+                                                                          int32_t* task_e, int32_t* task_s, bool open_all) {
+    walk_tasks<false>(h, cw, cells, groups, fronts, nullptr, task_e, task_s, nullptr, nullptr, open_all);
 }
 
 // Per group: offsets of its tasks within its lists (in frontier order), the
@@ -1127,29 +1178,14 @@ __global__ __launch_bounds__(kScanThreads) void walk_scan_kernel(TreeHdr* h, Wal
     }
 }
 
-__global__ __launch_bounds__(128) void walk_task_fill_kernel(TreeHdr* h, const TCellW* __restrict__ cw,
-                                                             const TCell* __restrict__ cells,
-                                                             const int32_t* __restrict__ groups,
-                                                             const int32_t* __restrict__ fronts,
-                                                             const WalkDesc* __restrict__ walks,
-                                                             const int32_t* __restrict__ task_e,
-                                                             const int32_t* __restrict__ task_s, int32_t* id_epj,
-                                                             int32_t* id_spj, bool open_all) {
-    if (h->err) return;
-    const int64_t ng = h->n_groups, nf = h->n_fronts, T = ng * n_chunks(h);
-    const float X = h->xmax;
-    for (;;) {
-        const int64_t t = next_tasks(&h->walk_cursor[1]) + (threadIdx.x & 31);
-        if (t - (threadIdx.x & 31) >= T) break;
-        if (t >= T) continue;
-        const int q = (int)(t / ng), g = (int)(t - (int64_t)q * ng);
-        WalkCtx x;
-        load_ctx(x, cw, cells, groups[g], X, open_all);
-        const WalkDesc& d = walks[g];
-        int ne, ns;
-        walk_chunk<true>(x, fronts, q * kChunk, (int)min(nf, (int64_t)(q + 1) * kChunk), ne, ns,
-                         id_epj + d.epj_begin + task_e[t], id_spj + d.spj_begin + task_s[t]);
-    }
+__global__ __launch_bounds__(kWalkWarps * 32) void walk_task_fill_kernel(TreeHdr* h, const TCellW* __restrict__ cw,
+                                                                         const TCell* __restrict__ cells,
+                                                                         const int32_t* __restrict__ groups,
+                                                                         const int32_t* __restrict__ fronts,
+                                                                         const WalkDesc* __restrict__ walks,
+                                                                         int32_t* task_e, int32_t* task_s,
+                                                                         int32_t* id_epj, int32_t* id_spj, bool open_all) {
+    walk_tasks<true>(h, cw, cells, groups, fronts, walks, task_e, task_s, id_epj, id_spj, open_all);
 }
 
 // Work queue: walks by descending cost bucket (ties in no fixed order; the
@@ -1505,6 +1541,11 @@ struct pgf_nbody {
 
 namespace {
 
+// Largest frontier cell: about a thousand frontier cells from 32,768 particles
+// on, cells of 64 below (3,000 stars: tree and lists 0.88 ms with cells of a
+// group's 512, 0.77 ms with 64).
+int front_limit_of(int64_t n) { return (int)std::max<int64_t>(64, n / 512); }
+
 int grid_for(const pgf_nbody* h, int64_t work, int threads) {
     int64_t b = (work + threads - 1) / threads;
     const int64_t lim = (int64_t)h->num_sms * 8;
@@ -1565,13 +1606,13 @@ cudaError_t enqueue_build(pgf_nbody* h) {
     if ((e = cub_select(h, h->cub_tmp.d, bytes, h->front_at.d, h->fronts.d, &hd->n_fronts)) != cudaSuccess) return e;
     task_check_kernel<<<1, 32, 0, s>>>(hd, h->cap_tasks);
     const int gt = h->num_sms * 16;
-    walk_task_count_kernel<<<gt, 128, 0, s>>>(hd, h->cw.d, h->cells.d, h->groups.d, h->fronts.d, h->task_e.d,
+    walk_task_count_kernel<<<gt, kWalkWarps * 32, 0, s>>>(hd, h->cw.d, h->cells.d, h->groups.d, h->fronts.d, h->task_e.d,
                                               h->task_s.d, h->open_all);
     group_reduce_kernel<<<grid_for(h, n, 128), 128, 0, s>>>(hd, h->cells.d, h->groups.d, h->walks.d, h->task_e.d,
                                                             h->task_s.d, h->cnt_e.d, h->cnt_s.d, h->bucket.d,
                                                             h->cfg.r_out * h->cfg.r_out);
     walk_scan_kernel<<<1, kScanThreads, 0, s>>>(hd, h->walks.d, h->cnt_e.d, h->cnt_s.d, h->cap_e, h->cap_s);
-    walk_task_fill_kernel<<<gt, 128, 0, s>>>(hd, h->cw.d, h->cells.d, h->groups.d, h->fronts.d, h->walks.d,
+    walk_task_fill_kernel<<<gt, kWalkWarps * 32, 0, s>>>(hd, h->cw.d, h->cells.d, h->groups.d, h->fronts.d, h->walks.d,
                                              h->task_e.d, h->task_s.d, h->id_epj.d, h->id_spj.d, h->open_all);
     queue_scatter_kernel<<<grid_for(h, n, 256), 256, 0, s>>>(hd, h->bucket.d, h->queue.d);
     return cudaGetLastError();
@@ -1867,7 +1908,7 @@ int pgf_nbody_create(const pgf_nbody_config* cfg, int64_t n, const double* pos, 
     for (auto* a : {&h->group_at, &h->groups, &h->cnt_e, &h->cnt_s, &h->bucket, &h->queue, &h->front_at, &h->fronts,
                     &h->inv_order})
         NB_TRY(a->alloc(n));
-    h->front_limit = (int)std::max<int64_t>(cfg->n_group_limit, n / 512);
+    h->front_limit = front_limit_of(n);
     NB_TRY(alloc_tasks(h, 64 * (n / std::max(1, cfg->n_group_limit / 4) + 1) + 4096));
     NB_TRY(h->walks.alloc(n));
     h->cap_e = 8 * n + 1024;  // first guesses; the first build sizes them
@@ -2136,7 +2177,6 @@ int pgf_nbody_set_group_limit(pgf_nbody* h, int n_group_limit) {
     if (n_group_limit < 1) return nb_fail(PGF_ERR_ARG, "n_group_limit must be >= 1");
     NB_CUDA(cudaStreamSynchronize(h->stream));
     h->cfg.n_group_limit = n_group_limit;
-    h->front_limit = (int)std::max<int64_t>(n_group_limit, h->n / 512);
     drop_graph(h);  // the captured steps build other lists now
     if (int r = build_fit(h)) return r;
     return pgf_nbody_force(h);
