@@ -72,7 +72,7 @@ constexpr int kLeafBins = 64;          // leaf size classes of the moments launc
 constexpr int kCellBins = kLeafBins + 8 * kLevels;  // and inner cells by level and child count
 constexpr int kScanThreads = 1024;
 
-enum : int32_t { kErrCells = 1, kErrEpj = 2, kErrSpj = 4, kErrTasks = 8 };
+enum : int32_t { kErrCells = 1, kErrEpj = 2, kErrSpj = 4, kErrTasks = 8, kErrBarrier = 16 };
 constexpr float kU = 5.9604645e-8f;  // 2^-24, unit roundoff of FP32
 
 struct TreeHdr {
@@ -95,7 +95,7 @@ struct TreeHdr {
     int32_t cell_hist[kCellBins];    // cells by moments class
     int32_t cell_cursor[kCellBins];  // their slots in the class-ordered cell list
     int32_t sample_slot;  // next record slot of the per-step sample
-    int32_t pad2;
+    unsigned bar;  // arrivals at the tree kernel's grid barriers
     unsigned long long walk_cursor[2];  // next task of the count and fill passes
 };
 
@@ -277,6 +277,7 @@ __global__ __launch_bounds__(256) void bbox_final_kernel(const double* __restric
     for (int d = 0; d < 3; ++d) xm = dmax(xm, dmax(fabs(h->root_lo[d]), fabs(h->root_lo[d] + h->side0)));
     h->xmax = __double2float_ru(xm);
     for (int L = 0; L < kLevels + 2; ++L) h->level_begin[L] = L == 0 ? 0 : 1;
+    h->bar = 0;
     h->n_groups = 0;
     h->n_fronts = 0;
     h->n_walk = 0;
@@ -342,39 +343,54 @@ __global__ __launch_bounds__(256) void gather_kernel(const int32_t* __restrict__
 
 // ---------------------------------------------------------------- octree, level by level
 
-// Octant boundaries of a cell at level L: child o holds [b[o], b[o + 1]).
-__device__ __forceinline__ void octants(const uint64_t* __restrict__ skey, int begin, int end, int L, int b[9]) {
-    const int shift = 3 * (kMaxLevel - 1 - L);
-    b[0] = begin;
-    b[8] = end;
-    for (int o = 1; o < 8; ++o) {
-        int lo = b[o - 1], hi = end;  // first index with digit >= o
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if ((int)((skey[mid] >> shift) & 7) < o) lo = mid + 1;
-            else hi = mid;
+// The tree is built by one cooperative launch (tree_kernel below): its levels,
+// the class order of the cells and the moments are phases of a kernel with one
+// CTA per SM, with a grid barrier between them.  As launches of their own
+// (three per level for 22 levels, and one per level of moments) they took
+// most of a small step: tree and lists 0.77 ms at 3,000 stars, 0.34 ms so (King 1M:
+// 2.92 and 2.44 ms).
+constexpr int kTreeThreads = 512;
+constexpr int kTreeWarps = kTreeThreads / 32;
+
+__device__ __forceinline__ unsigned long long tree_timer() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// Grid barrier of a cooperative launch: bar counts arrivals since the build
+// began.  A wait that takes longer than a second sets the build's error and
+// returns false in every CTA that sees it; the kernel then ends.
+__device__ bool grid_sync(unsigned* bar, unsigned& epoch, int32_t* err) {
+    __shared__ int s_ok;
+    __syncthreads();
+    epoch += gridDim.x;
+    if (threadIdx.x == 0) {
+        int ok = 1;
+        __threadfence();
+        atomicAdd(bar, 1u);
+        const unsigned long long t0 = tree_timer();
+        for (;;) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+            if ((int)(v - epoch) >= 0) break;
+            if (tree_timer() - t0 > 1000000000ull) {
+                atomicOr(err, kErrBarrier);
+                ok = 0;
+                break;
+            }
         }
-        b[o] = lo;
+        __threadfence();
+        s_ok = ok;
     }
+    __syncthreads();
+    return s_ok != 0;
 }
 
-// The cells of a level are split into kLevelBlocks contiguous chunks, one
-// per CTA, so that the child numbering (children of a level in their parents'
-// order) is a two-level scan: CTA sums here, their scan by one CTA, and the
-// CTA-local scans when the children are written.
-constexpr int kLevelBlocks = 1024;
-
-__device__ __forceinline__ void level_chunk(const TreeHdr* h, int L, int& c0, int& c1) {
-    const int lb = h->level_begin[L], le = h->level_begin[L + 1];
-    const int per = (le - lb + kLevelBlocks - 1) / kLevelBlocks;
-    c0 = min(le, lb + (int)blockIdx.x * per);
-    c1 = min(le, c0 + per);
-}
-
-// Exclusive scan of one value per thread over a 256-thread CTA; *total gets
-// the sum.  Every thread of the CTA must call it.
-__device__ __forceinline__ int cta256_excl_scan(int v, int* total) {
-    __shared__ int ws[8];
+// Exclusive scan of one value per thread over the CTA; *total gets the sum.
+// Every thread of the CTA must call it.
+__device__ __forceinline__ int cta_excl_scan(int v, int* total) {
+    __shared__ int ws[kTreeWarps];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int x = v;
 #pragma unroll
@@ -386,7 +402,7 @@ __device__ __forceinline__ int cta256_excl_scan(int v, int* total) {
     __syncthreads();
     int base = 0, tot = 0;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
+    for (int k = 0; k < kTreeWarps; ++k) {
         base += k < w ? ws[k] : 0;
         tot += ws[k];
     }
@@ -395,135 +411,27 @@ __device__ __forceinline__ int cta256_excl_scan(int v, int* total) {
     return base + x - v;
 }
 
-__global__ __launch_bounds__(256) void split_kernel(TreeHdr* h, TCell* cells, int32_t* nch, int4* bnd,
-                                                    int32_t* blocksum, const uint64_t* __restrict__ skey, int L,
-                                                    int n_leaf) {
-    if (h->err) return;
-    int c0, c1;
-    level_chunk(h, L, c0, c1);
-    const int lb = h->level_begin[L];
-    int sum = 0;
-    if (c1 - c0 <= (int)(blockDim.x >> 5)) {
-        // Few, large cells (the upper levels): a warp per cell, its seven
-        // binary searches run by seven lanes at once instead of one after
-        // another (each is a chain of dependent key loads).
-        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        if (c0 + w < c1) {
-            const int c = c0 + w;
-            TCell& cc = cells[c];
-            const int cnt = cc.end - cc.begin;
-            const bool leaf = cnt <= n_leaf || L >= kMaxLevel;
-            int bo = cc.end;
-            if (!leaf && lane < 7) {
-                const int shift = 3 * (kMaxLevel - 1 - L);
-                int lo = cc.begin, hi = cc.end;  // first index with digit >= lane + 1
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    if ((int)((skey[mid] >> shift) & 7) < lane + 1) lo = mid + 1;
-                    else hi = mid;
-                }
-                bo = lo;
-            }
-            int b[9];
-            b[0] = cc.begin;
-            b[8] = cc.end;
-#pragma unroll
-            for (int o = 1; o < 8; ++o) b[o] = __shfl_sync(0xffffffffu, bo, o - 1);
-            if (lane == 0) {
-                int k = 0;
-                if (!leaf) {
-                    for (int o = 0; o < 8; ++o) k += b[o + 1] > b[o];
-                    bnd[2 * (c - lb)] = make_int4(b[1], b[2], b[3], b[4]);
-                    bnd[2 * (c - lb) + 1] = make_int4(b[5], b[6], b[7], b[8]);
-                }
-                cc.leaf = leaf;
-                cc.n_child = k;
-                nch[c - lb] = k;
-                sum = k;
-            }
-        }
-    } else {
-        for (int c = c0 + (int)threadIdx.x; c < c1; c += blockDim.x) {
-            TCell& cc = cells[c];
-            const int cnt = cc.end - cc.begin;
-            const bool leaf = cnt <= n_leaf || L >= kMaxLevel;
-            int k = 0;
-            if (!leaf) {
-                int b[9];
-                octants(skey, cc.begin, cc.end, L, b);
-                for (int o = 0; o < 8; ++o) k += b[o + 1] > b[o];
-                // The octant ends, for the fill of this level.
-                bnd[2 * (c - lb)] = make_int4(b[1], b[2], b[3], b[4]);
-                bnd[2 * (c - lb) + 1] = make_int4(b[5], b[6], b[7], b[8]);
-            }
-            cc.leaf = leaf;
-            cc.n_child = k;
-            nch[c - lb] = k;
-            sum += k;
-        }
+// First index in [lo, hi) of the sorted keys whose octant digit is at least
+// `digit`, searched by a whole warp 32 ways at a time.
+__device__ __forceinline__ int warp_octant(const uint64_t* __restrict__ skey, int lo, int hi, int shift, int digit) {
+    const int lane = threadIdx.x & 31;
+    while (lo < hi) {
+        const int64_t len = hi - lo;
+        // probes split [lo, hi) evenly; each lane's is the last of its share
+        const int pos = (int)(lo + (len * (lane + 1) + 31) / 32 - 1);
+        const bool ge = (int)((skey[pos] >> shift) & 7) >= digit;
+        const unsigned m = __ballot_sync(0xffffffffu, ge);
+        if (!m) return hi;
+        const int first = __ffs(m) - 1;
+        const int p = __shfl_sync(0xffffffffu, pos, first);
+        const int before = __shfl_sync(0xffffffffu, pos, first ? first - 1 : 0);
+        if (first) lo = before + 1;
+        if (lo == p) return p;
+        hi = p;
     }
-    int tot;
-    (void)cta256_excl_scan(sum, &tot);
-    if (threadIdx.x == 0) blocksum[blockIdx.x] = tot;
+    return lo;
 }
 
-__global__ __launch_bounds__(kScanThreads) void level_scan_kernel(TreeHdr* h, int32_t* blocksum, int L, int cap) {
-    if (h->err) return;
-    const int le = h->level_begin[L + 1];
-    const int64_t tot = cta_exclusive_scan(
-        kLevelBlocks, [&](int i) { return (int64_t)blocksum[i]; },
-        [&](int i, int64_t v) { blocksum[i] = (int32_t)min(v, (int64_t)cap); });
-    if (threadIdx.x == 0) {
-        if ((int64_t)le + tot > cap) {
-            h->err |= kErrCells;
-            h->level_begin[L + 2] = le;
-        } else {
-            h->level_begin[L + 2] = le + (int)tot;
-        }
-    }
-}
-
-__global__ __launch_bounds__(256) void fill_kernel(TreeHdr* h, TCell* cells, const int32_t* __restrict__ nch,
-                                                   const int4* __restrict__ bnd, const int32_t* __restrict__ blockoff,
-                                                   int L) {
-    if (h->err) return;
-    int c0, c1;
-    level_chunk(h, L, c0, c1);
-    const int lb = h->level_begin[L], le = h->level_begin[L + 1];
-    int run = le + blockoff[blockIdx.x];
-    for (int t0 = c0; t0 < c1; t0 += blockDim.x) {  // uniform trip count over the CTA
-        const int c = t0 + (int)threadIdx.x;
-        const int k_c = c < c1 ? nch[c - lb] : 0;
-        int tot;
-        const int off = cta256_excl_scan(k_c, &tot);
-        if (c < c1 && k_c > 0) {
-            TCell& cc = cells[c];
-            const int first = run + off;
-            cc.first_child = first;
-            const int4 u = bnd[2 * (c - lb)], v = bnd[2 * (c - lb) + 1];
-            const int b[9] = {cc.begin, u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
-            int k = 0;
-            for (int o = 0; o < 8; ++o) {
-                if (b[o + 1] <= b[o]) continue;
-                TCell& ch = cells[first + k++];
-                ch.begin = b[o];
-                ch.end = b[o + 1];
-                ch.level = L + 1;
-                ch.parent = c;
-                ch.first_child = 0;
-                ch.n_child = 0;
-                ch.leaf = 0;
-            }
-        } else if (c < c1) {
-            cells[c].first_child = run + off;
-        }
-        run += tot;
-    }
-}
-
-// Moments, boxes and the SPJ records: LEAVES, every leaf of the tree from
-// its particles; otherwise the inner cells of level L from their children
-// (run deepest level first).
 // The cells in moments classes, so that the threads of a warp run loops of
 // the same length (GB300 issues each FP64 instruction for the whole warp,
 // whatever its active lanes): leaves by particle count, largest first, then
@@ -536,95 +444,210 @@ __device__ __forceinline__ int cell_bin(const TCell& c) {
     return kLeafBins + 8 * c.level + (8 - c.n_child);
 }
 
-// First slot of class b in the cell list (after the scatter).
-__device__ __forceinline__ int bin_start(const TreeHdr* h, int b) { return b == 0 ? 0 : h->cell_cursor[b - 1]; }
+struct TreeArgs {
+    TreeHdr* h;
+    TCell* cells;
+    TCellW* cw;
+    CMom* mom;
+    int32_t* nch;
+    int4* bnd;          // per cell of the level being split: its octant ends (2 x 4)
+    int32_t* blocksum;  // child counts per CTA
+    const uint64_t* skey;
+    int32_t* order;     // cells by moments class
+    const EpiDev* epi;
+    const double* m64;
+    double inv_theta2;
+    int n_leaf, cap;
+    SpjMix* spj;
+    SpjF32* spj32;
+    SpjQ64* spjq;
+};
 
-__global__ __launch_bounds__(256) void cell_hist_kernel(TreeHdr* h, const TCell* __restrict__ cells) {
-    __shared__ int hs[kCellBins];
-    for (int b = threadIdx.x; b < kCellBins; b += blockDim.x) hs[b] = 0;
-    __syncthreads();
-    if (!h->err) {
-        const int nc = h->level_begin[kLevels];
-        for (int64_t c = gtid(); c < nc; c += gstride()) atomicAdd(&hs[cell_bin(cells[c])], 1);
+// Moments, boxes and SPJ records of one cell: a leaf from its particles in
+// sorted order, an inner cell from its children in child order.
+__device__ void cell_moments(const TreeArgs& a, int64_t c) {
+    TCell& cc = a.cells[c];
+    const double side = ldexp(a.h->side0, -cc.level);
+    double m = 0, mx[3] = {0, 0, 0}, q[6] = {0, 0, 0, 0, 0, 0};
+    double ilo[3], ihi[3], olo[3], ohi[3];
+    for (int d = 0; d < 3; ++d) {
+        ilo[d] = olo[d] = 1e300;
+        ihi[d] = ohi[d] = -1e300;
     }
-    __syncthreads();
-    for (int b = threadIdx.x; b < kCellBins; b += blockDim.x)
-        if (hs[b]) atomicAdd(&h->cell_hist[b], hs[b]);
-}
-
-__global__ void cell_scan_kernel(TreeHdr* h) {
-    if (threadIdx.x != 0) return;
-    int run = 0;
-    for (int b = 0; b < kCellBins; ++b) {
-        h->cell_cursor[b] = run;
-        run += h->cell_hist[b];
-    }
-}
-
-__global__ __launch_bounds__(256) void cell_scatter_kernel(TreeHdr* h, const TCell* __restrict__ cells,
-                                                           int32_t* __restrict__ order) {
-    __shared__ int hs[kCellBins], base[kCellBins];
-    const int nc = h->err ? 0 : h->level_begin[kLevels];
-    for (int64_t c0 = (int64_t)blockIdx.x * blockDim.x; c0 < nc; c0 += gstride()) {
-        for (int b = threadIdx.x; b < kCellBins; b += blockDim.x) hs[b] = 0;
-        __syncthreads();
-        const int64_t c = c0 + threadIdx.x;
-        int b = -1, r = 0;
-        if (c < nc) {
-            b = cell_bin(cells[c]);
-            r = atomicAdd(&hs[b], 1);
+    double rsm = 0.0;
+    if (cc.leaf) {
+        for (int i = cc.begin; i < cc.end; ++i) {
+            const EpiDev e = a.epi[i];
+            const double mi = a.m64[i];
+            const double x[3] = {e.x, e.y, e.z};
+            m += mi;
+            for (int d = 0; d < 3; ++d) {
+                mx[d] += mi * x[d];
+                ilo[d] = kmin(ilo[d], x[d]);
+                ihi[d] = kmax(ihi[d], x[d]);
+                olo[d] = kmin(olo[d], x[d] - e.rs);
+                ohi[d] = kmax(ohi[d], x[d] + e.rs);
+            }
+            rsm = kmax(rsm, e.rs);
         }
-        __syncthreads();
-        for (int k = threadIdx.x; k < kCellBins; k += blockDim.x)
-            base[k] = hs[k] ? atomicAdd(&h->cell_cursor[k], hs[k]) : 0;
-        __syncthreads();
-        if (b >= 0) order[base[b] + r] = (int32_t)c;
-        __syncthreads();
+    } else {
+        for (int k = 0; k < cc.n_child; ++k) {
+            const int ci = cc.first_child + k;
+            const CMom& cm = a.mom[ci];
+            const TCell& ch = a.cells[ci];
+            m += cm.m;
+            for (int d = 0; d < 3; ++d) {
+                mx[d] += cm.mx[d];
+                ilo[d] = kmin(ilo[d], ch.in_lo[d]);
+                ihi[d] = kmax(ihi[d], ch.in_hi[d]);
+                olo[d] = kmin(olo[d], ch.out_lo[d]);
+                ohi[d] = kmax(ohi[d], ch.out_hi[d]);
+            }
+            rsm = kmax(rsm, (double)ch.rs_max);
+        }
     }
+    double com[3];
+    for (int d = 0; d < 3; ++d) com[d] = m > 0 ? mx[d] / m : 0.5 * (ilo[d] + ihi[d]);
+    if (cc.leaf) {
+        for (int i = cc.begin; i < cc.end; ++i) {
+            const EpiDev e = a.epi[i];
+            const double mi = a.m64[i];
+            const double dx = e.x - com[0], dy = e.y - com[1], dz = e.z - com[2];
+            q[0] += mi * dx * dx;
+            q[1] += mi * dy * dy;
+            q[2] += mi * dz * dz;
+            q[3] += mi * dx * dy;
+            q[4] += mi * dx * dz;
+            q[5] += mi * dy * dz;
+        }
+    } else {
+        for (int k = 0; k < cc.n_child; ++k) {
+            const int ci = cc.first_child + k;
+            const CMom& cm = a.mom[ci];
+            const TCell& ch = a.cells[ci];
+            const double dx = ch.com[0] - com[0], dy = ch.com[1] - com[1], dz = ch.com[2] - com[2];
+            q[0] += cm.q[0] + cm.m * dx * dx;
+            q[1] += cm.q[1] + cm.m * dy * dy;
+            q[2] += cm.q[2] + cm.m * dz * dz;
+            q[3] += cm.q[3] + cm.m * dx * dy;
+            q[4] += cm.q[4] + cm.m * dx * dz;
+            q[5] += cm.q[5] + cm.m * dy * dz;
+        }
+    }
+    for (int d = 0; d < 3; ++d) {
+        cc.com[d] = com[d];
+        cc.in_lo[d] = ilo[d];
+        cc.in_hi[d] = ihi[d];
+        cc.out_lo[d] = olo[d];
+        cc.out_hi[d] = ohi[d];
+    }
+    cc.crit = side * side * a.inv_theta2;
+    cc.rs_max = __double2float_ru(rsm);
+    TCellW w;
+    for (int d = 0; d < 3; ++d) {
+        w.com[d] = (float)com[d];
+        w.in_lo[d] = (float)ilo[d];
+        w.in_hi[d] = (float)ihi[d];
+        w.out_lo[d] = (float)olo[d];
+        w.out_hi[d] = (float)ohi[d];
+    }
+    w.crit = (float)cc.crit;
+    w.begin = cc.begin;
+    w.end = cc.end;
+    w.first_child = cc.first_child;
+    w.n_child = cc.n_child;
+    w.leaf = cc.leaf;
+    w.parent = cc.parent;
+    w.level = cc.level;
+    {
+        const float a = 0.5772f * ((float)sqrt(cc.crit) * 0.9999f - 1.7322f * (float)side);
+        w.apart = a > cc.rs_max ? a : 0.f;
+    }
+    a.cw[c] = w;
+    CMom& o = a.mom[c];
+    o.m = m;
+    for (int d = 0; d < 3; ++d) o.mx[d] = mx[d];
+    for (int k = 0; k < 6; ++k) o.q[k] = q[k];
+    // SPJ records of the cell, as the dispatch path packs them.
+    const double tr = q[0] + q[1] + q[2];
+    SpjMix s;
+    s.x = com[0];
+    s.y = com[1];
+    s.z = com[2];
+    s.m = (float)m;
+    s.pad0 = 0.f;
+    s.Q[0] = (float)(3.0 * q[0] - tr);
+    s.Q[1] = (float)(3.0 * q[1] - tr);
+    s.Q[2] = (float)(3.0 * q[2] - tr);
+    s.Q[3] = (float)(3.0 * q[3]);
+    s.Q[4] = (float)(3.0 * q[4]);
+    s.Q[5] = (float)(3.0 * q[5]);
+    s.tr = (float)tr;
+    s.pad1 = 0.f;
+    a.spj[c] = s;
+    SpjF32 f;
+    f.xh = (float)com[0];
+    f.yh = (float)com[1];
+    f.zh = (float)com[2];
+    f.xl = (float)(com[0] - (double)f.xh);
+    f.yl = (float)(com[1] - (double)f.yh);
+    f.zl = (float)(com[2] - (double)f.zh);
+    f.m = s.m;
+    f.tr = s.tr;
+    for (int k = 0; k < 6; ++k) f.Q[k] = s.Q[k];
+    f.pad[0] = f.pad[1] = 0.f;
+    a.spj32[c] = f;
+    SpjQ64 d64;
+    d64.m = m;
+    for (int k = 0; k < 6; ++k) d64.q[k] = q[k];
+    d64.pad = 0.0;
+    a.spjq[c] = d64;
 }
 
-template <bool LEAVES>
-__global__ __launch_bounds__(256) void moments_kernel(const TreeHdr* h, TCell* cells, TCellW* cw, CMom* mom,
-                                                      const EpiDev* __restrict__ epi, const double* __restrict__ m64,
-                                                      int L, double inv_theta2, SpjMix* spj, SpjF32* spj32,
-                                                      SpjQ64* spjq, const int32_t* __restrict__ order) {
-    if (h->err) return;
-    const int lb = LEAVES ? 0 : bin_start(h, kLeafBins + 8 * L);
-    const int le = LEAVES ? bin_start(h, kLeafBins) : bin_start(h, kLeafBins + 8 * L + 8);
-    for (int64_t t = lb + gtid(); t < le; t += gstride()) {
-        const int64_t c = order[t];
-        TCell& cc = cells[c];
-        const double side = ldexp(h->side0, -cc.level);
-        double m = 0, mx[3] = {0, 0, 0}, q[6] = {0, 0, 0, 0, 0, 0};
-        double ilo[3], ihi[3], olo[3], ohi[3];
-        for (int d = 0; d < 3; ++d) {
-            ilo[d] = olo[d] = 1e300;
-            ihi[d] = ohi[d] = -1e300;
-        }
-        double rsm = 0.0;
-        if (cc.leaf) {
-            for (int i = cc.begin; i < cc.end; ++i) {
-                const EpiDev e = epi[i];
-                const double mi = m64[i];
+// The same for the cell of a group of eight lanes (all 32 lanes call it; act:
+// whether this group has a cell): a lane per child or particle computes its
+// terms, and a lane per component adds them in the order of cell_moments, so
+// the results are the same.  Where cells are few, this is the latency of tens
+// of FP64 instructions instead of hundreds (64 cycles each).
+__device__ void cell_moments8(const TreeArgs& a, int64_t c, bool act, double (*__restrict__ buf)[8]) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int k = threadIdx.x & 7;
+    const int src = threadIdx.x & 24;  // first lane of the group
+    const TCell* const cc = a.cells + (act ? c : 0);
+    const bool leaf = act && cc->leaf;
+    const int begin = act ? (leaf ? cc->begin : cc->first_child) : 0;
+    const int n = act ? (leaf ? cc->end - cc->begin : cc->n_child) : 0;
+    int rounds = (n + 7) >> 3;
+#pragma unroll
+    for (int o = 8; o < 32; o <<= 1) rounds = max(rounds, __shfl_xor_sync(kAll, rounds, o));
+    double ilo[3], ihi[3], olo[3], ohi[3], rsm = 0.0;
+    for (int d = 0; d < 3; ++d) {
+        ilo[d] = olo[d] = 1e300;
+        ihi[d] = ohi[d] = -1e300;
+    }
+    double sum = 0.0;  // lanes 0..3: m, mx, my, mz
+    for (int r = 0; r < rounds; ++r) {
+        const int i = r * 8 + k, here = min(8, n - r * 8);
+        if (i < n) {
+            if (leaf) {
+                const EpiDev e = a.epi[begin + i];
+                const double mi = a.m64[begin + i];
                 const double x[3] = {e.x, e.y, e.z};
-                m += mi;
+                buf[0][k] = mi;
                 for (int d = 0; d < 3; ++d) {
-                    mx[d] += mi * x[d];
+                    buf[1 + d][k] = mi * x[d];
                     ilo[d] = kmin(ilo[d], x[d]);
                     ihi[d] = kmax(ihi[d], x[d]);
                     olo[d] = kmin(olo[d], x[d] - e.rs);
                     ohi[d] = kmax(ohi[d], x[d] + e.rs);
                 }
                 rsm = kmax(rsm, e.rs);
-            }
-        } else {
-            for (int k = 0; k < cc.n_child; ++k) {
-                const int ci = cc.first_child + k;
-                const CMom& cm = mom[ci];
-                const TCell& ch = cells[ci];
-                m += cm.m;
+            } else {
+                const CMom& cm = a.mom[begin + i];
+                const TCell& ch = a.cells[begin + i];
+                buf[0][k] = cm.m;
                 for (int d = 0; d < 3; ++d) {
-                    mx[d] += cm.mx[d];
+                    buf[1 + d][k] = cm.mx[d];
                     ilo[d] = kmin(ilo[d], ch.in_lo[d]);
                     ihi[d] = kmax(ihi[d], ch.in_hi[d]);
                     olo[d] = kmin(olo[d], ch.out_lo[d]);
@@ -633,102 +656,317 @@ __global__ __launch_bounds__(256) void moments_kernel(const TreeHdr* h, TCell* c
                 rsm = kmax(rsm, (double)ch.rs_max);
             }
         }
-        double com[3];
-        for (int d = 0; d < 3; ++d) com[d] = m > 0 ? mx[d] / m : 0.5 * (ilo[d] + ihi[d]);
-        if (cc.leaf) {
-            for (int i = cc.begin; i < cc.end; ++i) {
-                const EpiDev e = epi[i];
-                const double mi = m64[i];
-                const double dx = e.x - com[0], dy = e.y - com[1], dz = e.z - com[2];
-                q[0] += mi * dx * dx;
-                q[1] += mi * dy * dy;
-                q[2] += mi * dz * dz;
-                q[3] += mi * dx * dy;
-                q[4] += mi * dx * dz;
-                q[5] += mi * dy * dz;
+        __syncwarp();
+        if (k < 4)
+            for (int q = 0; q < here; ++q) sum += buf[k][q];
+        __syncwarp();
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+        const bool up = k & o;
+        // the lower lane's value is the first operand, as in the sequence
+        auto both = [&](double v, bool mx) {
+            const double u = __shfl_xor_sync(kAll, v, o);
+            const double p = up ? u : v, q = up ? v : u;
+            return mx ? kmax(p, q) : kmin(p, q);
+        };
+        for (int d = 0; d < 3; ++d) {
+            ilo[d] = both(ilo[d], false);
+            ihi[d] = both(ihi[d], true);
+            olo[d] = both(olo[d], false);
+            ohi[d] = both(ohi[d], true);
+        }
+        rsm = both(rsm, true);
+    }
+    const double m = __shfl_sync(kAll, sum, src);
+    // lanes 1..3: one coordinate of the centre of mass each
+    double cd = 0.0;
+    if (act && k >= 1 && k < 4) {
+        const int d = k - 1;
+        const double lo = d == 0 ? ilo[0] : (d == 1 ? ilo[1] : ilo[2]), hi = d == 0 ? ihi[0] : (d == 1 ? ihi[1] : ihi[2]);
+        cd = m > 0 ? sum / m : 0.5 * (lo + hi);
+    }
+    double com[3];
+    for (int d = 0; d < 3; ++d) com[d] = __shfl_sync(kAll, cd, src + 1 + d);
+    double q = 0.0;  // lanes 0..5: the second moment
+    for (int r = 0; r < rounds; ++r) {
+        const int i = r * 8 + k, here = min(8, n - r * 8);
+        if (i < n) {
+            double mi, x[3], q0[6] = {0, 0, 0, 0, 0, 0};
+            if (leaf) {
+                const EpiDev e = a.epi[begin + i];
+                mi = a.m64[begin + i];
+                x[0] = e.x;
+                x[1] = e.y;
+                x[2] = e.z;
+            } else {
+                const CMom& cm = a.mom[begin + i];
+                const TCell& ch = a.cells[begin + i];
+                mi = cm.m;
+                for (int d = 0; d < 3; ++d) x[d] = ch.com[d];
+                for (int u = 0; u < 6; ++u) q0[u] = cm.q[u];
+            }
+            const double dx = x[0] - com[0], dy = x[1] - com[1], dz = x[2] - com[2];
+            double t[6] = {mi * dx * dx, mi * dy * dy, mi * dz * dz, mi * dx * dy, mi * dx * dz, mi * dy * dz};
+            for (int u = 0; u < 6; ++u) buf[u][k] = leaf ? t[u] : q0[u] + t[u];
+        }
+        __syncwarp();
+        if (k < 6)
+            for (int u = 0; u < here; ++u) q += buf[k][u];
+        __syncwarp();
+    }
+    const double tr = __shfl_sync(kAll, q, src) + __shfl_sync(kAll, q, src + 1) + __shfl_sync(kAll, q, src + 2);
+    const double mxd = __shfl_sync(kAll, sum, src + 1 + (k < 3 ? k : 0));
+    if (!act) return;
+    TCell& cell = a.cells[c];
+    TCellW& w = a.cw[c];
+    if (k < 3) {
+        const double cx = k == 0 ? com[0] : (k == 1 ? com[1] : com[2]);
+        const double v[4] = {k == 0 ? ilo[0] : (k == 1 ? ilo[1] : ilo[2]), k == 0 ? ihi[0] : (k == 1 ? ihi[1] : ihi[2]),
+                             k == 0 ? olo[0] : (k == 1 ? olo[1] : olo[2]), k == 0 ? ohi[0] : (k == 1 ? ohi[1] : ohi[2])};
+        cell.com[k] = cx;
+        cell.in_lo[k] = v[0];
+        cell.in_hi[k] = v[1];
+        cell.out_lo[k] = v[2];
+        cell.out_hi[k] = v[3];
+        const float ch = (float)cx;
+        w.com[k] = ch;
+        w.in_lo[k] = (float)v[0];
+        w.in_hi[k] = (float)v[1];
+        w.out_lo[k] = (float)v[2];
+        w.out_hi[k] = (float)v[3];
+        a.mom[c].mx[k] = mxd;
+        (&a.spj[c].x)[k] = cx;
+        (&a.spj32[c].xh)[k] = ch;
+        (&a.spj32[c].xl)[k] = (float)(cx - (double)ch);
+    }
+    if (k < 6) {
+        a.mom[c].q[k] = q;
+        a.spjq[c].q[k] = q;
+        const float f = k < 3 ? (float)(3.0 * q - tr) : (float)(3.0 * q);
+        a.spj[c].Q[k] = f;
+        a.spj32[c].Q[k] = f;
+    } else if (k == 6) {
+        const double side = ldexp(a.h->side0, -cell.level);
+        const double crit = side * side * a.inv_theta2;
+        const float rs = __double2float_ru(rsm);
+        cell.crit = crit;
+        cell.rs_max = rs;
+        w.crit = (float)crit;
+        const float ap = 0.5772f * ((float)sqrt(crit) * 0.9999f - 1.7322f * (float)side);
+        w.apart = ap > rs ? ap : 0.f;
+        w.begin = cell.begin;
+        w.end = cell.end;
+        w.first_child = cell.first_child;
+        w.n_child = cell.n_child;
+        w.leaf = cell.leaf;
+        w.parent = cell.parent;
+        w.level = cell.level;
+    } else {
+        const float mf = (float)m, tf = (float)tr;
+        a.mom[c].m = m;
+        a.spj[c].m = mf;
+        a.spj[c].pad0 = 0.f;
+        a.spj[c].tr = tf;
+        a.spj[c].pad1 = 0.f;
+        a.spj32[c].m = mf;
+        a.spj32[c].tr = tf;
+        a.spj32[c].pad[0] = a.spj32[c].pad[1] = 0.f;
+        a.spjq[c].m = m;
+        a.spjq[c].pad = 0.0;
+    }
+}
+
+// Cells [lo, hi) of the class order.
+__device__ __forceinline__ void moments_range(const TreeArgs& a, int lo, int hi, double (*buf)[8]) {
+    const int64_t threads = (int64_t)gridDim.x * kTreeThreads;
+    if ((int64_t)(hi - lo) * 8 <= threads) {
+        // a group of eight lanes per cell, one round
+        const int64_t base = lo + (((int64_t)blockIdx.x * kTreeThreads + (threadIdx.x & ~31)) >> 3);
+        if (base >= hi) return;  // whole warps
+        const int64_t t = base + ((threadIdx.x & 31) >> 3);
+        cell_moments8(a, t < hi ? a.order[t] : 0, t < hi, buf);
+        return;
+    }
+    for (int64_t t = lo + gtid(); t < hi; t += threads) cell_moments(a, a.order[t]);
+}
+
+__global__ __launch_bounds__(kTreeThreads, 1) void tree_kernel(TreeArgs a) {
+    __shared__ double s_buf[kTreeWarps][4][6][8];
+    __shared__ int s_hist[kCellBins + 1], s_base[kCellBins];
+    __shared__ int s_b[9], s_before, s_total, s_sum;
+    TreeHdr* const h = a.h;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int G = gridDim.x, bid = blockIdx.x;
+    unsigned epoch = 0;
+    if (h->err) return;  // before the first barrier: every CTA sees it
+    // ---- levels: children of a level in their parents' order ----
+    int lb = 0, le = 1, depth = 0;
+    for (int L = 0; L < kLevels; ++L) {
+        depth = L;
+        const int per = (le - lb + G - 1) / G;
+        const int c0 = min(le, lb + bid * per), c1 = min(le, c0 + per);
+        const int shift = 3 * (kMaxLevel - 1 - L);
+        if (t == 0) s_sum = 0;
+        __syncthreads();
+        if (per <= 2) {
+            // Few, large cells: a warp per octant boundary.
+            for (int c = c0; c < c1; ++c) {
+                const int b0 = a.cells[c].begin, b1 = a.cells[c].end;
+                const bool leaf = b1 - b0 <= a.n_leaf || L >= kMaxLevel;
+                if (!leaf && warp < 7) {
+                    const int b = warp_octant(a.skey, b0, b1, shift, warp + 1);
+                    if (lane == 0) s_b[warp + 1] = b;
+                }
+                __syncthreads();
+                if (t == 0) {
+                    int n = 0;
+                    if (!leaf) {
+                        s_b[0] = b0;
+                        s_b[8] = b1;
+                        for (int o = 0; o < 8; ++o) n += s_b[o + 1] > s_b[o];
+                        a.bnd[2 * (c - lb)] = make_int4(s_b[1], s_b[2], s_b[3], s_b[4]);
+                        a.bnd[2 * (c - lb) + 1] = make_int4(s_b[5], s_b[6], s_b[7], s_b[8]);
+                    }
+                    a.cells[c].leaf = leaf;
+                    a.cells[c].n_child = n;
+                    a.nch[c - lb] = n;
+                    s_sum += n;
+                }
+                __syncthreads();
             }
         } else {
-            for (int k = 0; k < cc.n_child; ++k) {
-                const int ci = cc.first_child + k;
-                const CMom& cm = mom[ci];
-                const TCell& ch = cells[ci];
-                const double dx = ch.com[0] - com[0], dy = ch.com[1] - com[1], dz = ch.com[2] - com[2];
-                q[0] += cm.q[0] + cm.m * dx * dx;
-                q[1] += cm.q[1] + cm.m * dy * dy;
-                q[2] += cm.q[2] + cm.m * dz * dz;
-                q[3] += cm.q[3] + cm.m * dx * dy;
-                q[4] += cm.q[4] + cm.m * dx * dz;
-                q[5] += cm.q[5] + cm.m * dy * dz;
+            // Eight lanes per cell, seven of them searching one boundary each.
+            const int k = lane & 7, src = lane & 24;
+            for (int base = c0 + (t >> 5) * 4; base < c1; base += kTreeWarps * 4) {
+                const int c = base + (lane >> 3);
+                const bool act = c < c1;
+                const int b0 = act ? a.cells[c].begin : 0, b1 = act ? a.cells[c].end : 0;
+                const bool leaf = !act || b1 - b0 <= a.n_leaf || L >= kMaxLevel;
+                int bo = b1;
+                if (!leaf && k < 7) {
+                    int lo = b0, hi = b1;  // first index with digit >= k + 1
+                    while (lo < hi) {
+                        const int mid = (lo + hi) >> 1;
+                        if ((int)((a.skey[mid] >> shift) & 7) < k + 1) lo = mid + 1;
+                        else hi = mid;
+                    }
+                    bo = lo;
+                }
+                // child k holds [end of child k - 1, bo)
+                const int prev = __shfl_up_sync(0xffffffffu, bo, 1);
+                const bool has = !leaf && bo > (k ? prev : b0);
+                const unsigned m = __ballot_sync(0xffffffffu, has);
+                const int n = __popc((m >> src) & 0xffu);
+                if (act && !leaf) reinterpret_cast<int*>(a.bnd + 2 * (c - lb))[k] = bo;
+                if (act && k == 0) {
+                    a.cells[c].leaf = leaf;
+                    a.cells[c].n_child = n;
+                    a.nch[c - lb] = n;
+                    if (n) atomicAdd(&s_sum, n);
+                }
             }
         }
-        for (int d = 0; d < 3; ++d) {
-            cc.com[d] = com[d];
-            cc.in_lo[d] = ilo[d];
-            cc.in_hi[d] = ihi[d];
-            cc.out_lo[d] = olo[d];
-            cc.out_hi[d] = ohi[d];
+        __syncthreads();
+        if (t == 0) {
+            a.blocksum[(L & 1) * G + bid] = s_sum;
+            s_before = s_total = 0;
         }
-        cc.crit = side * side * inv_theta2;
-        cc.rs_max = __double2float_ru(rsm);
-        TCellW w;
-        for (int d = 0; d < 3; ++d) {
-            w.com[d] = (float)com[d];
-            w.in_lo[d] = (float)ilo[d];
-            w.in_hi[d] = (float)ihi[d];
-            w.out_lo[d] = (float)olo[d];
-            w.out_hi[d] = (float)ohi[d];
+        if (!grid_sync(&h->bar, epoch, &h->err)) return;
+        for (int k = t; k < G; k += kTreeThreads) {
+            const int v = __ldcg(a.blocksum + (L & 1) * G + k);
+            if (v) {
+                atomicAdd(&s_total, v);
+                if (k < bid) atomicAdd(&s_before, v);
+            }
         }
-        w.crit = (float)cc.crit;
-        w.begin = cc.begin;
-        w.end = cc.end;
-        w.first_child = cc.first_child;
-        w.n_child = cc.n_child;
-        w.leaf = cc.leaf;
-        w.parent = cc.parent;
-        w.level = cc.level;
-        {
-            const float a = 0.5772f * ((float)sqrt(cc.crit) * 0.9999f - 1.7322f * (float)side);
-            w.apart = a > cc.rs_max ? a : 0.f;
+        __syncthreads();
+        const int total = s_total;
+        if ((int64_t)le + total > a.cap) {
+            if (bid == 0 && t == 0) h->err |= kErrCells;
+            if (bid == 0 && t <= kLevels + 1 && t > L + 1) h->level_begin[t] = le;
+            return;  // every CTA
         }
-        cw[c] = w;
-        CMom& o = mom[c];
-        o.m = m;
-        for (int d = 0; d < 3; ++d) o.mx[d] = mx[d];
-        for (int k = 0; k < 6; ++k) o.q[k] = q[k];
-        // SPJ records of the cell, as the dispatch path packs them.
-        const double tr = q[0] + q[1] + q[2];
-        SpjMix s;
-        s.x = com[0];
-        s.y = com[1];
-        s.z = com[2];
-        s.m = (float)m;
-        s.pad0 = 0.f;
-        s.Q[0] = (float)(3.0 * q[0] - tr);
-        s.Q[1] = (float)(3.0 * q[1] - tr);
-        s.Q[2] = (float)(3.0 * q[2] - tr);
-        s.Q[3] = (float)(3.0 * q[3]);
-        s.Q[4] = (float)(3.0 * q[4]);
-        s.Q[5] = (float)(3.0 * q[5]);
-        s.tr = (float)tr;
-        s.pad1 = 0.f;
-        spj[c] = s;
-        SpjF32 f;
-        f.xh = (float)com[0];
-        f.yh = (float)com[1];
-        f.zh = (float)com[2];
-        f.xl = (float)(com[0] - (double)f.xh);
-        f.yl = (float)(com[1] - (double)f.yh);
-        f.zl = (float)(com[2] - (double)f.zh);
-        f.m = s.m;
-        f.tr = s.tr;
-        for (int k = 0; k < 6; ++k) f.Q[k] = s.Q[k];
-        f.pad[0] = f.pad[1] = 0.f;
-        spj32[c] = f;
-        SpjQ64 d64;
-        d64.m = m;
-        for (int k = 0; k < 6; ++k) d64.q[k] = q[k];
-        d64.pad = 0.0;
-        spjq[c] = d64;
+        int run = le + s_before;
+        for (int t0 = c0; t0 < c1; t0 += kTreeThreads) {  // uniform trip count over the CTA
+            const int c = t0 + t;
+            const int n = c < c1 ? a.nch[c - lb] : 0;
+            int tot;
+            const int off = cta_excl_scan(n, &tot);
+            if (c < c1) {
+                TCell& cc = a.cells[c];
+                const int first = run + off;
+                cc.first_child = first;
+                if (n > 0) {
+                    const int4 u = a.bnd[2 * (c - lb)], v = a.bnd[2 * (c - lb) + 1];
+                    const int b[9] = {cc.begin, u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+                    int k = 0;
+                    for (int o = 0; o < 8; ++o) {
+                        if (b[o + 1] <= b[o]) continue;
+                        TCell& ch = a.cells[first + k++];
+                        ch.begin = b[o];
+                        ch.end = b[o + 1];
+                        ch.level = L + 1;
+                        ch.parent = c;
+                        ch.first_child = 0;
+                        ch.n_child = 0;
+                        ch.leaf = 0;
+                    }
+                }
+            }
+            run += tot;
+        }
+        if (bid == 0 && t == 0) h->level_begin[L + 2 <= kLevels + 1 ? L + 2 : kLevels + 1] = le + total;
+        if (total == 0) break;  // every CTA
+        if (!grid_sync(&h->bar, epoch, &h->err)) return;
+        lb = le;
+        le += total;
+    }
+    const int nc = le;
+    if (bid == 0 && t > depth + 1 && t <= kLevels + 1) h->level_begin[t] = nc;
+    // ---- class order ----
+    for (int b = t; b < kCellBins; b += kTreeThreads) s_hist[b] = 0;
+    if (!grid_sync(&h->bar, epoch, &h->err)) return;  // first_child and leaf flags of the last level
+    for (int64_t c = gtid(); c < nc; c += gstride()) atomicAdd(&s_hist[cell_bin(a.cells[c])], 1);
+    __syncthreads();
+    for (int b = t; b < kCellBins; b += kTreeThreads)
+        if (s_hist[b]) atomicAdd(&h->cell_hist[b], s_hist[b]);
+    if (!grid_sync(&h->bar, epoch, &h->err)) return;
+    {
+        static_assert(kCellBins <= kTreeThreads, "one bin per thread");
+        int tot;
+        const int v = t < kCellBins ? __ldcg(&h->cell_hist[t]) : 0;
+        const int off = cta_excl_scan(v, &tot);
+        if (t < kCellBins) s_hist[t] = off;
+        if (t == 0) s_hist[kCellBins] = tot;
+        __syncthreads();
+    }
+    // s_hist: first slot of each class
+    for (int64_t cb = (int64_t)bid * kTreeThreads; cb < nc; cb += (int64_t)G * kTreeThreads) {
+        for (int b = t; b < kCellBins; b += kTreeThreads) s_base[b] = 0;
+        __syncthreads();
+        const int64_t c = cb + t;
+        int b = -1, r = 0;
+        if (c < nc) {
+            b = cell_bin(a.cells[c]);
+            r = atomicAdd(&s_base[b], 1);
+        }
+        __syncthreads();
+        for (int k = t; k < kCellBins; k += kTreeThreads)
+            if (s_base[k]) s_base[k] = s_hist[k] + atomicAdd(&h->cell_cursor[k], s_base[k]);
+        __syncthreads();
+        if (b >= 0) a.order[s_base[b] + r] = (int32_t)c;
+        __syncthreads();
+    }
+    if (!grid_sync(&h->bar, epoch, &h->err)) return;
+    // ---- moments: leaves, then the inner cells from the deepest level up ----
+    double (*const buf)[8] = s_buf[warp][lane >> 3];
+    moments_range(a, 0, s_hist[kLeafBins], buf);
+    for (int L = depth; L >= 0; --L) {
+        const int lo = s_hist[kLeafBins + 8 * L], hi = s_hist[kLeafBins + 8 * L + 8];
+        if (lo == hi) continue;  // every CTA
+        if (!grid_sync(&h->bar, epoch, &h->err)) return;
+        moments_range(a, lo, hi, buf);
     }
 }
 
@@ -1581,21 +1819,14 @@ cudaError_t enqueue_build(pgf_nbody* h) {
     gather_kernel<<<gn, 256, 0, s>>>(h->order.d, h->pos.d, h->mass.d, h->rs.d, n, h->epi.d, h->epj.d, h->epj_m64.d,
                                      h->epj_rs64.d, h->epj32.d, h->inv_order.d);
     const int gc = grid_for(h, h->cap_cells, 256);
-    for (int L = 0; L < kLevels; ++L) {
-        split_kernel<<<kLevelBlocks, 256, 0, s>>>(hd, h->cells.d, h->nch.d, h->bnd.d, h->blocksum.d, h->key_out.d, L,
-                                                  h->cfg.n_leaf_limit);
-        level_scan_kernel<<<1, kScanThreads, 0, s>>>(hd, h->blocksum.d, L, h->cap_cells);
-        fill_kernel<<<kLevelBlocks, 256, 0, s>>>(hd, h->cells.d, h->nch.d, h->bnd.d, h->blocksum.d, L);
+    {
+        TreeArgs a{hd, h->cells.d, h->cw.d, h->mom.d, h->nch.d, h->bnd.d, h->blocksum.d, h->key_out.d, h->cell_order.d,
+                   h->epi.d, h->epj_m64.d, h->inv_theta2, h->cfg.n_leaf_limit, h->cap_cells, h->spj.d, h->spj32.d,
+                   h->spjq.d};
+        void* args[] = {&a};
+        e = cudaLaunchCooperativeKernel((const void*)tree_kernel, dim3(h->num_sms), dim3(kTreeThreads), args, 0, s);
+        if (e != cudaSuccess) return e;
     }
-    cell_hist_kernel<<<h->num_sms * 2, 256, 0, s>>>(hd, h->cells.d);
-    cell_scan_kernel<<<1, 32, 0, s>>>(hd);
-    cell_scatter_kernel<<<h->num_sms * 2, 256, 0, s>>>(hd, h->cells.d, h->cell_order.d);
-    moments_kernel<true><<<gc, 256, 0, s>>>(hd, h->cells.d, h->cw.d, h->mom.d, h->epi.d, h->epj_m64.d, 0,
-                                            h->inv_theta2, h->spj.d, h->spj32.d, h->spjq.d, h->cell_order.d);
-    const int gm = h->num_sms * 2;
-    for (int L = kLevels - 1; L >= 0; --L)
-        moments_kernel<false><<<gm, 256, 0, s>>>(hd, h->cells.d, h->cw.d, h->mom.d, h->epi.d, h->epj_m64.d, L,
-                                                 h->inv_theta2, h->spj.d, h->spj32.d, h->spjq.d, h->cell_order.d);
     if ((e = cudaMemsetAsync(h->group_at.d, 0xff, sizeof(int32_t) * n, s)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(h->front_at.d, 0xff, sizeof(int32_t) * n, s)) != cudaSuccess) return e;
     group_mark_kernel<<<gc, 256, 0, s>>>(hd, h->cells.d, h->group_at.d, h->cfg.n_group_limit);
@@ -1916,7 +2147,7 @@ int pgf_nbody_create(const pgf_nbody_config* cfg, int64_t n, const double* pos, 
     NB_TRY(h->id_epj.alloc(h->cap_e));
     NB_TRY(alloc_spj(h));
     if (far_applies(cfg->eps2, n)) NB_TRY(h->spj_near.alloc(n));
-    NB_TRY(h->blocksum.alloc(kLevelBlocks));
+    NB_TRY(h->blocksum.alloc(2 * (size_t)h->num_sms));
     if (n <= kPlanRows) {
         // Parts cost at most a sixteenth of an SM's share each beyond one per
         // walk, so there are at most 16 num_sms further ones.
