@@ -724,6 +724,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
     // Changeover: pot_tot and pot_soft partials of neighbour pairs (all other
     // pairs add the same term to both, in a[k][3]).
     float dt[CO ? KI : 1], ds[CO ? KI : 1];
+    unsigned js_inv = 1u << 16;
     double rcut2d = 0.0;
     bool add_self = true, parts = false, further = false;  // further: a part >= 1
     int since = 0;
@@ -844,24 +845,27 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
         return nb;
     };
 
+    // ceil(n / n_js) without a division: exact for n + n_js <= 512, n_js <= 128,
+    // as (n + n_js - 1) times the excess of ceil(2^16 / n_js) stays below 2^16.
+    auto per_slice = [&](int n) -> int { return (int)(((unsigned)(n + n_js - 1) * js_inv) >> 16); };
+    static_assert(TE + CT <= 512 && CT <= 128, "per_slice");
+
     // One EPJ tile with KU i-particles per thread.
     auto ep_tile = [&](auto ku_c, const Hdr& h, int sl) {
         constexpr int KU = decltype(ku_c)::value;
         const auto& T = s.slot[sl].ep;
-        const int pn = (h.nn + n_js - 1) / n_js;
+        const int pn = per_slice(h.nn);
         const int j0 = min(h.nn, js * pn);
         const int j1 = min(h.nn, j0 + pn);
         if (j1 > j0) {
             float4 lo[KU];
             int kb[KU], c[KU];
-            bool vk[KU];
             CoRec ci[CO ? KU : 1];
 #pragma unroll
             for (int k = 0; k < KU; ++k) {
                 lo[k] = s.nlo[k][ct];
                 kb[k] = s.nkb[k][ct];
                 c[k] = 0;
-                vk[k] = slot + k * S < nip;
                 if constexpr (CO) ci[k] = s.co.coi[k][ct];
             }
             (void)ci;
@@ -869,6 +873,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
             for (int j = j0; j < j1; ++j) {
                 const float4 hh = T.nh[j];
                 const float4 ll = T.nl[j];
+                unsigned band = 0;  // i whose pair lies in the guard band (0 ulps where there is no i)
 #pragma unroll
                 for (int k = 0; k < KU; ++k) {
                     const float dx = (hh.x - xi(k)) + (ll.x - lo[k].x);
@@ -880,7 +885,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
                     const float rs2 = fmaxf(lo[k].w, ll.w);
                     const int e = __float_as_int(r2) - __float_as_int(rs2) + kb[k];
                     c[k] += (int)((unsigned)e >> 31);
-                    if ((unsigned)e < (unsigned)(2 * kb[k]) && vk[k]) c[k] += retest(k, h.base + T.nidx[j]);
+                    band |= (unsigned)e < (unsigned)(2 * kb[k]) ? 1u << k : 0u;
                     if constexpr (CO) {
                         const CoRec& cj = T.nco[j];
                         if ((e < 0) && cj.id != ci[k].id) {
@@ -908,6 +913,11 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
                         acc4(k, mri * (ri * ri), dx, dy, dz, mri);
                     }
                 }
+                if (band) {
+#pragma unroll
+                    for (int k = 0; k < KU; ++k)
+                        if (band >> k & 1u) c[k] += retest(k, h.base + T.nidx[j]);
+                }
             }
 #pragma unroll
             for (int k = 0; k < KU; ++k) s.cnt[k][ct] += c[k];
@@ -921,7 +931,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
         } else if constexpr (PK) {
             // far pairs of j, two per FP32x2 instruction
             const int np = (h.nf + 1) >> 1;
-            const int pp = (np + n_js - 1) / n_js;
+            const int pp = per_slice(np);
             const int f0 = min(np, js * pp);
             const int f1 = min(np, f0 + pp);
             const float2 e2 = make_float2(eps2, eps2);
@@ -950,7 +960,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
             }
             nfar = 2 * (f1 - f0);
         } else {
-            const int pf = (h.nf + n_js - 1) / n_js;
+            const int pf = per_slice(h.nf);
             const int f0 = min(h.nf, js * pf);
             const int f1 = min(h.nf, f0 + pf);
 #pragma unroll 4
@@ -984,7 +994,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
         const auto& T = s.slot[sl].sp;
         if constexpr (PK) {
             const int np = (h.nn + 1) >> 1;
-            const int pp = (np + n_js - 1) / n_js;
+            const int pp = per_slice(np);
             const int j0 = min(np, js * pp);
             const int j1 = min(np, j0 + pp);
             const float2 e2 = make_float2(eps2, eps2);
@@ -1029,7 +1039,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
             }
             since += 2 * (j1 - j0);
         } else {
-            const int ps = (h.nn + n_js - 1) / n_js;
+            const int ps = per_slice(h.nn);
             const int j0 = min(h.nn, js * ps);
             const int j1 = min(h.nn, j0 + ps);
 #pragma unroll 2
@@ -1080,6 +1090,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
             }
             S = (nip + ku - 1) / ku;
             n_js = CT / S;
+            js_inv = ((1u << 16) + n_js - 1) / (unsigned)n_js;
             js = ct / S;
             slot = ct - js * S;
             active = js < n_js;
