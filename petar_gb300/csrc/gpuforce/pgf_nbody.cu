@@ -149,6 +149,26 @@ __device__ __forceinline__ int64_t order_key(double x) {
 __device__ __forceinline__ double kmin(double a, double b) { return order_key(b) < order_key(a) ? b : a; }
 __device__ __forceinline__ double kmax(double a, double b) { return order_key(a) < order_key(b) ? b : a; }
 
+// (float)x and the rest x - (float)x as a float, on the integer pipe where both
+// are normal numbers: the same roundings (to nearest, ties to even) as the FP64
+// pipe's conversions and subtraction, at a dozen instructions instead of 64
+// cycles of that pipe each.
+__device__ __forceinline__ float2 split_rn(double x) {
+    const unsigned lo = (unsigned)__double2loint(x), hi = (unsigned)__double2hiint(x);
+    const unsigned e = (hi >> 20) & 0x7ffu, sign = hi & 0x80000000u;
+    if (e - 949u >= 1150u - 949u) {  // 0, too small for either part, too large, infinite, NaN
+        if (!((hi << 1) | lo)) return make_float2(__uint_as_float(sign), 0.f);
+        const float h = (float)x;
+        return make_float2(h, (float)(x - (double)h));
+    }
+    const unsigned m = ((hi & 0xfffffu) << 3) | (lo >> 29), r = lo & 0x1fffffffu;
+    const unsigned up = r + (m & 1u) > 0x10000000u;
+    const float h = __uint_as_float((sign | ((e - 896u) << 23) | m) + up);
+    const float scale = __uint_as_float(sign | ((e - 948u) << 23));
+    return make_float2(h, scale * (float)(int)(r - (up << 29)));
+}
+__device__ __forceinline__ float f32_rn(double x) { return split_rn(x).x; }
+
 __device__ __forceinline__ uint64_t spread3(uint64_t v) {
     v &= 0x1fffff;
     v = (v | (v << 32)) & 0x1f00000000ffffULL;
@@ -348,7 +368,7 @@ __global__ __launch_bounds__(256) void gather_kernel(const int32_t* __restrict__
 // CTA per SM, with a grid barrier between them.  As launches of their own
 // (three per level for 22 levels, and one per level of moments) they took
 // most of a small step: tree and lists 0.77 ms at 3,000 stars, 0.34 ms so (King 1M:
-// 2.92 and 2.44 ms).
+// 2.92 and 2.44 ms then).
 constexpr int kTreeThreads = 512;
 constexpr int kTreeWarps = kTreeThreads / 32;
 
@@ -463,11 +483,25 @@ struct TreeArgs {
     SpjQ64* spjq;
 };
 
+// What the cells of a level share: the opening criterion, and the distance
+// beyond which a cell's centre is surely outside it (before the cell's r_search).
+struct LevelTab {
+    double crit[kLevels];
+    float critf[kLevels], apart[kLevels];
+};
+
+__device__ __forceinline__ void level_tab(const TreeArgs& a, LevelTab& tab, int L) {
+    const double side = ldexp(a.h->side0, -L);
+    const double crit = side * side * a.inv_theta2;
+    tab.crit[L] = crit;
+    tab.critf[L] = (float)crit;
+    tab.apart[L] = 0.5772f * ((float)sqrt(crit) * 0.9999f - 1.7322f * (float)side);
+}
+
 // Moments, boxes and SPJ records of one cell: a leaf from its particles in
 // sorted order, an inner cell from its children in child order.
-__device__ void cell_moments(const TreeArgs& a, int64_t c) {
+__device__ void cell_moments(const TreeArgs& a, const LevelTab& tab, int64_t c) {
     TCell& cc = a.cells[c];
-    const double side = ldexp(a.h->side0, -cc.level);
     double m = 0, mx[3] = {0, 0, 0}, q[6] = {0, 0, 0, 0, 0, 0};
     double ilo[3], ihi[3], olo[3], ohi[3];
     for (int d = 0; d < 3; ++d) {
@@ -541,17 +575,21 @@ __device__ void cell_moments(const TreeArgs& a, int64_t c) {
         cc.out_lo[d] = olo[d];
         cc.out_hi[d] = ohi[d];
     }
-    cc.crit = side * side * a.inv_theta2;
+    cc.crit = tab.crit[cc.level];
     cc.rs_max = __double2float_ru(rsm);
     TCellW w;
+    float ch[3], cl[3];
     for (int d = 0; d < 3; ++d) {
-        w.com[d] = (float)com[d];
-        w.in_lo[d] = (float)ilo[d];
-        w.in_hi[d] = (float)ihi[d];
-        w.out_lo[d] = (float)olo[d];
-        w.out_hi[d] = (float)ohi[d];
+        const float2 c2 = split_rn(com[d]);
+        ch[d] = c2.x;
+        cl[d] = c2.y;
+        w.com[d] = c2.x;
+        w.in_lo[d] = f32_rn(ilo[d]);
+        w.in_hi[d] = f32_rn(ihi[d]);
+        w.out_lo[d] = f32_rn(olo[d]);
+        w.out_hi[d] = f32_rn(ohi[d]);
     }
-    w.crit = (float)cc.crit;
+    w.crit = tab.critf[cc.level];
     w.begin = cc.begin;
     w.end = cc.end;
     w.first_child = cc.first_child;
@@ -559,10 +597,7 @@ __device__ void cell_moments(const TreeArgs& a, int64_t c) {
     w.leaf = cc.leaf;
     w.parent = cc.parent;
     w.level = cc.level;
-    {
-        const float a = 0.5772f * ((float)sqrt(cc.crit) * 0.9999f - 1.7322f * (float)side);
-        w.apart = a > cc.rs_max ? a : 0.f;
-    }
+    w.apart = tab.apart[cc.level] > cc.rs_max ? tab.apart[cc.level] : 0.f;
     a.cw[c] = w;
     CMom& o = a.mom[c];
     o.m = m;
@@ -574,24 +609,24 @@ __device__ void cell_moments(const TreeArgs& a, int64_t c) {
     s.x = com[0];
     s.y = com[1];
     s.z = com[2];
-    s.m = (float)m;
+    s.m = f32_rn(m);
     s.pad0 = 0.f;
-    s.Q[0] = (float)(3.0 * q[0] - tr);
-    s.Q[1] = (float)(3.0 * q[1] - tr);
-    s.Q[2] = (float)(3.0 * q[2] - tr);
-    s.Q[3] = (float)(3.0 * q[3]);
-    s.Q[4] = (float)(3.0 * q[4]);
-    s.Q[5] = (float)(3.0 * q[5]);
-    s.tr = (float)tr;
+    s.Q[0] = f32_rn(3.0 * q[0] - tr);
+    s.Q[1] = f32_rn(3.0 * q[1] - tr);
+    s.Q[2] = f32_rn(3.0 * q[2] - tr);
+    s.Q[3] = f32_rn(3.0 * q[3]);
+    s.Q[4] = f32_rn(3.0 * q[4]);
+    s.Q[5] = f32_rn(3.0 * q[5]);
+    s.tr = f32_rn(tr);
     s.pad1 = 0.f;
     a.spj[c] = s;
     SpjF32 f;
-    f.xh = (float)com[0];
-    f.yh = (float)com[1];
-    f.zh = (float)com[2];
-    f.xl = (float)(com[0] - (double)f.xh);
-    f.yl = (float)(com[1] - (double)f.yh);
-    f.zl = (float)(com[2] - (double)f.zh);
+    f.xh = ch[0];
+    f.yh = ch[1];
+    f.zh = ch[2];
+    f.xl = cl[0];
+    f.yl = cl[1];
+    f.zl = cl[2];
     f.m = s.m;
     f.tr = s.tr;
     for (int k = 0; k < 6; ++k) f.Q[k] = s.Q[k];
@@ -609,7 +644,7 @@ __device__ void cell_moments(const TreeArgs& a, int64_t c) {
 // terms, and a lane per component adds them in the order of cell_moments, so
 // the results are the same.  Where cells are few, this is the latency of tens
 // of FP64 instructions instead of hundreds (64 cycles each).
-__device__ void cell_moments8(const TreeArgs& a, int64_t c, bool act, double (*__restrict__ buf)[8]) {
+__device__ void cell_moments8(const TreeArgs& a, const LevelTab& tab, int64_t c, bool act, double (*__restrict__ buf)[8]) {
     constexpr unsigned kAll = 0xffffffffu;
     const int k = threadIdx.x & 7;
     const int src = threadIdx.x & 24;  // first lane of the group
@@ -729,31 +764,29 @@ __device__ void cell_moments8(const TreeArgs& a, int64_t c, bool act, double (*_
         cell.in_hi[k] = v[1];
         cell.out_lo[k] = v[2];
         cell.out_hi[k] = v[3];
-        const float ch = (float)cx;
-        w.com[k] = ch;
-        w.in_lo[k] = (float)v[0];
-        w.in_hi[k] = (float)v[1];
-        w.out_lo[k] = (float)v[2];
-        w.out_hi[k] = (float)v[3];
+        const float2 ch = split_rn(cx);
+        w.com[k] = ch.x;
+        w.in_lo[k] = f32_rn(v[0]);
+        w.in_hi[k] = f32_rn(v[1]);
+        w.out_lo[k] = f32_rn(v[2]);
+        w.out_hi[k] = f32_rn(v[3]);
         a.mom[c].mx[k] = mxd;
         (&a.spj[c].x)[k] = cx;
-        (&a.spj32[c].xh)[k] = ch;
-        (&a.spj32[c].xl)[k] = (float)(cx - (double)ch);
+        (&a.spj32[c].xh)[k] = ch.x;
+        (&a.spj32[c].xl)[k] = ch.y;
     }
     if (k < 6) {
         a.mom[c].q[k] = q;
         a.spjq[c].q[k] = q;
-        const float f = k < 3 ? (float)(3.0 * q - tr) : (float)(3.0 * q);
+        const float f = f32_rn(k < 3 ? 3.0 * q - tr : 3.0 * q);
         a.spj[c].Q[k] = f;
         a.spj32[c].Q[k] = f;
     } else if (k == 6) {
-        const double side = ldexp(a.h->side0, -cell.level);
-        const double crit = side * side * a.inv_theta2;
         const float rs = __double2float_ru(rsm);
-        cell.crit = crit;
+        const float ap = tab.apart[cell.level];
+        cell.crit = tab.crit[cell.level];
         cell.rs_max = rs;
-        w.crit = (float)crit;
-        const float ap = 0.5772f * ((float)sqrt(crit) * 0.9999f - 1.7322f * (float)side);
+        w.crit = tab.critf[cell.level];
         w.apart = ap > rs ? ap : 0.f;
         w.begin = cell.begin;
         w.end = cell.end;
@@ -763,7 +796,7 @@ __device__ void cell_moments8(const TreeArgs& a, int64_t c, bool act, double (*_
         w.parent = cell.parent;
         w.level = cell.level;
     } else {
-        const float mf = (float)m, tf = (float)tr;
+        const float mf = f32_rn(m), tf = f32_rn(tr);
         a.mom[c].m = m;
         a.spj[c].m = mf;
         a.spj[c].pad0 = 0.f;
@@ -777,29 +810,38 @@ __device__ void cell_moments8(const TreeArgs& a, int64_t c, bool act, double (*_
     }
 }
 
-// Cells [lo, hi) of the class order.
-__device__ __forceinline__ void moments_range(const TreeArgs& a, int lo, int hi, double (*buf)[8]) {
+// Cells [lo, hi) of the class order, dealt to the CTAs a warp's share at a time:
+// the FP64 pipes of all SMs get the same number of shares, give or take one.
+// Dealt to the CTAs whole, the last shares fell to a few SMs; with that and the
+// conversions off the FP64 pipe the tree kernel went from 530 to 405 us at King
+// 1M, 367 to 242 at 262,144, 222 to 161 at 30,000 and 132 to 116 at 3,000.
+__device__ __forceinline__ void moments_range(const TreeArgs& a, const LevelTab& tab, int lo, int hi,
+                                              double (*buf)[8]) {
     const int64_t threads = (int64_t)gridDim.x * kTreeThreads;
+    const int64_t w = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    const int lane = threadIdx.x & 31;
     if ((int64_t)(hi - lo) * 8 <= threads) {
         // a group of eight lanes per cell, one round
-        const int64_t base = lo + (((int64_t)blockIdx.x * kTreeThreads + (threadIdx.x & ~31)) >> 3);
+        const int64_t base = lo + 4 * w;
         if (base >= hi) return;  // whole warps
-        const int64_t t = base + ((threadIdx.x & 31) >> 3);
-        cell_moments8(a, t < hi ? a.order[t] : 0, t < hi, buf);
+        const int64_t t = base + (lane >> 3);
+        cell_moments8(a, tab, t < hi ? a.order[t] : 0, t < hi, buf);
         return;
     }
-    for (int64_t t = lo + gtid(); t < hi; t += threads) cell_moments(a, a.order[t]);
+    for (int64_t t = lo + 32 * w + lane; t < hi; t += threads) cell_moments(a, tab, a.order[t]);
 }
 
 __global__ __launch_bounds__(kTreeThreads, 1) void tree_kernel(TreeArgs a) {
     __shared__ double s_buf[kTreeWarps][4][6][8];
     __shared__ int s_hist[kCellBins + 1], s_base[kCellBins];
     __shared__ int s_b[9], s_before, s_total, s_sum;
+    __shared__ LevelTab s_tab;
     TreeHdr* const h = a.h;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int G = gridDim.x, bid = blockIdx.x;
     unsigned epoch = 0;
     if (h->err) return;  // before the first barrier: every CTA sees it
+    if (t < kLevels) level_tab(a, s_tab, t);  // read after the barriers below
     // ---- levels: children of a level in their parents' order ----
     int lb = 0, le = 1, depth = 0;
     for (int L = 0; L < kLevels; ++L) {
@@ -961,12 +1003,12 @@ __global__ __launch_bounds__(kTreeThreads, 1) void tree_kernel(TreeArgs a) {
     if (!grid_sync(&h->bar, epoch, &h->err)) return;
     // ---- moments: leaves, then the inner cells from the deepest level up ----
     double (*const buf)[8] = s_buf[warp][lane >> 3];
-    moments_range(a, 0, s_hist[kLeafBins], buf);
+    moments_range(a, s_tab, 0, s_hist[kLeafBins], buf);
     for (int L = depth; L >= 0; --L) {
         const int lo = s_hist[kLeafBins + 8 * L], hi = s_hist[kLeafBins + 8 * L + 8];
         if (lo == hi) continue;  // every CTA
         if (!grid_sync(&h->bar, epoch, &h->err)) return;
-        moments_range(a, lo, hi, buf);
+        moments_range(a, s_tab, lo, hi, buf);
     }
 }
 
