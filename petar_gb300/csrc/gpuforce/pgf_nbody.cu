@@ -97,6 +97,8 @@ struct TreeHdr {
     int32_t sample_slot;  // next record slot of the per-step sample
     unsigned bar;  // arrivals at the tree kernel's grid barriers
     unsigned long long walk_cursor[2];  // next task of the count and fill passes
+    unsigned long long top_cursor;      // next run of the top pass
+    int32_t n_tasks[2];                 // queued tasks: near ones, others
 };
 
 // Cell fields the walk reads.
@@ -1278,21 +1280,37 @@ constexpr int kWalkWarps = 4;  // per CTA
 
 __device__ __forceinline__ int64_t n_chunks(const TreeHdr* h) { return (h->n_fronts + kChunk - 1) / kChunk; }
 
+// Task slots of a build: the groups in whole blocks of 32.
+__host__ __device__ __forceinline__ int64_t task_slots(int64_t n_groups, int64_t n_fronts) {
+    return (n_groups + 31) / 32 * 32 * ((n_fronts + kChunk - 1) / kChunk);
+}
+
 __global__ void task_check_kernel(TreeHdr* h, int64_t cap_tasks) {
     if (threadIdx.x != 0) return;
-    h->walk_cursor[0] = h->walk_cursor[1] = 0;
+    h->walk_cursor[0] = h->walk_cursor[1] = h->top_cursor = 0;
+    h->n_tasks[0] = h->n_tasks[1] = 0;
     if (h->err) return;
-    if ((int64_t)h->n_groups * n_chunks(h) > cap_tasks) h->err |= kErrTasks;
+    if (task_slots(h->n_groups, h->n_fronts) > cap_tasks) h->err |= kErrTasks;
 }
 
 // A task is (chunk q of frontier cells, block b of 32 groups), walked by one
 // warp, a lane per group: its threads walk the same subtrees for neighbouring
 // groups.  Warps take tasks from a counter, as their costs differ by orders of
-// magnitude: a chunk next to the groups against one whose ancestors they
-// close.  The tasks of every block run outwards from the chunk that holds its
-// own particles, so the expensive ones come first and the launch ends on
-// cheap ones (King 1M: tree and lists 3.36 -> 2.92 ms with this order and
-// the early exit in open_cell).
+// magnitude.
+//
+// Builds of fewer than kTopRows particles walk all chunk and block pairs, those
+// of every block outwards from the chunk that holds its own particles, so the
+// expensive ones come first and the launch ends on cheap ones.  In larger ones
+// most pairs are far apart: the block's groups close an ancestor of the
+// frontier cells, which gives one list entry or none, at the price of testing
+// the ancestors again for every frontier cell below.  There a pass over the
+// cells down to the frontier (top_run) settles all chunks without a cell that
+// some group opens, jumping over what closed cells cover, and queues the
+// others as tasks.  That leaves room for smaller frontier cells
+// (front_limit_of), so that no task outlasts the launch.  Tree and lists
+// without and with it: 131,072 particles 0.71 and 0.70 ms, 200,000 0.80 and
+// 0.77, 524,288 1.66 and 1.29, 1M 2.75 and 1.98 (2.31 without it at n / 512
+// particles per frontier cell).
 __device__ __forceinline__ int64_t next_task(unsigned long long* cursor) {
     unsigned long long t = 0;
     if ((threadIdx.x & 31) == 0) t = atomicAdd(cursor, 1ull);
@@ -1315,49 +1333,182 @@ __device__ __forceinline__ int front_of(const TCellW* __restrict__ cw, const int
     return lo;
 }
 
+constexpr int64_t kTopRows = 131072;
+constexpr int64_t kTopRuns = 16384;  // runs of the top pass, about
+
+struct WalkArgs {
+    TreeHdr* h;
+    int32_t* task_e;
+    int32_t* task_s;
+    int32_t* tasks;  // the queue: near tasks from the front, others from the end
+    int64_t cap_queue;
+    int32_t* id_epj;
+    int32_t* id_spj;
+    bool open_all;
+};
+
+// Chunks of a run of the top pass, and the runs per block.
+__device__ __forceinline__ int64_t top_run_len(int64_t nb, int64_t nq) {
+    const int64_t k = nb * nq / kTopRuns;
+    return k < 1 ? 1 : (k > 64 ? 64 : k);
+}
+
+// Run `unit` of the top pass: block unit % nb, chunks of run unit / nb.
 template <bool FILL>
-__device__ __forceinline__ void walk_tasks(TreeHdr* h, const TCellW* __restrict__ cw, const TCell* __restrict__ cells,
-                                           const int32_t* __restrict__ groups, const int32_t* __restrict__ fronts,
-                                           const WalkDesc* __restrict__ walks, int32_t* task_e, int32_t* task_s,
-                                           int32_t* id_epj, int32_t* id_spj, bool open_all) {
+__device__ void top_run(const WalkArgs& a, const TCellW* __restrict__ cw, const TCell* __restrict__ cells, const int32_t* __restrict__ groups,
+                        const int32_t* __restrict__ fronts, const WalkDesc* __restrict__ walks,
+                        int64_t unit, int64_t ng, int64_t nb, int64_t nf, int64_t nq) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int64_t len = top_run_len(nb, nq), r = unit / nb, b = unit - r * nb;
+    const int64_t q1 = min(nq, (r + 1) * len);
+    const int64_t g = b * 32 + lane;
+    const bool valid = g < ng;
+    int own = 0;
+    if (!FILL) own = front_of(cw, fronts, (int)nf, cw[groups[min(ng - 1, b * 32 + 16)]].begin) / kChunk;
+    WalkCtx x;
+    load_ctx(x, cw, cells, groups[valid ? g : ng - 1], a.h->xmax, a.open_all);
+    int cache_c[kLevels];  // opened ancestors of the current chain
+    int n_cached = 0;
+    int closed_end = valid ? 0 : 0x7fffffff;  // rows before this one lie in cells already listed
+    for (int64_t q = r * len; q < q1;) {
+        const int least = __reduce_min_sync(kAll, closed_end);
+        if (cw[fronts[q * kChunk]].begin < least) {
+            // closed for every lane, up to the frontier cell that begins at `least`
+            int64_t to = q1;
+            const int last = fronts[min(nf, q1 * kChunk) - 1];
+            if (least < cw[last].end) to = front_of(cw, fronts, (int)nf, least) / kChunk;
+            if (!FILL && valid)
+                for (int64_t k = q; k < to; ++k) a.task_e[k * ng + g] = a.task_s[k * ng + g] = 0;
+            if (to > q) {
+                q = to;
+                continue;
+            }
+        }
+        int found[kChunk], n = 0;
+        bool opened = false;
+        for (int64_t fi = q * kChunk; fi < min(nf, (q + 1) * kChunk); ++fi) {
+            const int f = fronts[fi];
+            const TCellW fw = cw[f];
+            if (fw.begin < closed_end) continue;
+            // climb to the deepest opened ancestor known; the others are new
+            int fresh[kLevels], nfr = 0;
+            int c = fw.parent, lvl = fw.level - 1;
+            while (c >= 0 && !(lvl < n_cached && cache_c[lvl] == c)) {
+                fresh[nfr++] = c;
+                c = cw[c].parent;
+                --lvl;
+            }
+            n_cached = lvl + 1;
+            int closed = -1;
+            for (int k = nfr - 1; k >= 0 && closed < 0; --k) {  // root side first
+                if (open_cell(x, fresh[k], cw[fresh[k]])) cache_c[n_cached++] = fresh[k];
+                else closed = fresh[k];
+            }
+            if (closed < 0) {
+                if (open_cell(x, f, fw)) {
+                    opened = true;
+                    continue;
+                }
+                closed = f;
+            }
+            const TCellW w = cw[closed];
+            closed_end = w.end;
+            // listed by the frontier cell that starts its range
+            if (w.begin == fw.begin) found[n++] = closed;
+        }
+        if (__any_sync(kAll, opened)) {
+            if (!FILL && lane == 0) {
+                const int64_t d = q < own ? own - q : q - own;
+                const int32_t t = (int32_t)(q * nb + b);
+                if (d <= 8) a.tasks[atomicAdd(&a.h->n_tasks[0], 1)] = t;
+                else a.tasks[a.cap_queue - 1 - atomicAdd(&a.h->n_tasks[1], 1)] = t;
+            }
+        } else if (valid) {
+            const int64_t slot = q * ng + g;
+            if (!FILL) {
+                a.task_e[slot] = 0;
+                a.task_s[slot] = n;
+            } else if (n > 0) {
+                int32_t* const os = a.id_spj + walks[g].spj_begin + a.task_s[slot];
+#pragma unroll
+                for (int k = 0; k < kChunk; ++k)
+                    if (k < n) os[k] = found[k];
+            }
+        }
+        ++q;
+    }
+}
+
+template <bool FILL, bool TOP>
+__device__ __forceinline__ void walk_tasks(const WalkArgs& a, const TCellW* __restrict__ cw, const TCell* __restrict__ cells, const int32_t* __restrict__ groups,
+                                           const int32_t* __restrict__ fronts, const WalkDesc* __restrict__ walks) {
+    TreeHdr* const h = a.h;
     if (h->err) return;
     const int lane = threadIdx.x & 31;
-    const int64_t ng = h->n_groups, nf = h->n_fronts, nb = (ng + 31) / 32, T = nb * n_chunks(h);
+    const int64_t ng = h->n_groups, nf = h->n_fronts, nb = (ng + 31) / 32, nq = n_chunks(h);
     const float X = h->xmax;
+    const int64_t near = TOP ? h->n_tasks[0] : 0, queued = TOP ? near + h->n_tasks[1] : 0;
+    int64_t T = nb * nq;
+    if (TOP) {
+        const int64_t len = top_run_len(nb, nq), runs = (nq + len - 1) / len * nb;
+        T = queued + (FILL ? runs : 0);
+    }
     for (;;) {
         const int64_t t = next_task(&h->walk_cursor[FILL ? 1 : 0]);
         if (t >= T) break;
-        const int64_t nq = n_chunks(h);
-        const int o = (int)(t / nb), b = (int)(t - (int64_t)o * nb);
+        int q, b;
+        if (!TOP) {
+            const int o = (int)(t / nb);
+            b = (int)(t - (int64_t)o * nb);
+            const int mid = groups[min((int)ng - 1, b * 32 + 16)];
+            // own chunk, then 1 after, 1 before, 2 after, ... (wrapping around)
+            const int own = front_of(cw, fronts, (int)nf, cw[mid].begin) / kChunk;
+            q = (int)((own + ((o & 1) ? (o + 1) / 2 : -(o / 2))) % nq);
+            if (q < 0) q += (int)nq;
+        } else {
+            if (t >= queued) {
+                if (FILL) top_run<true>(a, cw, cells, groups, fronts, walks, t - queued, ng, nb, nf, nq);
+                continue;
+            }
+            const int64_t e = a.tasks[t < near ? t : a.cap_queue - 1 - (t - near)];
+            q = (int)(e / nb);
+            b = (int)(e - (int64_t)q * nb);
+        }
         const int g = b * 32 + lane;
         const bool valid = g < ng;
-        const int mid = groups[min((int)ng - 1, b * 32 + 16)];
-        // own chunk, then 1 after, 1 before, 2 after, ... (wrapping around)
-        const int own = front_of(cw, fronts, (int)nf, cw[mid].begin) / kChunk;
-        int q = (int)((own + ((o & 1) ? (o + 1) / 2 : -(o / 2))) % nq);
-        if (q < 0) q += (int)nq;
         WalkCtx x;
-        load_ctx(x, cw, cells, groups[valid ? g : (int)ng - 1], X, open_all);
+        load_ctx(x, cw, cells, groups[valid ? g : (int)ng - 1], X, a.open_all);
         const int64_t slot = (int64_t)q * ng + g;
         if (!valid) continue;
         int ne, ns;
         walk_chunk<FILL>(x, fronts, q * kChunk, (int)min(nf, (int64_t)(q + 1) * kChunk), ne, ns,
-                         FILL ? id_epj + walks[g].epj_begin + task_e[slot] : nullptr,
-                         FILL ? id_spj + walks[g].spj_begin + task_s[slot] : nullptr);
+                         FILL ? a.id_epj + walks[g].epj_begin + a.task_e[slot] : nullptr,
+                         FILL ? a.id_spj + walks[g].spj_begin + a.task_s[slot] : nullptr);
         if (!FILL) {
-            task_e[slot] = ne;
-            task_s[slot] = ns;
+            a.task_e[slot] = ne;
+            a.task_s[slot] = ns;
         }
     }
 }
 
+__global__ __launch_bounds__(kWalkWarps * 32) void walk_top_kernel(WalkArgs a, const TCellW* __restrict__ cw, const TCell* __restrict__ cells, const int32_t* __restrict__ groups,
+    const int32_t* __restrict__ fronts, const WalkDesc* __restrict__ walks) {
+    if (a.h->err) return;
+    const int64_t ng = a.h->n_groups, nf = a.h->n_fronts, nb = (ng + 31) / 32, nq = n_chunks(a.h);
+    const int64_t len = top_run_len(nb, nq), runs = (nq + len - 1) / len * nb;
+    for (;;) {
+        const int64_t u = next_task(&a.h->top_cursor);
+        if (u >= runs) break;
+        top_run<false>(a, cw, cells, groups, fronts, walks, u, ng, nb, nf, nq);
+    }
+}
+
 // Counts of every (chunk, group), stored at q * n_groups + g.
-__global__ __launch_bounds__(kWalkWarps * 32) void walk_task_count_kernel(TreeHdr* h, const TCellW* __restrict__ cw,
-                                                                          const TCell* __restrict__ cells,
-                                                                          const int32_t* __restrict__ groups,
-                                                                          const int32_t* __restrict__ fronts,
-                                                                          int32_t* task_e, int32_t* task_s, bool open_all) {
-    walk_tasks<false>(h, cw, cells, groups, fronts, nullptr, task_e, task_s, nullptr, nullptr, open_all);
+template <bool TOP>
+__global__ __launch_bounds__(kWalkWarps * 32) void walk_task_count_kernel(WalkArgs a, const TCellW* __restrict__ cw, const TCell* __restrict__ cells, const int32_t* __restrict__ groups,
+    const int32_t* __restrict__ fronts, const WalkDesc* __restrict__ walks) {
+    walk_tasks<false, TOP>(a, cw, cells, groups, fronts, walks);
 }
 
 // Per group: offsets of its tasks within its lists (in frontier order), the
@@ -1458,14 +1609,10 @@ __global__ __launch_bounds__(kScanThreads) void walk_scan_kernel(TreeHdr* h, Wal
     }
 }
 
-__global__ __launch_bounds__(kWalkWarps * 32) void walk_task_fill_kernel(TreeHdr* h, const TCellW* __restrict__ cw,
-                                                                         const TCell* __restrict__ cells,
-                                                                         const int32_t* __restrict__ groups,
-                                                                         const int32_t* __restrict__ fronts,
-                                                                         const WalkDesc* __restrict__ walks,
-                                                                         int32_t* task_e, int32_t* task_s,
-                                                                         int32_t* id_epj, int32_t* id_spj, bool open_all) {
-    walk_tasks<true>(h, cw, cells, groups, fronts, walks, task_e, task_s, id_epj, id_spj, open_all);
+template <bool TOP>
+__global__ __launch_bounds__(kWalkWarps * 32) void walk_task_fill_kernel(WalkArgs a, const TCellW* __restrict__ cw, const TCell* __restrict__ cells, const int32_t* __restrict__ groups,
+    const int32_t* __restrict__ fronts, const WalkDesc* __restrict__ walks) {
+    walk_tasks<true, TOP>(a, cw, cells, groups, fronts, walks);
 }
 
 // Work queue: walks by descending cost bucket (ties in no fixed order; the
@@ -1779,6 +1926,7 @@ struct pgf_nbody {
     int front_limit = 1;              // frontier: topmost cells with at most this many particles
     int64_t cap_tasks = 0;
     DArr<int32_t> task_e, task_s;     // per (frontier, group) counts, then offsets
+    DArr<int32_t> tasks;              // queued (frontier, block) pairs
     DArr<WalkDesc> walks;
     int64_t cap_e = 0, cap_s = 0;
     DArr<int32_t> id_epj, id_spj;
@@ -1823,8 +1971,11 @@ namespace {
 
 // Largest frontier cell: about a thousand frontier cells from 32,768 particles
 // on, cells of 64 below (3,000 stars: tree and lists 0.88 ms with cells of a
-// group's 512, 0.77 ms with 64).
-int front_limit_of(int64_t n) { return (int)std::max<int64_t>(64, n / 512); }
+// group's 512, 0.77 ms with 64); half that from 524,288 on, where the top pass
+// makes frontier cells cheap (1M: 2.14 ms with n / 512, 1.98 with n / 1024).
+int front_limit_of(int64_t n) {
+    return (int)std::max<int64_t>(64, std::min<int64_t>(n / 512, std::max<int64_t>(512, n / 1024)));
+}
 
 int grid_for(const pgf_nbody* h, int64_t work, int threads) {
     int64_t b = (work + threads - 1) / threads;
@@ -1879,14 +2030,16 @@ cudaError_t enqueue_build(pgf_nbody* h) {
     if ((e = cub_select(h, h->cub_tmp.d, bytes, h->front_at.d, h->fronts.d, &hd->n_fronts)) != cudaSuccess) return e;
     task_check_kernel<<<1, 32, 0, s>>>(hd, h->cap_tasks);
     const int gt = h->num_sms * 16;
-    walk_task_count_kernel<<<gt, kWalkWarps * 32, 0, s>>>(hd, h->cw.d, h->cells.d, h->groups.d, h->fronts.d, h->task_e.d,
-                                              h->task_s.d, h->open_all);
+    const WalkArgs wa{hd, h->task_e.d, h->task_s.d, h->tasks.d, h->cap_tasks / 32, h->id_epj.d, h->id_spj.d, h->open_all};
+    const bool top = n >= kTopRows;
+    if (top)
+        walk_top_kernel<<<gt, kWalkWarps * 32, 0, s>>>(wa, h->cw.d, h->cells.d, h->groups.d, h->fronts.d, h->walks.d);
+    (top ? walk_task_count_kernel<true> : walk_task_count_kernel<false>)<<<gt, kWalkWarps * 32, 0, s>>>(wa, h->cw.d, h->cells.d, h->groups.d, h->fronts.d, h->walks.d);
     group_reduce_kernel<<<grid_for(h, n, 128), 128, 0, s>>>(hd, h->cells.d, h->groups.d, h->walks.d, h->task_e.d,
                                                             h->task_s.d, h->cnt_e.d, h->cnt_s.d, h->bucket.d,
                                                             h->cfg.r_out * h->cfg.r_out);
     walk_scan_kernel<<<1, kScanThreads, 0, s>>>(hd, h->walks.d, h->cnt_e.d, h->cnt_s.d, h->cap_e, h->cap_s);
-    walk_task_fill_kernel<<<gt, kWalkWarps * 32, 0, s>>>(hd, h->cw.d, h->cells.d, h->groups.d, h->fronts.d, h->walks.d,
-                                             h->task_e.d, h->task_s.d, h->id_epj.d, h->id_spj.d, h->open_all);
+    (top ? walk_task_fill_kernel<true> : walk_task_fill_kernel<false>)<<<gt, kWalkWarps * 32, 0, s>>>(wa, h->cw.d, h->cells.d, h->groups.d, h->fronts.d, h->walks.d);
     queue_scatter_kernel<<<grid_for(h, n, 256), 256, 0, s>>>(hd, h->bucket.d, h->queue.d);
     return cudaGetLastError();
 }
@@ -2032,6 +2185,7 @@ cudaError_t alloc_tasks(pgf_nbody* h, int64_t cap) {
     h->cap_tasks = cap;
     cudaError_t e = h->task_e.alloc(cap);
     if (e == cudaSuccess) e = h->task_s.alloc(cap);
+    if (e == cudaSuccess) e = h->tasks.alloc(cap / 32);
     return e;
 }
 
@@ -2080,7 +2234,7 @@ int build_fit(pgf_nbody* h) {
                 NB_CUDA(alloc_spj(h));
                 resized = true;
             }
-            const double tt = f * (double)t.n_groups * (double)((t.n_fronts + kChunk - 1) / kChunk) + 1024;
+            const double tt = f * (double)task_slots(t.n_groups, t.n_fronts) + 1024;
             if (off((double)h->cap_tasks, tt)) {
                 NB_CUDA(alloc_tasks(h, (int64_t)std::ceil(tt)));
                 resized = true;
@@ -2106,7 +2260,7 @@ int build_fit(pgf_nbody* h) {
             NB_CUDA(alloc_spj(h));
         }
         if (t.err & kErrTasks)
-            NB_CUDA(alloc_tasks(h, (int64_t)(f * (double)t.n_groups * (double)((t.n_fronts + kChunk - 1) / kChunk)) + 1024));
+            NB_CUDA(alloc_tasks(h, (int64_t)(f * (double)task_slots(t.n_groups, t.n_fronts)) + 1024));
         drop_graph(h);
         bind_params(h);
     }
