@@ -281,7 +281,7 @@ __global__ __launch_bounds__(W * 32, W == 4 ? 3 : 1) void far_kernel(Params p) {
         }
         if (n_far == 0) continue;
 
-        // Sum over the threads: rows 0 and 1 in FP64, the others by a
+        // Sum over the threads: rows 0 and 1 as (hi, lo) pairs, the others by a
         // reduce-scatter (lane l ends with three coefficients).
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -348,7 +348,8 @@ __global__ __launch_bounds__(W * 32, W == 4 ? 3 : 1) void far_kernel(Params p) {
     }
 }
 
-// EPI rows about their walk's centre, one warp per walk.
+// EPI rows about their walk's centre, one warp per walk (conversions on the
+// integer pipe: 58 -> 24 us for 1M rows).
 __global__ __launch_bounds__(256) void epi_rel_kernel(Params p, EpiRel* __restrict__ out, AccF32* __restrict__ out_acc) {
     const int n_walk = p.n_root < p.n_walk ? p.n_root : walk_count(p);
     const int lane = threadIdx.x & 31;

@@ -1,16 +1,16 @@
 // Warp-specialised mixed-precision soft-force kernel for sm_103a.
 //
 // Same pair arithmetic, precision scheme and outputs as mixed_kernel
-// (pgf_kernels_mixed.cu): walk-relative coordinates formed in FP64 and rounded
-// to FP32, near EPJ with hi/lo coordinates, the linear cutoff and the exact
-// neighbour count, far EPJ as plain gravity, EP-SP with the traceless
-// quadrupole, FP32 partial sums flushed into FP64.  The difference is the
-// data flow inside a CTA:
+// (pgf_kernels_mixed.cu): walk-relative coordinates in FP32, near EPJ with
+// hi/lo coordinates, the linear cutoff and the exact neighbour count, far EPJ
+// as plain gravity, EP-SP with the traceless quadrupole, FP32 partial sums
+// flushed into wider accumulators.  The difference is the data flow inside a
+// CTA:
 //
 // * One producer warp walks the work queue.  For every walk pass it emits a
 //   PASS_BEGIN item, then one item per j tile, then PASS_END.  For a tile it
-//   gathers the EPJ/SPJ records through the id list (L2-resident), forms x - c
-//   in FP64, classifies near/far, compacts with warp ballots and writes the
+//   gathers the EPJ/SPJ records through the id list (L2-resident), forms
+//   x - c, classifies near/far, compacts with warp ballots and writes the
 //   FP32 tile into a slot of a shared-memory ring.
 // * CW consumer warps take the items in order.  They never stage data and
 //   never wait for each other inside a pass: each waits only for the slot it
@@ -27,6 +27,12 @@
 //   j-slices are combined as (hi, lo) pairs once per pass, and the i set up
 //   from EpiRel rows, so that a pass issues FP64 only to write its results
 //   (parts of split walks: not even there).
+// * Bound by the FMA pipe (73% of its cycles at King 1M, consumers waiting 6% of
+//   theirs) and, at three consumer warps per SMSP, by latency.  Without FP64 in
+//   the passes: 65,536 stars 0.784 -> 0.607 ms, 20,000 binary stars 0.486 ->
+//   0.282; with the slices' divisions and the re-test's branch out of the tiles
+//   and the final sums on all threads 0.585 and 0.252 ms; 1M binaries, with the
+//   far-field pass before it, 14.67 -> 14.27 ms in all.
 // * Ambiguous neighbour pairs (within the guard band of r_search; a few per
 //   evaluation) are tested exactly in FP64 where they are met.
 // * Every mbarrier wait is bounded by 1 s of %globaltimer; on expiry the thread
@@ -41,7 +47,7 @@ namespace {
 // Ring geometry is a template parameter of each variant: TE EPJ entries per
 // EP tile (TE / 32 per producer lane), TE SPJ entries per SP tile (TE / 2
 // with TMA staging), NS ring slots.
-constexpr int kFlush = 256;   // pairs per consumer thread between FP64 flushes
+constexpr int kFlush = 256;   // pairs per consumer thread between flushes
 constexpr unsigned long long kWaitLimitNs = 1000000000ull;
 constexpr int kErrWaitTimeout = 1;
 

@@ -151,26 +151,6 @@ __device__ __forceinline__ int64_t order_key(double x) {
 __device__ __forceinline__ double kmin(double a, double b) { return order_key(b) < order_key(a) ? b : a; }
 __device__ __forceinline__ double kmax(double a, double b) { return order_key(a) < order_key(b) ? b : a; }
 
-// (float)x and the rest x - (float)x as a float, on the integer pipe where both
-// are normal numbers: the same roundings (to nearest, ties to even) as the FP64
-// pipe's conversions and subtraction, at a dozen instructions instead of 64
-// cycles of that pipe each.
-__device__ __forceinline__ float2 split_rn(double x) {
-    const unsigned lo = (unsigned)__double2loint(x), hi = (unsigned)__double2hiint(x);
-    const unsigned e = (hi >> 20) & 0x7ffu, sign = hi & 0x80000000u;
-    if (e - 949u >= 1150u - 949u) {  // 0, too small for either part, too large, infinite, NaN
-        if (!((hi << 1) | lo)) return make_float2(__uint_as_float(sign), 0.f);
-        const float h = (float)x;
-        return make_float2(h, (float)(x - (double)h));
-    }
-    const unsigned m = ((hi & 0xfffffu) << 3) | (lo >> 29), r = lo & 0x1fffffffu;
-    const unsigned up = r + (m & 1u) > 0x10000000u;
-    const float h = __uint_as_float((sign | ((e - 896u) << 23) | m) + up);
-    const float scale = __uint_as_float(sign | ((e - 948u) << 23));
-    return make_float2(h, scale * (float)(int)(r - (up << 29)));
-}
-__device__ __forceinline__ float f32_rn(double x) { return split_rn(x).x; }
-
 __device__ __forceinline__ uint64_t spread3(uint64_t v) {
     v &= 0x1fffff;
     v = (v | (v << 32)) & 0x1f00000000ffffULL;
@@ -346,20 +326,12 @@ __global__ __launch_bounds__(256) void gather_kernel(const int32_t* __restrict__
         const double x = pos[3 * o], y = pos[3 * o + 1], z = pos[3 * o + 2];
         const double m = mass[o], r = rs[o];
         epi[s] = EpiDev{x, y, z, r};
-        const EpjMix e{x, y, z, (float)m, (float)(r * r)};
+        const EpjMix e{x, y, z, f32_rn(m), f32_rn(r * r)};
         epj[s] = e;
         m64[s] = m;
         rs64[s] = r;
-        EpjF32 f;
-        f.xh = (float)x;
-        f.yh = (float)y;
-        f.zh = (float)z;
-        f.xl = (float)(x - (double)f.xh);
-        f.yl = (float)(y - (double)f.yh);
-        f.zl = (float)(z - (double)f.zh);
-        f.m = e.m;
-        f.rs2 = e.rs2;
-        epj32[s] = f;
+        const float2 fx = split_rn(x), fy = split_rn(y), fz = split_rn(z);
+        epj32[s] = EpjF32{fx.x, fy.x, fz.x, e.m, fx.y, fy.y, fz.y, e.rs2};
     }
 }
 
