@@ -37,8 +37,10 @@ struct Smem64 {
     int w;
 };
 
-// 1/sqrt(a) for normal a.
+// 1/sqrt(a).  The step from the estimate is for normal a; r^2 that underflowed
+// or overflowed (a source 1e154 away: 1/r is 0) takes the library's function.
 __device__ __forceinline__ double rsqrt_fp64(double a) {
+    if ((((unsigned)__double2hiint(a) >> 20) - 1u) >= 0x7feu) return rsqrt(a);
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
     const double e = fma(-(a * y), y, 1.0);
