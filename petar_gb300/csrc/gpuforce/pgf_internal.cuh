@@ -171,25 +171,6 @@ __device__ __forceinline__ EpiRel make_epi_rel(const EpiDev& e, double cx, doubl
     return r;
 }
 
-// An FP64 value as FP32 (hi, lo) without the FP64 pipe: hi the leading 24 bits,
-// lo the other 29 rounded to 24 (hi + lo to 2^-48 of it).  Values below 2^-74
-// lose lo, values below 2^-126 are 0, those beyond FP32's range infinite.
-__device__ __forceinline__ void split_f64(unsigned blo, unsigned bhi, float& h, float& l) {
-    const int e = (int)((bhi >> 20) & 0x7ffu);
-    const unsigned sign = bhi & 0x80000000u;
-    const unsigned m23 = ((bhi & 0xfffffu) << 3) | (blo >> 29);
-    unsigned hb = sign | ((unsigned)(e - 896) << 23) | m23;
-    float scale = __uint_as_float(sign | ((unsigned)(e - 948) << 23));
-    if (e < 949) scale = 0.f;
-    if (e < 897) hb = sign;
-    if (e > 1150) {  // infinities and NaN included
-        hb = sign | 0x7f800000u | ((e == 0x7ff && (m23 | blo)) ? 0x400000u : 0u);
-        scale = 0.f;
-    }
-    h = __uint_as_float(hb);
-    l = scale * (float)(blo & 0x1fffffffu);
-}
-
 // Error-free sum: s + e == a + b exactly (round-to-nearest, no reassociation).
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
     s = a + b;

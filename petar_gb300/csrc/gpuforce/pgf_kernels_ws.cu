@@ -298,45 +298,47 @@ __device__ __forceinline__ void co_k_f32(float r, float r_in, float norm, float 
     }
 }
 
-// FP64 records in the forms of EpjF32 and SpjF32 (split on the integer pipe).
-__device__ __forceinline__ void load_epj_mix(const EpjMix* e, float4& r0, float4& r1) {
+// FP64 records in the forms of EpjF32, SpjF32 and EpiRel, with x - c in the
+// place of x: the difference is taken in FP64, so that a cluster far from the
+// origin keeps the separations its FP64 positions hold, and split on the
+// integer pipe (as 48-bit pairs of x and c a call
+// on 33,333 stars takes 0.43 ms, so 0.47, but companions 1e-5 apart were off by
+// 1e-5 of their force 4e4 from the origin).
+__device__ __forceinline__ void load_centred(const uint4& a, const uint4& b, const WalkDesc& wd, float4& r0, float4& r1) {
+    const float2 x = split_rn(__dsub_rn(__hiloint2double((int)a.y, (int)a.x), wd.cx));
+    const float2 y = split_rn(__dsub_rn(__hiloint2double((int)a.w, (int)a.z), wd.cy));
+    const float2 z = split_rn(__dsub_rn(__hiloint2double((int)b.y, (int)b.x), wd.cz));
+    r0.x = x.x;
+    r0.y = y.x;
+    r0.z = z.x;
+    r1.x = x.y;
+    r1.y = y.y;
+    r1.z = z.y;
+}
+
+__device__ __forceinline__ void load_epj_mix(const EpjMix* e, const WalkDesc& wd, float4& r0, float4& r1) {
     const uint4 a = __ldg(reinterpret_cast<const uint4*>(e)), b = __ldg(reinterpret_cast<const uint4*>(e) + 1);
-    split_f64(a.x, a.y, r0.x, r1.x);
-    split_f64(a.z, a.w, r0.y, r1.y);
-    split_f64(b.x, b.y, r0.z, r1.z);
+    load_centred(a, b, wd, r0, r1);
     r0.w = __uint_as_float(b.z);
     r1.w = __uint_as_float(b.w);
 }
 
-__device__ __forceinline__ void load_spj_mix(const SpjMix* e, float4 (&r)[4]) {
+__device__ __forceinline__ void load_spj_mix(const SpjMix* e, const WalkDesc& wd, float4 (&r)[4]) {
     const uint4* src = reinterpret_cast<const uint4*>(e);
     const uint4 a = __ldg(src), b = __ldg(src + 1);
     const float4 c = __ldg(reinterpret_cast<const float4*>(src + 2)), d = __ldg(reinterpret_cast<const float4*>(src + 3));
-    split_f64(a.x, a.y, r[0].x, r[1].x);
-    split_f64(a.z, a.w, r[0].y, r[1].y);
-    split_f64(b.x, b.y, r[0].z, r[1].z);
+    load_centred(a, b, wd, r[0], r[1]);
     r[0].w = __uint_as_float(b.z);
     r[1].w = d.z;  // tr
     r[2] = c;
     r[3] = d;
 }
 
-// An EpiRel row from the FP64 one: x - c from both (hi, lo) pairs.
 __device__ __forceinline__ void load_epi_mix(const EpiDev* e, const WalkDesc& wd, float eps2, float4& hi, float4& lo) {
     const uint4 a = __ldg(reinterpret_cast<const uint4*>(e)), b = __ldg(reinterpret_cast<const uint4*>(e) + 1);
-    float xh, xl, s, t;
-    split_f64(a.x, a.y, xh, xl);
-    two_sum(xh, -wd.ch[0], s, t);
-    two_sum(s, t + (xl - wd.cl[0]), hi.x, lo.x);
-    split_f64(a.z, a.w, xh, xl);
-    two_sum(xh, -wd.ch[1], s, t);
-    two_sum(s, t + (xl - wd.cl[1]), hi.y, lo.y);
-    split_f64(b.x, b.y, xh, xl);
-    two_sum(xh, -wd.ch[2], s, t);
-    two_sum(s, t + (xl - wd.cl[2]), hi.z, lo.z);
-    split_f64(b.z, b.w, xh, xl);
-    const float p = xh * xh;
-    hi.w = p + fmaf(2.f * xh, xl, fmaf(xh, xh, -p));
+    load_centred(a, b, wd, hi, lo);
+    const double rs = __hiloint2double((int)b.w, (int)b.z);
+    hi.w = f32_rn(__dmul_rn(rs, rs));
     lo.w = __int_as_float(kband_near(fmaxf(fabsf(hi.x), fmaxf(fabsf(hi.y), fabsf(hi.z))), hi.w, eps2));
 }
 
@@ -398,12 +400,13 @@ __device__ void producer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
         // Walk centre as an FP32 (hi, lo) pair.  A search forms it here: the same
         // values, but with the descriptor's copies its tile loop, which bounds it,
         // compiles to slower code (1M binaries 1.72 ms against 1.43).
-        const float chx = SR ? (float)wd.cx : wd.ch[0];
-        const float chy = SR ? (float)wd.cy : wd.ch[1];
-        const float chz = SR ? (float)wd.cz : wd.ch[2];
-        const float clx = SR ? (float)(wd.cx - (double)chx) : wd.cl[0];
-        const float cly = SR ? (float)(wd.cy - (double)chy) : wd.cl[1];
-        const float clz = SR ? (float)(wd.cz - (double)chz) : wd.cl[2];
+        // FP64 records come with the centre taken off (MX).
+        const float chx = MX ? 0.f : SR ? (float)wd.cx : wd.ch[0];
+        const float chy = MX ? 0.f : SR ? (float)wd.cy : wd.ch[1];
+        const float chz = MX ? 0.f : SR ? (float)wd.cz : wd.ch[2];
+        const float clx = MX ? 0.f : SR ? (float)(wd.cx - (double)chx) : wd.cl[0];
+        const float cly = MX ? 0.f : SR ? (float)(wd.cy - (double)chy) : wd.cl[1];
+        const float clz = MX ? 0.f : SR ? (float)(wd.cz - (double)chz) : wd.cl[2];
         const float rcut2 = SR ? (float)wd.rcut2 : wd.rcut2f;
         const float rsmax2 = wd.rs_max * wd.rs_max;
         const float hmax = fmaxf(wd.hx, fmaxf(wd.hy, wd.hz));
@@ -500,7 +503,7 @@ __device__ void producer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
                     for (int qq = 0; qq < QB; ++qq) {
                         if (id[qq] >= 0) {
                             if constexpr (MX) {
-                                load_epj_mix(p.epj + id[qq], r0[qq], r1[qq]);
+                                load_epj_mix(p.epj + id[qq], wd, r0[qq], r1[qq]);
                             } else {
                                 const float4* src = reinterpret_cast<const float4*>(p.epj32 + id[qq]);
                                 r0[qq] = __ldg(src);
@@ -621,7 +624,7 @@ __device__ void producer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
                     for (int qq = 0; qq < QSB; ++qq) {
                         if (id[qq] >= 0) {
                             if constexpr (MX) {
-                                load_spj_mix(p.spj + id[qq], r[qq]);
+                                load_spj_mix(p.spj + id[qq], wd, r[qq]);
                             } else {
                                 const float4* src = reinterpret_cast<const float4*>(p.spj32 + id[qq]);
 #pragma unroll

@@ -17,9 +17,9 @@
 // that device is current, and later calls reuse it.
 //
 // The pair kernel is the default warp-specialised one, reading the caller's
-// FP64 records (split into FP32 pairs on the integer pipe), with its walks
-// split on the device (pgf_plan.cu).  Measured on GB300, 33,333 stars: one
-// call 1.35 -> 0.46 ms (before: the CTA-synchronous kernel, walks whole).
+// FP64 records (x - c in FP64, split into FP32 pairs on the integer pipe), with
+// its walks split on the device (pgf_plan.cu).  Measured on GB300, 33,333 stars:
+// one call 1.35 -> 0.47 ms (before: the CTA-synchronous kernel, walks whole).
 #include "petar_gpuforce.h"
 #include "pgf_internal.cuh"
 
