@@ -7,17 +7,20 @@
 // radius R (the farthest i from the walk centre) with R / D small acts on
 // all n_i particles through the same few derivatives of its field: expanding
 // it costs about 700 operations once, however many i there are.  On the 1M
-// binary Plummer workload 64% of the EP-SP pairs pass the test below (35% at
-// 65k stars, 45% in a King 1M model with theta = 0.4).
+// binary Plummer workload 51% of the EP-SP pairs pass the test below (16% at
+// 65k stars, 34% in a King 1M model with theta = 0.4).
 //
-// Test.  A source is expanded when the first dropped terms, bounded for an i
-// at distance R straight towards it, stay below 2e-6 of the source's own
-// force: (P + 1) rho^P for the monopole (P = 8: rho = R / D <= 0.14) and
-// 84 rho^6 |Q| / (m D^2) for the quadrupole, whose terms end two orders
-// earlier.  Summed over a walk's sources, and away from that one direction,
-// the truncation is far below the FP32 rounding of the pair sums (1e-9 rms
-// of the force on Plummer and King models, against 7e-8).  The leading terms
-// (potential and uniform force) are summed as (hi, lo) FP32 pairs.
+// Test.  A source is expanded when the dropped terms, bounded for an i at
+// distance R straight towards it, stay below 2^-23 of the source's own force,
+// half the FP32 rounding of a pair (2e-7 over sources on one side):
+// 10.8 rho^8 for the monopole (rho = R / D) and 105 rho^6 |Q| / (m D^2) for the
+// quadrupole, whose terms end two orders earlier; these are the first dropped
+// terms, 9 and 84, and at rho = 0.14 a fifth and a quarter of them for the rest.
+// The bound holds source by source because nothing averages truncation out
+// where a walk's distant sources lie on one side: with 2e-6 for each of the two
+// terms (64% of the pairs at the 1M workload) such a walk's force was off by
+// 1.3e-6 where its pairs are off by 2.4e-7.  The leading terms (potential and
+// uniform force) are summed as (hi, lo) FP32 pairs.
 //
 // One CTA per walk, from the same queue order as the interaction kernel (a
 // split walk is handled whole; its parts share the compacted list).  Each of
@@ -31,11 +34,11 @@
 // list, so results do not depend on the grid.
 //
 // Measured on GB300 at the 1M binary workload (all walks in one launch): the
-// pair kernel alone 22.9 ms; this pass 2.7 ms and the pair kernel 12.0 ms
-// after it, with the force error against FP64 at median 5.2e-8 / p99.9
-// 5.9e-7 from 7.0e-8 / 6.5e-7.  FP64 instructions are what costs here (the
-// FP64 pipe issues one per warp in 64 cycles): with the leading sums and the
-// results in FP64 the pass took 3.7 ms.
+// pair kernel alone 22.7 ms; this pass 2.6 ms and the pair kernel 13.6 ms
+// after it, with the force error against FP64 at median 6.4e-8 / p99.9 4.9e-7
+// from 7.3e-8 / 5.5e-7.  FP64 instructions are what costs here (the FP64 pipe
+// issues one per warp in 64 cycles): with the leading sums and the results in
+// FP64 the pass took 1 ms more.
 #include "pgf_internal.cuh"
 #include "pgf_localexp.cuh"
 
@@ -44,8 +47,9 @@ namespace {
 
 constexpr int kRing = 64;      // per warp: 32 sources arrive while fewer than 32 wait
 constexpr int kMinI = 32;      // fewer i: direct pairs (33 n_i operations) cost about as much
-constexpr float kRhoMax = 0.14f;
-constexpr float kQuadTol = 2e-6f / 84.f;
+constexpr float kTrunc = 1.f / 8388608.f;  // truncation of a source as a share of its force
+constexpr float kRhoMax = 0.1f;            // 10.8 rho^8 < kTrunc, without quadrupole
+constexpr float kMonoErr = 10.8f, kQuadErr = 105.f;
 constexpr int kPad = 96;  // coefficients padded to 3 per lane
 
 constexpr int kStage = 2048;  // list entries of half a quarter
@@ -167,9 +171,10 @@ __global__ __launch_bounds__(W * 32, W == 4 ? 3 : 1) void far_kernel(Params p) {
         int ex;
         (void)frexpf(R / kRhoMax, &ex);
         const float inv = ldexpf(1.f, -ex);
-        const float Rs = R * inv;  // in (0.07, 0.14]
+        const float Rs = R * inv;  // in (0.05, 0.1]
         const float lim2 = (Rs / kRhoMax) * (Rs / kRhoMax);
-        const float kq = (Rs * Rs * Rs) * (Rs * Rs * Rs) / kQuadTol;
+        const float kq = (Rs * Rs * Rs) * (Rs * Rs * Rs) * (kQuadErr / kTrunc);
+        const float km = (Rs * Rs) * ((Rs * Rs * Rs) * (Rs * Rs * Rs)) * (kMonoErr / kTrunc);
         const float chx = wd.ch[0], chy = wd.ch[1], chz = wd.ch[2];
         const float clx = wd.cl[0], cly = wd.cl[1], clz = wd.cl[2];
 
@@ -209,7 +214,8 @@ __global__ __launch_bounds__(W * 32, W == 4 ? 3 : 1) void far_kernel(Params p) {
                 const float d2 = fmaf(hx, hx, fmaf(hy, hy, hz * hz));
                 const float d4 = d2 * d2;
                 const bool valid = id >= 0;
-                const bool far = valid && d2 >= lim2 && d2 < 1e16f && fabsf(m) < 1e30f && qn * kq <= fabsf(m) * (d4 * d4);
+                const bool far = valid && d2 >= lim2 && d2 < 1e16f && fabsf(m) < 1e30f &&
+                                 fmaf(km, fabsf(m), kq * qn) <= fabsf(m) * (d4 * d4);
                 const int id_cur = id;
                 id = id_next;
                 id_next = base + 64 + lane < n_w ? __ldg(ids + base + 64 + lane) : -1;
