@@ -1099,7 +1099,9 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
     PGF_CUDA(t.epi_rel.ensure(ni));
     PGF_CUDA(t.id_epj.ensure(ne));
     PGF_CUDA(t.id_spj.ensure(ns));
-    const bool far = far_applies(g.eps2, ni) && ns > 0 && t.mode != PGF_MODE_NEIGHBOR_SEARCH;
+    double sp_pairs = 0.0;
+    for (int w = 0; w < n_walk; ++w) sp_pairs += (double)n_epi[w] * (double)n_spj[w];
+    const bool far = far_applies(g.eps2, ni, sp_pairs) && ns > 0 && t.mode != PGF_MODE_NEIGHBOR_SEARCH;
     if (far) {
         PGF_CUDA(t.id_spj_near.ensure(ns));
         PGF_CUDA(t.spj_near.ensure(n_walk));

@@ -496,12 +496,27 @@ inline cudaError_t reset_counters(const Params& p, cudaStream_t s) {
     return cudaMemsetAsync(p.queue_head, 0, kLaunchCounters * sizeof(int32_t), s);
 }
 
-// The far-field pass pays from some thousand i-particles per launch: below,
-// its launch costs more than the pairs it saves.  It expands unsoftened
-// gravity only.
-constexpr int64_t kFarMinRows = 8192;
+// The far-field pass pays where enough superparticles are distant: where lists
+// are long (few walks of a large cluster do), or fairly long in launches that
+// fill the GPU.  With the pass and without it: Plummer models at theta = 0.3 of
+// 33,333 stars (2,200 EP-SP pairs per i) 0.54 and 0.51 ms a call, 65,536 (3,500)
+// 0.99 and 0.97, 98,304 (4,300) 1.40 and 1.43, 196,608 (5,700) 2.75 and 2.91;
+// 200-walk calls on 65,536 stars (3,500) 1.47 and 1.39 ms in all, on 393,216
+// (6,900) 8.47 and 8.82; 230,253 stars in five clusters (2,900) 2.58 and 2.42,
+// 112,126 in three (3,800) 1.48 and 1.52; King models at theta = 0.4: 131,072
+// (2,850) 1.205 and 1.218, 180,000 (3,000) 1.60 and 1.66.  It expands
+// unsoftened gravity only.
+constexpr int64_t kFarMinRows = 8192, kFarPairs = 4000;   // EP-SP pairs per i
+constexpr int64_t kFarRows = 80000, kFarRowsPairs = 3000;
 constexpr int64_t kFarWideRows = 40000;
-inline bool far_applies(double eps2, int64_t n_i) { return eps2 == 0.0 && n_i >= kFarMinRows; }
+inline bool far_applies(double eps2, int64_t n_i, double sp_pairs) {
+    return eps2 == 0.0 && n_i >= kFarMinRows &&
+           sp_pairs >= (double)n_i * (double)(n_i >= kFarRows ? kFarRowsPairs : kFarPairs);
+}
+// The device-resident step, which knows its lists only on the device: King
+// models, 65,536 particles 0.97 ms with the pass and 0.95 without, 131,072 1.50
+// and 1.52, 262,144 2.41 and 2.52.
+inline bool far_applies_step(double eps2, int64_t n) { return eps2 == 0.0 && n >= kFarRows; }
 
 // Tile of the default pair kernel: the parts of a device plan start at
 // multiples of it.

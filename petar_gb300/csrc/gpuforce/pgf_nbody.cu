@@ -1902,7 +1902,7 @@ struct pgf_nbody {
     DArr<WalkDesc> walks;
     int64_t cap_e = 0, cap_s = 0;
     DArr<int32_t> id_epj, id_spj;
-    DArr<int32_t> id_spj_near;  // far-field pass (far_applies): the compacted lists and their lengths
+    DArr<int32_t> id_spj_near;  // far-field pass (far_applies_step): the compacted lists and their lengths
     DArr<SpjNear> spj_near;
     // force scratch and results
     // split plan of launches with few walks (kPlanRows)
@@ -2129,7 +2129,7 @@ void bind_params(pgf_nbody* h) {
     bind_counters(p, h->flags.d + 4);
     p.part_align = kPartAlign;
     p.flush_tiles = h->planned() ? 1 : 0;
-    if (far_applies(h->cfg.eps2, h->n)) {
+    if (far_applies_step(h->cfg.eps2, h->n)) {
         p.id_spj_near = h->id_spj_near.d;
         p.spj_near = h->spj_near.d;
         p.far_wide = h->n <= kFarWideRows ? 1 : 0;
@@ -2163,7 +2163,7 @@ cudaError_t alloc_tasks(pgf_nbody* h, int64_t cap) {
 
 cudaError_t alloc_spj(pgf_nbody* h) {
     cudaError_t e = h->id_spj.alloc(h->cap_s);
-    if (e == cudaSuccess && far_applies(h->cfg.eps2, h->n)) e = h->id_spj_near.alloc(h->cap_s);
+    if (e == cudaSuccess && far_applies_step(h->cfg.eps2, h->n)) e = h->id_spj_near.alloc(h->cap_s);
     return e;
 }
 
@@ -2314,7 +2314,7 @@ int pgf_nbody_create(const pgf_nbody_config* cfg, int64_t n, const double* pos, 
     h->cap_s = 8 * n + 1024;
     NB_TRY(h->id_epj.alloc(h->cap_e));
     NB_TRY(alloc_spj(h));
-    if (far_applies(cfg->eps2, n)) NB_TRY(h->spj_near.alloc(n));
+    if (far_applies_step(cfg->eps2, n)) NB_TRY(h->spj_near.alloc(n));
     NB_TRY(h->blocksum.alloc(2 * (size_t)h->num_sms));
     if (n <= kPlanRows) {
         // Parts cost at most a sixteenth of an SM's share each beyond one per

@@ -19,13 +19,12 @@ from petar_gb300.walks import WalkBatch
 pytestmark = pytest.mark.gpu
 
 
-# Few i with long lists (eight warps per walk), and many i (four)
-@pytest.mark.parametrize("rows,n_s", [(8192, 4200), (81920, 60)])
+@pytest.mark.parametrize("rows", [8192, 40960])  # eight warps per walk, and four
 @pytest.mark.parametrize("near,far,quad", [(7.2, 7.4, 0.0), (7.2, 8.5, 3e-4), (7.5, 30.0, 0.0), (7.2, 400.0, 1e-4),
                                            (10.02, 10.3, 0.0), (10.5, 16.0, 1e-4)])
-def test_one_sided_sources(rows, n_s, near, far, quad):
+def test_one_sided_sources(rows, near, far, quad):
     rng = np.random.default_rng(3)
-    n_i, R = 64, 0.1
+    n_i, n_s, R = 64, 4200, 0.1
     nw = rows // n_i
     u = rng.normal(size=(nw, 3))
     u /= np.linalg.norm(u, axis=1)[:, None]
@@ -51,14 +50,16 @@ def test_one_sided_sources(rows, n_s, near, far, quad):
                    epj_disp=np.zeros(nw + 1, np.int64), id_epj=np.zeros(0, np.int32),
                    spj_disp=np.arange(nw + 1, dtype=np.int64) * n_s, id_spj=np.arange(nw * n_s, dtype=np.int32),
                    eps2=0.0, rcut2=1e-4, G=1.0)
+    own = wb.subset(np.arange(64))  # those compared
+    n = own.epi_rs.size
     with_pass = gpuforce.compute(wb)
-    o = oracle.force(wb)
+    o = oracle.force(own)
     wb.eps2 = 1e-300
     pairs = gpuforce.compute(wb)
     mag = np.linalg.norm(o["acc"], axis=1)  # one side: the sum of the magnitudes, to the spread of 0.05
-    err = lambda f: np.linalg.norm(f["acc"] - o["acc"], axis=1) / mag
+    err = lambda f: np.linalg.norm(f["acc"][:n] - o["acc"], axis=1) / mag
     ef, ep = err(with_pass), err(pairs)
     assert ef.max() <= ep.max() + 2 * 2.0 ** -23, (ef.max(), ep.max())
     assert ef.mean() <= ep.mean() + 2.0 ** -23, (ef.mean(), ep.mean())
-    pf, pp = (np.abs(f["pot"] - o["pot"]) / np.abs(o["pot"]) for f in (with_pass, pairs))
+    pf, pp = (np.abs(f["pot"][:n] - o["pot"]) / np.abs(o["pot"]) for f in (with_pass, pairs))
     assert pf.max() <= pp.max() + 2 * 2.0 ** -23, (pf.max(), pp.max())
