@@ -332,7 +332,7 @@ const char *pgf_last_error(void);
  *
  * The mixed-precision kernels still need scratch (walk descriptors, work
  * order, queue cursor, result rows of the parts that expensive walks are
- * split into).  It lives in one static device array of about 15 MB that every GPU loading the library keeps until the
+ * split into).  It lives in one static device array of about 16 MB that every GPU loading the library keeps until the
  * process exits, sized for at most PGF_NOALLOC_MAX_WALKS walks per call;
  * larger calls return PGF_ERR_CAPACITY.  The first call on each device looks
  * up that array's device address (with the device current) and keeps it; make

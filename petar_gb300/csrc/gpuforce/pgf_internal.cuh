@@ -285,6 +285,10 @@ struct Params {
     // out_nnb).
     Accp* part_accp;
     int32_t* part_nnb;
+    // Part 0 writes rows of its own there too: the walks' rows may overlap
+    // (only the combine kernel writes those of a split walk, whole results).
+    int32_t part0_rows;
+    int32_t pad1;
     // scratch
     // Launch counters, kLaunchCounters ints that lie together and are zeroed
     // before each launch (reset_counters): the work-queue cursor, the number
@@ -617,6 +621,7 @@ struct PlanArgs {
     int32_t* n_desc;
     int32_t* n_split;
     int cap_desc, cap_splits, row0;
+    int part0_rows;  // Params::part0_rows
     int64_t cap_rows;
 };
 cudaError_t launch_plan(const PlanArgs& a, cudaStream_t s);

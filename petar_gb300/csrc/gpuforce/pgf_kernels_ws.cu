@@ -741,7 +741,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
     float dt[CO ? KI : 1], ds[CO ? KI : 1];
     unsigned js_inv = 1u << 16;
     double rcut2d = 0.0;
-    bool add_self = true, parts = false, further = false;  // further: a part >= 1
+    bool add_self = true, parts = false, further = false;  // further: writes part rows
     int since = 0;
 #pragma unroll
     for (int k = 0; k < (CO ? KI : 1); ++k) dt[k] = ds[k] = 0.f;
@@ -1112,7 +1112,7 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
             gbase = wd.i_begin + h.ipass + slot;
             ibase = wd.i_root + h.ipass + slot;
             parts = wd.n_parts > 1;
-            further = wd.part != 0;
+            further = wd.part != 0 || (parts && p.part0_rows);
             if constexpr (!SR) add_far = spj_list(p, wd).add_far;
             if constexpr (CO) {
                 rcut2d = wd.rcut2;

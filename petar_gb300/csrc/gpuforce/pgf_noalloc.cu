@@ -11,7 +11,7 @@
 // per-walk descriptors (centre, box, largest r_search), the work-queue order,
 // the queue cursor, and the result rows of the parts that expensive walks are
 // split into.  Here that scratch is the file-scope array g_noalloc_scratch,
-// sized for PGF_NOALLOC_MAX_WALKS walks (about 15 MB); every GPU that loads the library keeps it until the process
+// sized for PGF_NOALLOC_MAX_WALKS walks (about 16 MB); every GPU that loads the library keeps it until the process
 // exits.  Host code cannot use the array's name as a device address: the first
 // call on each device looks the address up with cudaGetSymbolAddress while
 // that device is current, and later calls reuse it.
@@ -33,10 +33,11 @@ using namespace pgf;
 
 constexpr int kMaxWalks = PGF_NOALLOC_MAX_WALKS;
 // Parts of split walks: at most 16 per SM beyond one per walk, and their
-// result rows (33,333 stars want 150,000 in quarters of an SM's share).
+// result rows (200,000 stars want 266,000 in eighths of an SM's share: 2.62 ms a
+// call, 2.83 in quarters; 33,333 stars 325,000: 0.48 ms, 0.47 in quarters).
 constexpr int kMaxParts = 2560;
 constexpr int kMaxDescs = kMaxWalks + kMaxParts;
-constexpr int kPartRows = 1 << 18;
+constexpr int kPartRows = 9 << 15;
 constexpr int kMaxDevices = 64;
 constexpr size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 constexpr size_t kFlagsOff = 0;  // [0], [1] descriptors and split walks of the plan, [2] input error bits, [3] the kernels' error word, [4..6] launch counters
@@ -268,6 +269,7 @@ extern "C" int pgf_force_device_noalloc(int n_walk, const int64_t* walk_table, c
     p.part_align = kPartAlign;
     p.part_accp = reinterpret_cast<Accp*>(base + kRowsOff);
     p.part_nnb = reinterpret_cast<int32_t*>(base + kRowNnbOff);
+    p.part0_rows = a.part0_rows = 1;  // the caller's walks may share rows
     p.eps2 = eps2;
     p.G = G;
     p.out_accp = reinterpret_cast<Accp*>(accp);

@@ -89,7 +89,7 @@ __global__ __launch_bounds__(kPlanThreads) void plan_kernel(PlanArgs a) {
             const WalkDesc d = a.roots[k];
             const int p = walk_parts(d, walk_cost(a, k, d), target) - 1;
             parts += p;
-            rows += (long long)p * d.n_i;
+            if (p > 0) rows += (long long)(p + a.part0_rows) * d.n_i;
         }
         v = make_longlong2(parts, rows);
 #pragma unroll
@@ -149,7 +149,7 @@ __global__ __launch_bounds__(kPlanThreads) void plan_kernel(PlanArgs a) {
                     d.n_spj = s1 - s0;
                     d.part = (uint16_t)j;
                     d.n_parts = (uint16_t)np;
-                    if (j > 0) d.i_begin = a.row0 + row + (j - 1) * d0.n_i;
+                    if (j + a.part0_rows > 0) d.i_begin = a.row0 + row + (j + a.part0_rows - 1) * d0.n_i;
                     a.walks[w] = d;
                     atomicAdd(&s.hist[q], 1);
                 } else {
@@ -159,7 +159,7 @@ __global__ __launch_bounds__(kPlanThreads) void plan_kernel(PlanArgs a) {
             if (pass == 0) {
                 const int r = atomicAdd(a.n_split, 1);
                 a.splits[r] = SplitRec{d0.i_begin, a.row0 + row, d0.n_i, np};
-                row += (np - 1) * d0.n_i;
+                row += (np - 1 + a.part0_rows) * d0.n_i;
             }
             dsc += np - 1;
         }
@@ -180,7 +180,7 @@ __global__ __launch_bounds__(kPlanThreads) void plan_kernel(PlanArgs a) {
 // combine_parts_kernel, the number of records read on the device.
 __global__ __launch_bounds__(128) void combine_plan_kernel(const SplitRec* __restrict__ recs, const int32_t* n_split,
                                                            Accp* accp, int32_t* nnb, const Accp* part_accp,
-                                                           const int32_t* part_nnb, double G) {
+                                                           const int32_t* part_nnb, int part0_rows, double G) {
     const int n = *n_split;
     if (n == 0) return;
     // few walks: several CTAs each (3,000 stars: 22 -> 10 us)
@@ -190,11 +190,11 @@ __global__ __launch_bounds__(128) void combine_plan_kernel(const SplitRec* __res
         for (int i = (q % m) * blockDim.x + threadIdx.x; i < r.n_i; i += m * blockDim.x) {
             const int64_t r0 = (int64_t)r.row0 + i;
             float2 a[4];
-            load_pairs(accp + r0, a);
-            int c = nnb[r0];
+            load_pairs(part0_rows ? part_accp + r.rows1 + i : accp + r0, a);
+            int c = part0_rows ? part_nnb[r.rows1 + i] : nnb[r0];
 #pragma unroll 8
             for (int k = 1; k < r.n_parts; ++k) {
-                const int64_t row = (int64_t)r.rows1 + (int64_t)(k - 1) * r.n_i + i;
+                const int64_t row = (int64_t)r.rows1 + (int64_t)(k - 1 + part0_rows) * r.n_i + i;
                 float2 b[4];
                 load_pairs(part_accp + row, b);
 #pragma unroll
@@ -219,7 +219,7 @@ cudaError_t launch_plan(const PlanArgs& a, cudaStream_t s) {
 cudaError_t launch_combine_plan(const PlanArgs& a, const Params& p, cudaStream_t s) {
     combine_plan_kernel<<<a.num_sms * 4, 128, 0, s>>>(a.splits, a.n_split, p.out_accp, p.out_nnb,
                                                       p.part_accp ? p.part_accp : p.out_accp,
-                                                      p.part_nnb ? p.part_nnb : p.out_nnb, p.G);
+                                                      p.part_nnb ? p.part_nnb : p.out_nnb, a.part0_rows, p.G);
     return cudaGetLastError();
 }
 
