@@ -346,9 +346,10 @@ const char *pgf_last_error(void);
  * device first, and the call copies the check's result to the host and waits
  * on the stream for it (so it also waits for the work queued on the stream
  * before it) before it launches the force kernels.  Those are then left
- * running on the stream.  Their waits are bounded (1 s); should one run out,
- * the next call reports it as PGF_ERR_DEVICE, and the results of the call that
- * it happened in are not complete.
+ * running on the stream.  Their waits are bounded (pgf_set_wait_limit_ns);
+ * should one run out, the last kernel of the call, which has no waits,
+ * evaluates the call again, so the results are complete in any case and the
+ * check is the only device-side failure the call can report.
  *
  * walk_table: 6 int64 per walk: i_begin, n_i, epj_begin, n_epj, spj_begin,
  *   n_spj (rows of epi; offsets into id_epj / id_spj).

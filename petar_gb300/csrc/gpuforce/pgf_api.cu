@@ -1339,6 +1339,10 @@ bool valid_tag(int tag) { return tag >= 0 && tag < kMaxTags; }
 
 }  // namespace
 
+namespace pgf {
+WaitHooks wait_hooks() { return WaitHooks{g.wait_limit_ns, g.stall_after_items}; }
+}  // namespace pgf
+
 extern "C" {
 
 int pgf_initialize(int rank, double eps2, double rcut2, double G) {

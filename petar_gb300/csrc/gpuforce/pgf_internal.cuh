@@ -329,7 +329,17 @@ struct Params {
     // Result of the device-side check of a host-direct dispatch's ids, or
     // null: when it is non-zero the force kernels run nothing.
     const int32_t* input_err;
+    // The CTA-synchronous kernel runs only when this word is non-zero (null:
+    // always).  A null order is the walks as they lie.
+    const int32_t* run_if;
 };
+
+// Limit of the bounded waits and the stall test hook, as set through the C ABI.
+struct WaitHooks {
+    uint64_t wait_limit_ns;  // 0: 1 s
+    int stall_after_items;   // 0: none
+};
+WaitHooks wait_hooks();
 
 // Number of walks of this launch.
 __device__ __forceinline__ int walk_count(const Params& p) {

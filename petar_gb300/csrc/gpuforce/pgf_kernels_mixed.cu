@@ -158,6 +158,7 @@ __device__ __forceinline__ double as_double(unsigned lo, unsigned hi) {
 
 __global__ __launch_bounds__(kThreads, PGF_MINB) void mixed_kernel(Params p) {
     if (p.input_err && *p.input_err) return;  // the inputs failed their check: run nothing
+    if (p.run_if && !*p.run_if) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem& s = *reinterpret_cast<Smem*>(smem_raw);
     const int tid = threadIdx.x;
@@ -177,7 +178,7 @@ __global__ __launch_bounds__(kThreads, PGF_MINB) void mixed_kernel(Params p) {
         __syncthreads();
         const int wq = s.w;
         if (wq >= n_walk) break;
-        const int widx = p.order[wq];
+        const int widx = p.order ? p.order[wq] : wq;
         const WalkDesc wd = p.walks[widx];
         const double cx = wd.cx, cy = wd.cy, cz = wd.cz;
         const float rcut2 = (float)wd.rcut2;
@@ -542,13 +543,20 @@ __global__ __launch_bounds__(256) void retest_kernel(Params p) {
 cudaError_t launch_mixed(const Params& p, cudaStream_t s, int num_sms) {
     if (p.n_walk <= 0) return cudaSuccess;
     cudaError_t e;
-    static int per_sm = 0;
+    // Per device: the attribute and the occupancy belong to its context.
+    constexpr int kMaxDevices = 64;
+    static int per_sm_of[kMaxDevices] = {};
+    int dev = 0;
+    e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    int per_sm = dev < kMaxDevices ? per_sm_of[dev] : 0;
     if (per_sm == 0) {
         e = cudaFuncSetAttribute(mixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));
         if (e != cudaSuccess) return e;
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mixed_kernel, kThreads, sizeof(Smem));
         if (e != cudaSuccess) return e;
         if (per_sm < 1) per_sm = 1;
+        if (dev < kMaxDevices) per_sm_of[dev] = per_sm;
     }
     int grid = num_sms * per_sm;
     if (grid > p.n_walk) grid = p.n_walk;

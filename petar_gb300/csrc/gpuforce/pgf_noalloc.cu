@@ -40,7 +40,7 @@ constexpr int kMaxDescs = kMaxWalks + kMaxParts;
 constexpr int kPartRows = 9 << 15;
 constexpr int kMaxDevices = 64;
 constexpr size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
-constexpr size_t kFlagsOff = 0;  // [0], [1] descriptors and split walks of the plan, [2] input error bits, [3] the kernels' error word, [4..6] launch counters
+constexpr size_t kFlagsOff = 0;  // [0], [1] descriptors and split walks of the plan, [2] input error bits, [3] the pair kernel's error word, [4..6] launch counters, [7..9] those of the kernel behind it
 constexpr size_t kDescOff = 256;
 constexpr size_t kPlanOff = align256(kDescOff + sizeof(WalkDesc) * kMaxWalks);
 constexpr size_t kOrderOff = align256(kPlanOff + sizeof(WalkDesc) * kMaxDescs);
@@ -218,7 +218,7 @@ extern "C" int pgf_force_device_noalloc(int n_walk, const int64_t* walk_table, c
     int32_t* flags = reinterpret_cast<int32_t*>(base + kFlagsOff);
     WalkDesc* desc = reinterpret_cast<WalkDesc*>(base + kDescOff);
 
-    e = cudaMemsetAsync(flags, 0, 3 * sizeof(int32_t), s);
+    e = cudaMemsetAsync(flags, 0, 4 * sizeof(int32_t), s);
     if (e != cudaSuccess) return fail(errbuf, errbuf_len, PGF_ERR_CUDA, "pgf_force_device_noalloc: %s", cudaGetErrorString(e));
     walk_prep_kernel<<<n_walk, 128, 0, s>>>(n_walk, walk_table, epi, n_epi_total, n_epj_total, n_spj_total, id_epj,
                                             n_id_epj, id_spj, n_id_spj, rcut2, desc, flags + 2);
@@ -226,16 +226,10 @@ extern "C" int pgf_force_device_noalloc(int n_walk, const int64_t* walk_table, c
     if (e != cudaSuccess) return fail(errbuf, errbuf_len, PGF_ERR_CUDA, "pgf_force_device_noalloc: prep: %s", cudaGetErrorString(e));
     // The interaction kernels trust the lists, so the validation result is
     // read back (into this stack variable) before they are launched.
-    int32_t err[2] = {0, 0};
-    e = cudaMemcpyAsync(err, flags + 2, sizeof(err), cudaMemcpyDeviceToHost, s);
+    int32_t err_bits = 0;
+    e = cudaMemcpyAsync(&err_bits, flags + 2, sizeof(err_bits), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(errbuf, errbuf_len, PGF_ERR_CUDA, "pgf_force_device_noalloc: %s", cudaGetErrorString(e));
-    const int32_t err_bits = err[0];
-    if (err[1]) {
-        (void)cudaMemsetAsync(flags + 3, 0, sizeof(int32_t), s);
-        return fail(errbuf, errbuf_len, PGF_ERR_DEVICE,
-                    "pgf_force_device_noalloc: a wait in an earlier call's kernels ran out (its results are not complete)");
-    }
     if (err_bits)
         return fail(errbuf, errbuf_len, PGF_ERR_ARG, "pgf_force_device_noalloc: %s%s%s", (err_bits & kBadWalk) ? "walk table row out of range; " : "",
                     (err_bits & kBadEpjId) ? "EPJ id out of range; " : "", (err_bits & kBadSpjId) ? "SPJ id out of range" : "");
@@ -276,10 +270,29 @@ extern "C" int pgf_force_device_noalloc(int n_walk, const int64_t* walk_table, c
     p.out_nnb = n_ngb;
     bind_counters(p, flags + 4);
     p.err = flags + 3;
-    e = reset_counters(p, s);
+    const WaitHooks hooks = wait_hooks();
+    p.wait_limit_ns = hooks.wait_limit_ns;
+    p.stall_after_items = hooks.stall_after_items;
+    // The call has returned when the pair kernel runs, so a wait of its that
+    // runs out has nobody to report to: then the CTA-synchronous kernel, which
+    // has no waits, evaluates the walks again, whole.  Else it ends at once
+    // (1.8 us of a call's 430 on 33,333 stars).
+    Params q = p;
+    q.walks = desc;
+    q.order = nullptr;
+    q.n_walk = q.n_root = n_walk;
+    q.n_walk_dev = nullptr;
+    q.part_accp = nullptr;
+    q.part_nnb = nullptr;
+    q.part0_rows = 0;
+    q.retest_cap = 0;  // neighbours in the guard band are tested in place
+    q.run_if = p.err;
+    bind_counters(q, flags + 7);
+    e = cudaMemsetAsync(flags + 4, 0, 2 * kLaunchCounters * sizeof(int32_t), s);
     if (e == cudaSuccess) e = launch_plan(a, s);
     if (e == cudaSuccess) e = launch_ws_fp64_records(p, s, g_num_sms[dev]);
     if (e == cudaSuccess) e = launch_combine_plan(a, p, s);
+    if (e == cudaSuccess) e = launch_mixed(q, s, g_num_sms[dev]);
     if (e != cudaSuccess) return fail(errbuf, errbuf_len, PGF_ERR_CUDA, "pgf_force_device_noalloc: launch: %s", cudaGetErrorString(e));
     return PGF_OK;
 }
