@@ -217,15 +217,19 @@ int pgf_set_walk_split(int enable);
  * pgf_autotune_dispatch sets it too.  Results are as for pgf_set_walk_split. */
 int pgf_set_walk_split_unit(int div);
 
-/* Limit of every bounded wait inside the warp-specialised kernels, in
+/* Limit of every bounded wait inside the warp-specialised kernels and at the
+ * grid barriers of the device-resident tree, in
  * nanoseconds of the GPU's global timer (0 restores the default, 1 s).  A
  * wait that runs out sets the device error word and its warp returns, so the
- * kernel ends and the next retrieve reports PGF_ERR_DEVICE instead of the
+ * kernel ends and the next retrieve (pgf_nbody_force, pgf_nbody_run and
+ * pgf_nbody_create themselves) reports PGF_ERR_DEVICE instead of the
  * launch hanging.  No counterpart in the reference, whose kernels do not wait. */
 int pgf_set_wait_limit_ns(uint64_t limit_ns);
 /* Test hook for the path above: with items > 0 the producer warp of the
  * warp-specialised kernels stops publishing ring items after that many, so
  * that the consumers' waits run out (no fault, no trap; every warp returns).
+ * With items > 0 the first CTA of the device-resident tree leaves before its
+ * first grid barrier, so that the others' waits run out.
  * 0 (the default) turns it off.  For failure-detection tests only. */
 int pgf_test_stall_producer(int items);
 

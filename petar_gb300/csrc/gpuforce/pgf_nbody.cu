@@ -353,9 +353,9 @@ __device__ __forceinline__ unsigned long long tree_timer() {
 }
 
 // Grid barrier of a cooperative launch: bar counts arrivals since the build
-// began.  A wait that takes longer than a second sets the build's error and
+// began.  A wait that takes longer than the limit sets the build's error and
 // returns false in every CTA that sees it; the kernel then ends.
-__device__ bool grid_sync(unsigned* bar, unsigned& epoch, int32_t* err) {
+__device__ bool grid_sync(unsigned* bar, unsigned& epoch, int32_t* err, uint64_t limit_ns) {
     __shared__ int s_ok;
     __syncthreads();
     epoch += gridDim.x;
@@ -368,7 +368,7 @@ __device__ bool grid_sync(unsigned* bar, unsigned& epoch, int32_t* err) {
             unsigned v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
             if ((int)(v - epoch) >= 0) break;
-            if (tree_timer() - t0 > 1000000000ull) {
+            if (tree_timer() - t0 > limit_ns) {
                 atomicOr(err, kErrBarrier);
                 ok = 0;
                 break;
@@ -455,6 +455,8 @@ struct TreeArgs {
     SpjMix* spj;
     SpjF32* spj32;
     SpjQ64* spjq;
+    uint64_t wait_limit_ns;  // of the grid barriers
+    int stall;               // test hook: the first CTA leaves before its first barrier
 };
 
 // What the cells of a level share: the opening criterion, and the distance
@@ -815,6 +817,7 @@ __global__ __launch_bounds__(kTreeThreads, 1) void tree_kernel(TreeArgs a) {
     const int G = gridDim.x, bid = blockIdx.x;
     unsigned epoch = 0;
     if (h->err) return;  // before the first barrier: every CTA sees it
+    if (a.stall && bid == 0) return;
     if (t < kLevels) level_tab(a, s_tab, t);  // read after the barriers below
     // ---- levels: children of a level in their parents' order ----
     int lb = 0, le = 1, depth = 0;
@@ -888,7 +891,7 @@ __global__ __launch_bounds__(kTreeThreads, 1) void tree_kernel(TreeArgs a) {
             a.blocksum[(L & 1) * G + bid] = s_sum;
             s_before = s_total = 0;
         }
-        if (!grid_sync(&h->bar, epoch, &h->err)) return;
+        if (!grid_sync(&h->bar, epoch, &h->err, a.wait_limit_ns)) return;
         for (int k = t; k < G; k += kTreeThreads) {
             const int v = __ldcg(a.blocksum + (L & 1) * G + k);
             if (v) {
@@ -934,7 +937,7 @@ __global__ __launch_bounds__(kTreeThreads, 1) void tree_kernel(TreeArgs a) {
         }
         if (bid == 0 && t == 0) h->level_begin[L + 2 <= kLevels + 1 ? L + 2 : kLevels + 1] = le + total;
         if (total == 0) break;  // every CTA
-        if (!grid_sync(&h->bar, epoch, &h->err)) return;
+        if (!grid_sync(&h->bar, epoch, &h->err, a.wait_limit_ns)) return;
         lb = le;
         le += total;
     }
@@ -942,12 +945,12 @@ __global__ __launch_bounds__(kTreeThreads, 1) void tree_kernel(TreeArgs a) {
     if (bid == 0 && t > depth + 1 && t <= kLevels + 1) h->level_begin[t] = nc;
     // ---- class order ----
     for (int b = t; b < kCellBins; b += kTreeThreads) s_hist[b] = 0;
-    if (!grid_sync(&h->bar, epoch, &h->err)) return;  // first_child and leaf flags of the last level
+    if (!grid_sync(&h->bar, epoch, &h->err, a.wait_limit_ns)) return;  // first_child and leaf flags of the last level
     for (int64_t c = gtid(); c < nc; c += gstride()) atomicAdd(&s_hist[cell_bin(a.cells[c])], 1);
     __syncthreads();
     for (int b = t; b < kCellBins; b += kTreeThreads)
         if (s_hist[b]) atomicAdd(&h->cell_hist[b], s_hist[b]);
-    if (!grid_sync(&h->bar, epoch, &h->err)) return;
+    if (!grid_sync(&h->bar, epoch, &h->err, a.wait_limit_ns)) return;
     {
         static_assert(kCellBins <= kTreeThreads, "one bin per thread");
         int tot;
@@ -974,14 +977,14 @@ __global__ __launch_bounds__(kTreeThreads, 1) void tree_kernel(TreeArgs a) {
         if (b >= 0) a.order[s_base[b] + r] = (int32_t)c;
         __syncthreads();
     }
-    if (!grid_sync(&h->bar, epoch, &h->err)) return;
+    if (!grid_sync(&h->bar, epoch, &h->err, a.wait_limit_ns)) return;
     // ---- moments: leaves, then the inner cells from the deepest level up ----
     double (*const buf)[8] = s_buf[warp][lane >> 3];
     moments_range(a, s_tab, 0, s_hist[kLeafBins], buf);
     for (int L = depth; L >= 0; --L) {
         const int lo = s_hist[kLeafBins + 8 * L], hi = s_hist[kLeafBins + 8 * L + 8];
         if (lo == hi) continue;  // every CTA
-        if (!grid_sync(&h->bar, epoch, &h->err)) return;
+        if (!grid_sync(&h->bar, epoch, &h->err, a.wait_limit_ns)) return;
         moments_range(a, s_tab, lo, hi, buf);
     }
 }
@@ -1927,6 +1930,7 @@ struct pgf_nbody {
     cudaGraphExec_t exec = nullptr;
     int graph_steps = 0;
     double graph_dt = 0.0;
+    WaitHooks graph_hooks{};
     cudaEvent_t ev[6] = {};
     double last_tree_ms = 0, last_force_ms = 0;
     int64_t steps_done = 0;
@@ -1987,7 +1991,10 @@ cudaError_t enqueue_build(pgf_nbody* h) {
     {
         TreeArgs a{hd, h->cells.d, h->cw.d, h->mom.d, h->nch.d, h->bnd.d, h->blocksum.d, h->key_out.d, h->cell_order.d,
                    h->epi.d, h->epj_m64.d, h->inv_theta2, h->cfg.n_leaf_limit, h->cap_cells, h->spj.d, h->spj32.d,
-                   h->spjq.d};
+                   h->spjq.d, 1000000000ull, 0};
+        const WaitHooks hooks = wait_hooks();
+        if (hooks.wait_limit_ns) a.wait_limit_ns = hooks.wait_limit_ns;
+        a.stall = hooks.stall_after_items > 0;
         void* args[] = {&a};
         e = cudaLaunchCooperativeKernel((const void*)tree_kernel, dim3(h->num_sms), dim3(kTreeThreads), args, 0, s);
         if (e != cudaSuccess) return e;
@@ -2038,6 +2045,9 @@ PlanArgs plan_args(pgf_nbody* h) {
 cudaError_t enqueue_force(pgf_nbody* h) {
     cudaError_t e = reset_counters(h->p, h->stream);
     if (e != cudaSuccess) return e;
+    const WaitHooks hooks = wait_hooks();
+    h->p.wait_limit_ns = hooks.wait_limit_ns;
+    h->p.stall_after_items = hooks.stall_after_items;
     if (h->cfg.precision == PGF_PRECISION_FP64) return launch_fp64(h->p, h->stream, h->num_sms);
     if (h->variant == 0) {
         e = launch_mixed(h->p, h->stream, h->num_sms);
@@ -2091,14 +2101,17 @@ int read_hdr(pgf_nbody* h, TreeHdr* out) {
     return PGF_OK;
 }
 
+int barrier_error() { return nb_fail(PGF_ERR_DEVICE, "a grid barrier of the device tree ran out"); }
+
 int check_errors(pgf_nbody* h) {
     TreeHdr t;
     if (int r = read_hdr(h, &t)) return r;
     int32_t kerr = 0;
     NB_CUDA(cudaMemcpy(&kerr, h->flags.d + 2, sizeof(int32_t), cudaMemcpyDeviceToHost));
+    if (t.err_sticky & kErrBarrier) return barrier_error();
     if (t.err_sticky)
         return nb_fail(PGF_ERR_CAPACITY, "device list builder ran out of room (bits %d: 1 cells, 2 EPJ entries, "
-                       "4 SPJ entries); raise list_capacity_factor", t.err_sticky);
+                       "4 SPJ entries, 8 list tasks); raise list_capacity_factor", t.err_sticky);
     if (kerr) return nb_fail(PGF_ERR_DEVICE, "device error word %d", kerr);
     return PGF_OK;
 }
@@ -2219,6 +2232,7 @@ int build_fit(pgf_nbody* h) {
             bind_params(h);
             continue;
         }
+        if (t.err & kErrBarrier) return barrier_error();  // no array is too small: building again would not help
         if (t.err & kErrCells) {
             if (h->cap_cells >= 1 << 30) return nb_fail(PGF_ERR_CAPACITY, "more than 2^30 tree cells");
             NB_CUDA(alloc_cells(h, h->cap_cells * 2));
@@ -2395,7 +2409,10 @@ int pgf_nbody_run(pgf_nbody* h, int n_steps, double dt, int use_graph, double* m
         if (ms) *ms = 0.0;
         return PGF_OK;
     }
-    if (use_graph && (!h->exec || h->graph_steps != n_steps || h->graph_dt != dt)) {
+    const WaitHooks hooks = wait_hooks();
+    if (use_graph && (!h->exec || h->graph_steps != n_steps || h->graph_dt != dt ||
+                      h->graph_hooks.wait_limit_ns != hooks.wait_limit_ns ||
+                      h->graph_hooks.stall_after_items != hooks.stall_after_items)) {
         if (h->exec) {
             cudaGraphExecDestroy(h->exec);
             h->exec = nullptr;
@@ -2418,6 +2435,7 @@ int pgf_nbody_run(pgf_nbody* h, int n_steps, double dt, int use_graph, double* m
         }
         h->graph_steps = n_steps;
         h->graph_dt = dt;
+        h->graph_hooks = hooks;
     }
     if (int r = clear_errors(h)) return r;
     NB_CUDA(cudaEventRecord(h->ev[3], h->stream));
