@@ -314,8 +314,6 @@ int setup_device(int rank) {
             for (auto& ev : c) PGF_CUDA(cudaEventCreate(&ev));
     }
     PGF_CUDA(g.scratch.ensure(kScratchInts));
-    g.retest_cap = 1 << 20;
-    PGF_CUDA(g.retest.ensure((size_t)g.retest_cap));
     PGF_CUDA(cudaMemset(g.scratch.d, 0, kScratchInts * sizeof(int32_t)));
     PGF_CUDA(g.hd_err.ensure(kHdErrWords * kMaxTags));
     PGF_CUDA(cudaMemset(g.hd_err.d, 0, kHdErrWords * kMaxTags * sizeof(int32_t)));
@@ -644,6 +642,14 @@ bool runs_far(const TagState& t) {
     if (t.mode == PGF_MODE_NEIGHBOR_SEARCH) return false;
     if (t.mode == PGF_MODE_GRADIENT || t.mode == PGF_MODE_FORCE_CHANGEOVER) return true;
     return t.precision == PGF_PRECISION_MIXED && t.variant != 0;
+}
+
+// Re-test records, for the CTA-synchronous kernel alone (25 MB).
+int ensure_retest(const TagState& t) {
+    if (t.mode != PGF_MODE_FORCE || t.precision != PGF_PRECISION_MIXED || t.variant != 0) return PGF_OK;
+    PGF_CUDA(g.retest.ensure((size_t)1 << 20));
+    g.retest_cap = 1 << 20;
+    return PGF_OK;
 }
 
 // Main kernel of the tag's precision and variant on stream s, bracketed by two
@@ -1123,6 +1129,7 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
     t.n_epi.assign(n_epi, n_epi + n_walk);
     t.precision = g.precision;
     t.variant = g.variant;
+    if (int r = ensure_retest(t)) return r;
     Params& p = t.params;
     p = Params{};
     p.epi = t.epi.d;
@@ -1461,6 +1468,7 @@ int pgf_recompute(int tag) {
     PGF_CUDA(cudaEventRecord(t.ev[0], g.stream));
     t.precision = g.precision;
     t.variant = g.variant;
+    if (int r = ensure_retest(t)) return r;
     return launch_tag(t);
 }
 
@@ -1911,6 +1919,7 @@ int pgf_finalize(void) {
     g.h_spj_q64.release();
     g.scratch.release();
     g.retest.release();
+    g.retest_cap = 0;
     g.hd_err.release();
     if (g.ev_send0) cudaEventDestroy(g.ev_send0);
     if (g.ev_send1) cudaEventDestroy(g.ev_send1);

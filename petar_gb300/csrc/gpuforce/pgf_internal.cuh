@@ -239,8 +239,8 @@ struct Retest {
     int64_t j_begin;  // offset in id_epj
     int32_t i;        // EPI row
     int32_t n;        // number of list entries
-    int32_t walk;     // walk (descriptor index) of the i-particle
     int32_t row;      // result row
+    int32_t pad;
 };
 
 // Superparticles of one walk left to the pair kernels by the far-field pass:

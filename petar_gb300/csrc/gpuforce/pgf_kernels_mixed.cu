@@ -467,7 +467,7 @@ __global__ __launch_bounds__(kThreads, PGF_MINB) void mixed_kernel(Params p) {
                                 rr.i = ri[k];
                                 rr.row = gi[k];
                                 rr.n = rt.nt;
-                                rr.walk = widx;
+                                rr.pad = 0;
                                 p.retest[slot_r] = rr;
                             } else {
                                 cnt[k] += exact_count(p, ri[k], rt.base, rt.nt);

@@ -1917,8 +1917,7 @@ struct pgf_nbody {
     DArr<Accp> out_accp;
     DArr<int32_t> out_nnb;
     DArr<int32_t> flags;  // [0], [1] descriptors and split walks of the plan, [2] kernel error word, [4..6] launch counters
-    DArr<Retest> retest;
-    int retest_cap = 1 << 20;
+    DArr<Retest> retest;  // kernel variant 0 only (ensure_retest)
     DArr<TreeHdr> hdr;
     DArr<double> part;    // bbox partials
     DArr<double> energy;  // partials + result
@@ -2116,6 +2115,16 @@ int check_errors(pgf_nbody* h) {
     return PGF_OK;
 }
 
+void bind_params(pgf_nbody* h);
+
+// Re-test records (25 MB), for the CTA-synchronous kernel alone.
+cudaError_t ensure_retest(pgf_nbody* h) {
+    if (h->retest.d || h->variant != 0 || h->cfg.precision != PGF_PRECISION_MIXED) return cudaSuccess;
+    const cudaError_t e = h->retest.alloc((size_t)1 << 20);
+    if (e == cudaSuccess) bind_params(h);
+    return e;
+}
+
 void bind_params(pgf_nbody* h) {
     Params& p = h->p;
     p = Params{};
@@ -2149,7 +2158,7 @@ void bind_params(pgf_nbody* h) {
     }
     p.err = h->flags.d + 2;
     p.retest = h->retest.d;
-    p.retest_cap = h->retest_cap;
+    p.retest_cap = (int)h->retest.n;
 }
 
 cudaError_t alloc_cells(pgf_nbody* h, int cap) {
@@ -2332,9 +2341,9 @@ int pgf_nbody_create(const pgf_nbody_config* cfg, int64_t n, const double* pos, 
     NB_TRY(h->blocksum.alloc(2 * (size_t)h->num_sms));
     if (n <= kPlanRows) {
         // Parts cost at most a sixteenth of an SM's share each beyond one per
-        // walk, so there are at most 16 num_sms further ones.
+        // walk, so there are at most 16 num_sms further ones; a walk has at most 31.
         const int64_t extra = 16 * (int64_t)h->num_sms;
-        h->plan_rows = std::min<int64_t>(extra * std::max(cfg->n_group_limit, cfg->n_leaf_limit), 4 << 20);
+        h->plan_rows = std::min<int64_t>({extra * std::max(cfg->n_group_limit, cfg->n_leaf_limit), 31 * n, 4 << 20});
         NB_TRY(h->plan_walks.alloc(n + extra));
         NB_TRY(h->plan_order.alloc(n + extra));
         NB_TRY(h->splits.alloc(extra));
@@ -2342,7 +2351,7 @@ int pgf_nbody_create(const pgf_nbody_config* cfg, int64_t n, const double* pos, 
     NB_TRY(h->out_accp.alloc(n + h->plan_rows));
     NB_TRY(h->out_nnb.alloc(n + h->plan_rows));
     NB_TRY(h->flags.alloc(8));
-    NB_TRY(h->retest.alloc(h->retest_cap));
+    NB_TRY(ensure_retest(h));
     NB_TRY(h->hdr.alloc(1));
     h->bbox_blocks = (int)std::min<int64_t>((n + 255) / 256, 1024);
     NB_TRY(h->part.alloc(6 * (size_t)h->bbox_blocks));
@@ -2564,6 +2573,7 @@ int pgf_nbody_autotune(pgf_nbody* h, int repeats, int* best_variant, double* bes
     for (int v = 0; v < PGF_NUM_KERNEL_VARIANTS; ++v) {
         if (!valid_variant(v)) continue;
         h->variant = v;
+        NB_CUDA(ensure_retest(h));
         NB_CUDA(enqueue_force(h));  // warm-up
         NB_CUDA(cudaEventRecord(h->ev[0], h->stream));
         for (int r = 0; r < repeats; ++r) NB_CUDA(enqueue_force(h));
