@@ -1861,6 +1861,7 @@ static_assert(offsetof(pgf_nbody_sample, n_ngb) == offsetof(SampleRec, n_ngb), "
 struct pgf_nbody {
     int device = 0;
     int num_sms = 1;
+    int tree_ctas = 1;  // of the tree kernel
     cudaStream_t stream = nullptr;
     int64_t n = 0;
     pgf_nbody_config cfg{};
@@ -1995,7 +1996,13 @@ cudaError_t enqueue_build(pgf_nbody* h) {
         if (hooks.wait_limit_ns) a.wait_limit_ns = hooks.wait_limit_ns;
         a.stall = hooks.stall_after_items > 0;
         void* args[] = {&a};
-        e = cudaLaunchCooperativeKernel((const void*)tree_kernel, dim3(h->num_sms), dim3(kTreeThreads), args, 0, s);
+        // One CTA per SM, fewer where the context may use only part of them (the
+        // first build, outside a capture, finds out).
+        while ((e = cudaLaunchCooperativeKernel((const void*)tree_kernel, dim3(h->tree_ctas), dim3(kTreeThreads), args,
+                                                0, s)) == cudaErrorCooperativeLaunchTooLarge && h->tree_ctas > 1) {
+            (void)cudaGetLastError();
+            h->tree_ctas = (h->tree_ctas + 1) / 2;
+        }
         if (e != cudaSuccess) return e;
     }
     if ((e = cudaMemsetAsync(h->group_at.d, 0xff, sizeof(int32_t) * n, s)) != cudaSuccess) return e;
@@ -2306,6 +2313,7 @@ int pgf_nbody_create(const pgf_nbody_config* cfg, int64_t n, const double* pos, 
     } while (0)
     NB_TRY(cudaGetDevice(&h->device));
     NB_TRY(cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->device));
+    h->tree_ctas = h->num_sms;
     NB_TRY(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     for (auto& e : h->ev) NB_TRY(cudaEventCreate(&e));
     const size_t n3 = 3 * (size_t)n;
