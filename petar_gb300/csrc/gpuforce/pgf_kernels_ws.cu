@@ -839,7 +839,9 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
         since = 0;
     };
     // Exact FP64 neighbour test of a pair inside the guard band (a few pairs per
-    // evaluation); the changeover mode adds the pair's difference when it is one.
+    // evaluation); the changeover mode adds the pair's difference when it is one,
+    // formed in FP64, to the flushed (hi, lo) sums: the FP32 partial sums would
+    // round it to 24 bits.
     auto retest = [&](int k, int64_t jidx) -> int {
         const int gi = ibase + k * S;
         if (p.retest_total) atomicAdd(p.retest_total, 1);
@@ -852,9 +854,13 @@ __device__ void consumer(const Params& p, Smem<CW, KI, PK, TE, NS, MD, TM>& s, i
             if (nb && ci.id != cj.id) {
                 double d[5];
                 co_pair_diff(ei, ci, e, e.m, cj, p.eps2, rcut2d, d);
-                acc3(k, 1.f, (float)d[0], (float)d[1], (float)d[2]);
-                dt[k] += (float)d[3];
-                ds[k] += (float)d[4];
+                auto add = [](float2& v, double x) {
+                    const float h = (float)x;
+                    v = add_pair(v, make_float2(h, (float)(x - (double)h)));
+                };
+                for (int q = 0; q < 3; ++q) add(s.acc[k][q][ct], d[q]);
+                add(s.co.dtot[k][ct], d[3]);
+                add(s.co.dsoft[k][ct], d[4]);
             }
         }
         return nb;
