@@ -107,13 +107,14 @@ __global__ __launch_bounds__(kT, 2) void fp64_kernel(Params p) {
                     m = p.epj_m64[id];
                     rs = p.epj_rs64[id];
                     // Conservative: 0.1% over the radii and the FP32 rounding
-                    // of the absolute coordinates.
+                    // of the absolute coordinates.  A NaN among them (which
+                    // fmaxf hides in d2) makes the entry near.
                     const EpjF32 f = p.epj32[id];
                     const float dx = fabsf(f.xh - chx), dy = fabsf(f.yh - chy), dz = fabsf(f.zh - chz);
                     const float ex = fmaxf(dx - wd.hx, 0.f), ey = fmaxf(dy - wd.hy, 0.f), ez = fmaxf(dz - wd.hz, 0.f);
                     const float d2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
                     const float R = sqrtf(fmaxf(fmaxf(rsmax2, f.rs2), rc2));
-                    const float Rm = R * 1.001f + 1e-6f * (fmaxf(dx, fmaxf(dy, dz)) + hmax + cmax);
+                    const float Rm = R * 1.001f + 1e-6f * ((dx + dy + dz) + hmax + cmax);
                     near = !(d2 > Rm * Rm);
                 }
                 const unsigned bn = __ballot_sync(0xffffffffu, near);
