@@ -47,8 +47,8 @@ enum {
 
 /* Kernel selection for pgf_set_precision. */
 enum {
-    PGF_PRECISION_MIXED = 0, /* FP64 walk-relative coordinates, FP32 pair arithmetic,
-                                FP64 cross-tile sums, exact neighbour counts (default) */
+    PGF_PRECISION_MIXED = 0, /* walk-relative coordinates as FP32 (hi, lo) pairs, FP32 pair
+                                arithmetic, (hi, lo) sums, exact neighbour counts (default) */
     PGF_PRECISION_FP64 = 1   /* plain FP64 throughout */
 };
 
@@ -175,7 +175,16 @@ typedef struct pgf_profile {
  * the first call, as src/force_gpu_cuda.cu:549-553 does. */
 int pgf_initialize(int rank, double eps2, double rcut2, double G);
 
-/* Chooses the kernel used by later dispatches (PGF_PRECISION_*). */
+/* Chooses the kernel used by later dispatches (PGF_PRECISION_*).
+ *
+ * With PGF_PRECISION_MIXED, eps2 = 0 and long superparticle lists, the distant
+ * superparticles of a walk of 32 or more i-particles act on it through one local
+ * expansion, which leaves out at most 2^-23 of each one's force.  Lists are long
+ * from 4,000 EP-SP pairs per i-particle of the dispatch on (3,000 in dispatches of
+ * 80,000 i-particles or more; below 8,192 never), and in device-resident steps
+ * from 80,000 particles on; a row's last FP32 bits therefore depend on the
+ * dispatch it is part of.  Kernel variant 0, FP64 and the allocation-free call
+ * run every pair. */
 int pgf_set_precision(int precision);
 
 /* Selects what later dispatches compute (PGF_MODE_*).  Each tag keeps the
@@ -208,7 +217,10 @@ int pgf_set_dispatch_stages(int stages);
  * When a dispatch has few walks for the GPU's CTAs, each walk costing more
  * than a sixteenth of one SM's even share runs as up to 32 parts over slices
  * of its EPJ and SPJ lists, and the parts are added in a fixed order; results then differ
- * from an unsplit launch by FP32 summation order only (counts are exact).
+ * from an unsplit launch by FP32 summation order only (counts are exact).  With 0,
+ * dispatches of up to 400,000 i-particles also flush their FP32 partial sums at the end of
+ * every 256 list entries, as the device-resident step does, so that its results and
+ * theirs over the same lists agree far below FP32 rounding.
  * All modes; no counterpart in the reference. */
 int pgf_set_walk_split(int enable);
 

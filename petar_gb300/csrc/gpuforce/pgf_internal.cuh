@@ -536,8 +536,11 @@ inline bool far_applies_step(double eps2, int64_t n) { return eps2 == 0.0 && n >
 // multiples of it.
 constexpr int kPartAlign = 256;
 // Launches with more i-particles than this run their walks whole in the
-// device-resident step (they have enough of them: a King model of 1M has
-// 7,000 walks for 456 CTAs); up to it, whole walks flush at tile ends.
+// device-resident step (in groups of 512 they have enough of them: a King model
+// of 1M has 7,000 walks for 456 CTAs); up to it, whole walks flush at tile ends.
+// Step split and whole: King models of 262,144 2.40 and 2.64 ms, 400,000 3.35 and
+// 3.45, 524,288 4.27 and 4.27, 700,000 5.42 and 5.37, 1M 8.00 and 7.81.  Larger
+// groups leave fewer walks (600,000 particles in groups of 4,096: 7.9 and 31.7).
 constexpr int64_t kPlanRows = 400000;
 
 // First entry of part j of n entries in n_parts parts.
