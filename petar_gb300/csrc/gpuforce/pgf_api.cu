@@ -1033,7 +1033,8 @@ int dispatch_walks(int tag, int n_walk, const void* const* epi, const int* n_epi
     // 2.71 in eight; 65k, 5 M: 1.13 against 1.51 in four).  A neighbour search
     // has little to overlap with: its lists are gathered from host memory
     // faster than the host packs them (200k binaries, 27 M entries: 1.54 ms in
-    // one launch, 2.2 to 2.7 in stages), so it runs in one where that works.
+    // one launch, 2.2 to 2.7 in stages; 1M binaries 7.6 and 11.8; 30,000 0.38 in
+    // one), so it runs in one where that works.
     const bool hd_walks = use_hd() && hd_walks_ok(n_walk, epi, n_epi, il, id_epj, n_epj, id_spj, n_spj, t.mode);
     int n_chunks = g.stages;
     if (n_chunks == 0) {

@@ -26,13 +26,15 @@
 //   in shared memory with a two-sum (no FP64 in the pair loops either); the
 //   j-slices are combined as (hi, lo) pairs once per pass, and the i set up
 //   from EpiRel rows, so that a pass issues FP64 only to write its results
-//   (parts of split walks: not even there).
-// * Bound by the FMA pipe (73% of its cycles at King 1M, consumers waiting 6% of
-//   theirs) and, at three consumer warps per SMSP, by latency.  Without FP64 in
+//   (parts of split walks: not even there; FP64 records: x - c of each entry
+//   and i as well).
+// * Bound by the FMA pipe (74% of its cycles at 1M binaries, barrier stalls 0.25
+//   per issue) and, at three consumer warps per SMSP, by latency.  Without FP64 in
 //   the passes: 65,536 stars 0.784 -> 0.607 ms, 20,000 binary stars 0.486 ->
 //   0.282; with the slices' divisions and the re-test's branch out of the tiles
-//   and the final sums on all threads 0.585 and 0.252 ms; 1M binaries, with the
-//   far-field pass before it, 14.67 -> 14.27 ms in all.
+//   and the final sums on all threads 0.585 and 0.252 ms (all three with a
+//   far-field pass before it that neither size runs any more: 65,536 stars 0.615
+//   ms, all pairs); 1M binaries 13.7 ms after a pass of 2.6.
 // * Ambiguous neighbour pairs (within the guard band of r_search; a few per
 //   evaluation) are tested exactly in FP64 where they are met.
 // * Every mbarrier wait is bounded by 1 s of %globaltimer; on expiry the thread
